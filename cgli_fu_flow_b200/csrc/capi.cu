@@ -58,7 +58,6 @@ struct cgli_ctx {
   double *d_out = nullptr;     // device scratch for norms / bulk flux
   int update_blocks = 0;         // partial sums of the per-row update kernels (routine path, DP-LUR)
   int sweep_update_blocks = 0;   // partial sums of the update after the wavefront passes
-  int sweep_tiles = 0;
   cgli::SweepArgs sw;
   bool metrics_checked = false;
   cudaGraphExec_t iter_graph = nullptr;
@@ -195,6 +194,8 @@ int read_norms(cgli_ctx *c, double er[5], int nblocks) {
   if (status) {
     int zero = 0;
     cudaMemcpy(c->d.status, &zero, sizeof(int), cudaMemcpyHostToDevice);
+    // products that were never read are left behind: only the sentinel again
+    cudaMemset(c->sw.xbuf, 0xff, c->sw.hand_bytes);
     return fail(CGLI_ETIMEOUT, "a wavefront tile gave up waiting for its neighbour (bounded spin)");
   }
   for (int v = 0; v < 5; v++) er[v] = c->h_norms[v];
@@ -241,6 +242,14 @@ int check_channel_metrics(cgli_ctx *c) {
     CUDA_TRY(cudaMemcpy((void *)c->sw.etdytab, et.data(), sizeof(double) * d.Y, cudaMemcpyHostToDevice));
   }
   c->sw.channel_metrics = ok ? 1 : 0;
+  if (!ok) {
+    const bool mixed = c->p.precision == CGLI_MIXED;
+    if (!c->sw.met) {
+      int rc = alloc(c, (size_t)cgli::skew_size(d) * 9 * (mixed ? sizeof(float) : sizeof(double)), &c->sw.met);
+      if (rc) return rc;
+    }
+    cgli::launch_metric_stream(d, c->sw, c->stream, mixed);
+  }
   c->d.face_tables = 0;
   c->d.face_tables = cgli::check_face_tables(c->d, c->d.status + 8, c->stream) ? 1 : 0;
   cgli::launch_inverse_j(d, c->stream);
@@ -314,73 +323,50 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
   if (rc == CGLI_OK) rc = alloc(c, 16 * sizeof(int), (void **)&d.status);
   if (rc == CGLI_OK) rc = alloc(c, 3 * 4 * sizeof(double) * d.Y, (void **)&d.ftab);
   c->update_blocks = p->nx * p->ny;
-  // the wavefront's tile grid for this context's precision
-  const bool mixed_passes = p->precision == CGLI_MIXED;
-  const int nti = mixed_passes ? cgli::sweep_tiles_x<float>(p->nx) : cgli::sweep_tiles_x<double>(p->nx);
-  const int ntj = mixed_passes ? cgli::sweep_tiles_y<float>(p->ny) : cgli::sweep_tiles_y<double>(p->ny);
-  const int tile_i = mixed_passes ? cgli::SweepTile<float>::TI : cgli::SweepTile<double>::TI;
-  const int tile_j = mixed_passes ? cgli::SweepTile<float>::TJ : cgli::SweepTile<double>::TJ;
-  c->sweep_tiles = nti * ntj;
-  c->sweep_update_blocks = cgli::sweep_update_blocks(d, mixed_passes);
-  size_t nblk = (size_t)std::max(std::max(c->update_blocks, c->sweep_tiles), c->sweep_update_blocks);
+  c->sweep_update_blocks = cgli::sweep_update_blocks(d);
+  size_t nblk = (size_t)std::max(c->update_blocks, c->sweep_update_blocks);
   if (rc == CGLI_OK) rc = alloc(c, 5 * sizeof(double) * nblk, (void **)&d.partial);
   {
     cgli::SweepArgs &a = c->sw;
     memset(&a, 0, sizeof a);
     const bool mixed = p->precision == CGLI_MIXED;
     const size_t es = mixed ? sizeof(float) : sizeof(double);
-    const size_t nsk = (size_t)(mixed ? cgli::skew_size<float>(d) : cgli::skew_size<double>(d));
-    const size_t plane = (size_t)d.Y * d.Z;
-    for (int v = 0; v < 5; v++) {
-      if (mixed) {
-        if (rc == CGLI_OK) rc = alloc(c, nsk * es, (void **)&a.dqf[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.halo_ff[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.halo_bf[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.hxpf[v]);
-      } else {
-        if (rc == CGLI_OK) rc = alloc(c, nsk * es, (void **)&a.dq[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.halo_f[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.halo_b[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.hxp[v]);
-      }
+    const size_t nsk = (size_t)cgli::skew_size(d), plane = (size_t)d.Y * d.Z;
+    // the wavefront's tile grid for this context's precision
+    const int nti = mixed ? cgli::sweep_tiles_x<float>(p->nx) : cgli::sweep_tiles_x<double>(p->nx);
+    const int ntj = cgli::sweep_tiles_y(p->ny);
+    const size_t block = (size_t)cgli::sweep_steps(d) * 5 * cgli::SWEEP_TJ * es;   // one column block's five values, every step
+    if (rc == CGLI_OK) rc = alloc(c, nsk * 5 * es, &a.dq);
+    if (rc == CGLI_OK) rc = alloc(c, nsk * cgli::CR_N * es, &a.cellrec);
+    for (int side = 0; side < 2; side++) {
+      if (rc == CGLI_OK) rc = alloc(c, ntj * block, &a.halo[side]);
+      if (rc == CGLI_OK) rc = alloc(c, ntj * block, &a.hx[side]);
+      if (rc == CGLI_OK) rc = alloc(c, cgli::REC_N * plane * es, &a.hrec[side]);
     }
-    if (rc == CGLI_OK)
-      rc = alloc(c, nsk * cgli::CR_N * es, mixed ? (void **)&a.cellrecf : (void **)&a.cellrec);
-    for (int v = 0; v < cgli::REC_N; v++) {
-      if (mixed) {
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.hrecf_f[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.hrecf_b[v]);
-      } else {
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.hrec_f[v]);
-        if (rc == CGLI_OK) rc = alloc(c, plane * es, (void **)&a.hrec_b[v]);
-      }
+    const size_t xb = (size_t)nti * ntj * block, yb = (size_t)p->nx * ntj * p->nz * 5 * es;
+    a.hand_bytes = xb + yb;
+    if (rc == CGLI_OK) rc = alloc(c, a.hand_bytes, &a.xbuf);
+    if (rc == CGLI_OK) {
+      a.ybuf = (char *)a.xbuf + xb;
+      if (cudaMemset(a.xbuf, 0xff, a.hand_bytes) != cudaSuccess) rc = fail(CGLI_ECUDA, "cudaMemset");   // the sentinel
     }
-    size_t xb = (size_t)c->sweep_tiles * tile_j * p->nz * 5 * es;
-    size_t yb = (size_t)c->sweep_tiles * tile_i * p->nz * 5 * es;
-    if (rc == CGLI_OK) rc = alloc(c, xb, mixed ? (void **)&a.xbuff : (void **)&a.xbuf);
-    if (rc == CGLI_OK) rc = alloc(c, yb, mixed ? (void **)&a.ybuff : (void **)&a.ybuf);
     if (rc == CGLI_OK) rc = alloc(c, 64, (void **)&a.ticket);
     double *jt = nullptr, *et = nullptr;
     if (rc == CGLI_OK) rc = alloc(c, sizeof(double) * d.Y, (void **)&jt);
     if (rc == CGLI_OK) rc = alloc(c, sizeof(double) * d.Y, (void **)&et);
     a.Jtab = jt; a.etdytab = et;
     a.spin_limit = CGLI_WAIT_LIMIT_DEFAULT;
+    // the tickets' order of the tiles
+    std::vector<int> order;
+    cgli::sweep_tile_order(nti, ntj, mixed ? cgli::SweepTile<float>::TI : cgli::SweepTile<double>::TI, order);
+    int *dorder = nullptr;
+    if (rc == CGLI_OK) rc = alloc(c, sizeof(int) * order.size(), (void **)&dorder);
+    if (rc == CGLI_OK) cudaMemcpy(dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice);
+    a.order = dorder;
   }
   if (rc == CGLI_OK) {
     cudaError_t e = cgli::sweep_kernel_attributes();
     if (e != cudaSuccess) rc = fail(CGLI_ECUDA, std::string("sweep kernel attributes: ") + cudaGetErrorString(e));
-  }
-  if (rc == CGLI_OK) {
-    // wavefront clusters along x, and the tickets' order of the cluster
-    // rows (anti-diagonals of the grid of clusters)
-    cgli::SweepArgs &a = c->sw;
-    a.cluster_x = cgli::sweep_cluster_x(nti, ntj, mixed_passes);
-    std::vector<int> order;
-    cgli::sweep_tile_order(nti / a.cluster_x, ntj, order);
-    int *dorder = nullptr;
-    rc = alloc(c, sizeof(int) * order.size(), (void **)&dorder);
-    if (rc == CGLI_OK) cudaMemcpy(dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice);
-    a.order = dorder;
   }
   if (rc == CGLI_OK && cudaMallocHost(&c->h_norms, 16 * sizeof(double)) != cudaSuccess)
     rc = fail(CGLI_ENOMEM, "cudaMallocHost");
@@ -1047,8 +1033,9 @@ int cgli_profile_stages(cgli_ctx *c, int reps, double *ms) {
     CUDA_TRY(cudaEventRecord(ev[7], c->stream));
     cgli::launch_sweep_pass(c->d, c->sw, c->stream, mixed, true, false);
     CUDA_TRY(cudaEventRecord(ev[8], c->stream));
-    cgli::launch_sweep_pass(c->d, c->sw, c->stream, mixed, false, false);
+    cgli::launch_sweep_pass(c->d, c->sw, c->stream, mixed, false, true);
     cgli::launch_sweep_pass(c->d, c->sw, c->stream, mixed, true, true);
+    cgli::launch_sweep_update(c->d, c->sw, c->stream, mixed);
     rc = last_launch("profile_stages"); if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     for (int s = 0; s < CGLI_NSTAGES; s++) {

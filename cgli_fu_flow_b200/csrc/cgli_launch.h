@@ -22,115 +22,85 @@ __host__ __device__ __forceinline__ int rec_vec_pos(int u, int t) {
   return sizeof(T) == 8 ? (u ^ (t & 7)) : (u ^ ((t >> 1) & 3));
 }
 
-// Wavefront geometry per arithmetic type of the passes: TI x TJ (i, j)
-// columns per CTA (one thread each, so TI * TJ <= 1024 and a multiple of
-// 32), the depth of the ring of record stages in shared memory, and the
-// largest cluster of CTAs along x (1: no clusters).  Measured at
-// 256x192x192: the FP64 passes are fastest on 16 x 16 tiles with a 3-step
-// ring, the FP32 passes on 8 x 16 tiles in clusters of 8.
-#ifndef CGLI_SWEEP_TI
-#define CGLI_SWEEP_TI 16
-#endif
-#ifndef CGLI_SWEEP_TJ
-#define CGLI_SWEEP_TJ 16
-#endif
-#ifndef CGLI_SWEEP_RING
-#define CGLI_SWEEP_RING 3
-#endif
-#ifndef CGLI_SWEEP_CLUSTER_MAX
-#define CGLI_SWEEP_CLUSTER_MAX 1
-#endif
-#ifndef CGLI_SWEEP_TI_F32
-#define CGLI_SWEEP_TI_F32 8
-#endif
-#ifndef CGLI_SWEEP_TJ_F32
-#define CGLI_SWEEP_TJ_F32 16
-#endif
-#ifndef CGLI_SWEEP_RING_F32
-#define CGLI_SWEEP_RING_F32 2
-#endif
-#ifndef CGLI_SWEEP_CLUSTER_MAX_F32
-#define CGLI_SWEEP_CLUSTER_MAX_F32 8
-#endif
+// Wavefront geometry per arithmetic type of the passes: a CTA holds TI x rows
+// of SWEEP_TJ = 32 j columns (a warp per row, a lane per column); the steps of
+// records in flight per row on the channel grid and on general grids (what
+// shared memory holds).  TI = 4 with two CTAs per SM has faster steps but
+// twice the hand-overs between CTAs: 0.104 / 0.108 against 0.118 / 0.116 ms a
+// pass at 64^3, 0.55 / 0.53 against 0.49 / 0.46 at 256x192x192 (FP64).
+constexpr int SWEEP_TJ = 32;
 template <typename T> struct SweepTile;
 template <> struct SweepTile<double> {
-  static constexpr int TI = CGLI_SWEEP_TI, TJ = CGLI_SWEEP_TJ, RING = CGLI_SWEEP_RING;
-  static constexpr int CLUSTER_MAX = CGLI_SWEEP_CLUSTER_MAX;
+  static constexpr int TI = 8, TJ = SWEEP_TJ, RING = 4, RING_GENERAL = 3;
 };
 template <> struct SweepTile<float> {
-  static constexpr int TI = CGLI_SWEEP_TI_F32, TJ = CGLI_SWEEP_TJ_F32, RING = CGLI_SWEEP_RING_F32;
-  static constexpr int CLUSTER_MAX = CGLI_SWEEP_CLUSTER_MAX_F32;
+  static constexpr int TI = 8, TJ = SWEEP_TJ, RING = 4, RING_GENERAL = 4;
 };
-static_assert(SweepTile<double>::TI * SweepTile<double>::TJ <= 1024 &&
-                  (SweepTile<double>::TI * SweepTile<double>::TJ) % 32 == 0, "FP64 sweep tile shape");
-static_assert(SweepTile<float>::TI * SweepTile<float>::TJ <= 1024 &&
-                  (SweepTile<float>::TI * SweepTile<float>::TJ) % 32 == 0, "FP32 sweep tile shape");
 constexpr int CGLI_TIMEOUT_CODE = 6;
 
-// buffers of the tile-wavefront sweeps (kernels_sweep.cu)
+// Buffers of the wavefront sweeps (kernels_sweep.cu), in the arithmetic type
+// of the passes (double, or float for CGLI_MIXED).  A row's stream holds the
+// blocks of its forward steps s = 0 .. sweep_steps - 1, 32 columns each.
 struct SweepArgs {
-  // per-cell sweep data in the tile-skewed layout: slot (tile, forward step,
-  // thread) = (tile * S + s) * TI*TJ + t, S = Nz + TI + TJ - 2
-  double *dq[5];                  // dQ: forward result, then backward result (in place)
   // per slot, CR_N consecutive words: the split-Jacobian / diagonal record
   // (REC_N) and the residual MR (5), so that the residual writes and the
   // sweep reads whole 16-byte vectors of one cell
-  double *cellrec;
-  // the same in float for CGLI_MIXED
-  float *dqf[5], *cellrecf;
-  // periodic lagged halos, indexed j*Z_m + k: dQ of plane ie (forward) / 3
-  // (backward) and the records of planes 2 / ie+1
-  double *halo_f[5], *halo_b[5], *hrec_f[REC_N], *hrec_b[REC_N];
-  float *halo_ff[5], *halo_bf[5], *hrecf_f[REC_N], *hrecf_b[REC_N];
-  // the halo neighbour's product A.dQ of the current pass per (j, k), formed
-  // before the pass from the halo record and the lagged dQ
-  double *hxp[5];
-  float *hxpf[5];
-  double *xbuf, *ybuf;            // products handed between tiles
-  float *xbuff, *ybuff;
-  unsigned int *ticket;           // tile ticket counter
-  const int *order;               // tile visiting order (anti-diagonals)
+  void *cellrec;
+  void *dq;                       // per block [5][32]: forward result, then backward result (in place)
+  void *met;                      // per block [9][32]: the metric terms (general grids only)
+  // periodic lagged halos, [0] forward (plane ie), [1] backward (plane 3): dQ
+  // in step order [column block][step][5][32] and the products formed from
+  // it (k_halo_products); the records of planes 2 / ie+1 as [REC_N][j][k]
+  void *halo[2], *hx[2], *hrec[2];
+  // products handed between CTAs: [tile][step][5][32] along x, [row][column
+  // block][k][5] along y; hand_bytes of both, contiguous from xbuf
+  void *xbuf, *ybuf;
+  size_t hand_bytes;
+  unsigned int *ticket;           // tile ticket counters of the two passes
+  const int *order;               // tile visiting order
   const double *Jtab, *etdytab;   // per-j metrics of a grid uniform in x and z
   int channel_metrics;            // 1: use Jtab / etdytab instead of the 3-D arrays
   int spin_limit;                 // bounded wait (polls) for a neighbouring tile
-  int cluster_x;                  // wavefront CTAs per cluster along x (1: no clusters)
+  template <typename T>
+  __host__ __device__ __forceinline__ T *buf(void *p) const { return static_cast<T *>(p); }
 };
 
-// slot of cell (i, j, k) in the tile-skewed layout of the passes in type T
-template <typename T>
+// steps of a row's stream (a full block of columns)
+__host__ __device__ __forceinline__ int sweep_steps(const Dev &d) { return d.nz + SWEEP_TJ - 1; }
+// slot of cell (i, j, k) in the rows' streams
 __host__ __device__ __forceinline__ long long skew_slot(const Dev &d, int i, int j, int k) {
-  constexpr int TI = SweepTile<T>::TI, TJ = SweepTile<T>::TJ;
-  const int ntj = (d.ny + TJ - 1) / TJ;
-  const int S = d.nz + TI + TJ - 2;
-  const int il = (i - 3) % TI, jl = (j - 2) % TJ;
-  const int tile = ((i - 3) / TI) * ntj + (j - 2) / TJ;
-  const int s = (k - 2) + il + jl;
-  return ((long long)tile * S + s) * (TI * TJ) + il * TJ + jl;
+  const int ntj = (d.ny + SWEEP_TJ - 1) / SWEEP_TJ, jl = (j - 2) % SWEEP_TJ;
+  const long long stream = (long long)(i - 3) * ntj + (j - 2) / SWEEP_TJ;
+  return (stream * sweep_steps(d) + (k - 2) + jl) * SWEEP_TJ + jl;
 }
-template <typename T>
 __host__ __device__ __forceinline__ long long skew_size(const Dev &d) {
-  constexpr int TI = SweepTile<T>::TI, TJ = SweepTile<T>::TJ;
-  const long long ntiles = (long long)((d.nx + TI - 1) / TI) * ((d.ny + TJ - 1) / TJ);
-  return ntiles * (d.nz + TI + TJ - 2) * (TI * TJ);
+  return (long long)d.nx * ((d.ny + SWEEP_TJ - 1) / SWEEP_TJ) * sweep_steps(d) * SWEEP_TJ;
+}
+// word of the first of (j, k)'s five values (SWEEP_TJ apart) in the halos
+__host__ __device__ __forceinline__ long long halo_slot(const Dev &d, int j, int k) {
+  const int jl = (j - 2) % SWEEP_TJ;
+  return ((long long)((j - 2) / SWEEP_TJ) * sweep_steps(d) + (k - 2) + jl) * (5 * SWEEP_TJ) + jl;
 }
 // tiles of the wavefront in x and y for the passes in type T
 template <typename T> inline int sweep_tiles_x(int nx) { return (nx + SweepTile<T>::TI - 1) / SweepTile<T>::TI; }
-template <typename T> inline int sweep_tiles_y(int ny) { return (ny + SweepTile<T>::TJ - 1) / SweepTile<T>::TJ; }
+inline int sweep_tiles_y(int ny) { return (ny + SWEEP_TJ - 1) / SWEEP_TJ; }
 
-void sweep_tile_order(int nti, int ntj, std::vector<int> &order);
+void sweep_tile_order(int nti, int ntj, int ti, std::vector<int> &order);
 // shared-memory opt-in of the wavefront kernels (once per process and device)
 cudaError_t sweep_kernel_attributes();
-int sweep_cluster_x(int nti, int ntj, bool mixed);
+// a.met from the metrics of every interior cell
+void launch_metric_stream(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed);
 // the four wavefront passes (two sweeps) of one inner iteration
 void launch_sweeps(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed);
 // the update and norm partials after the last pass (k_update_skewed)
 void launch_sweep_update(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed);
 // partial sums (blocks) the update after the wavefront passes writes
-int sweep_update_blocks(const Dev &d, bool mixed);
+int sweep_update_blocks(const Dev &d);
 // everything of a fused inner iteration before the sweeps
 void launch_fused_residual(const Dev &d, const SweepArgs &a, cudaStream_t s, int precision);
-// one pass (forward / backward, final with the update) of the sweeps
-void launch_sweep_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed, bool backward, bool final_pass);
+// one pass of the first or the last sweep (a forward one with both passes'
+// halo products)
+void launch_sweep_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed, bool backward, bool last);
 // Dual_time_stepping.cpp:737-922 residual on the natural layout: MR and
 // NL = NR = D^-1 MR on the interior cells
 void launch_dts_residual(const Dev &d, cudaStream_t s);

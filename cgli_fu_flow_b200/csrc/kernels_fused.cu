@@ -1,8 +1,6 @@
 // Fast path of one inner iteration: halo and boundaries, fluxes, viscous
 // terms, residual assembly, four wavefront sweep passes with the update
 // fused into the last one.
-#include <type_traits>
-
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
 
@@ -45,7 +43,7 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
 
   const int ie = d.nx + 2;
   const bool halo_plane = (i == 2 || i == ie + 1);
-  const long long slot = halo_plane ? 0 : skew_slot<typename std::conditional<MIXED, float, double>::type>(d, i, j, k);
+  const long long slot = halo_plane ? 0 : skew_slot(d, i, j, k);
   double r8, r9, r10;   // record words stored together with MR
   {
     // the cell's sweep record; planes 2 and ie+1 (the periodic halo copies)
@@ -56,14 +54,10 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
                 deltaT, r);
     const long long h = (long long)j * d.dj + k;
     if (halo_plane) {
+      void *const hrec = a.hrec[i == 2 ? 0 : 1];
       for (int v2 = 0; v2 < REC_N; v2++) {
-        if (MIXED) {
-          if (i == 2) a.hrecf_f[v2][h] = (float)r[v2];
-          else a.hrecf_b[v2][h] = (float)r[v2];
-        } else {
-          if (i == 2) a.hrec_f[v2][h] = r[v2];
-          else a.hrec_b[v2][h] = r[v2];
-        }
+        if (MIXED) a.buf<float>(hrec)[v2 * d.di + h] = (float)r[v2];
+        else a.buf<double>(hrec)[v2 * d.di + h] = r[v2];
       }
       return;
     }
@@ -73,11 +67,11 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
     // slot's position in its step block, whose size is a multiple of 8)
     const int t = (int)(slot & 7);
     if (MIXED) {
-      float4 *o = reinterpret_cast<float4 *>(a.cellrecf + slot * CR_N);
+      float4 *o = reinterpret_cast<float4 *>(a.buf<float>(a.cellrec) + slot * CR_N);
       o[rec_vec_pos<float>(0, t)] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
       o[rec_vec_pos<float>(1, t)] = make_float4((float)r[4], (float)r[5], (float)r[6], (float)r[7]);
     } else {
-      double2 *o = reinterpret_cast<double2 *>(a.cellrec + slot * CR_N);
+      double2 *o = reinterpret_cast<double2 *>(a.buf<double>(a.cellrec) + slot * CR_N);
 #pragma unroll
       for (int q = 0; q < 5; q++) o[rec_vec_pos<double>(q, t)] = make_double2(r[2 * q], r[2 * q + 1]);
     }
@@ -127,11 +121,11 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
   // (record words 0..10, MR 11..15)
   const int t = (int)(slot & 7);
   if (MIXED) {
-    float4 *o = reinterpret_cast<float4 *>(a.cellrecf + slot * CR_N);
+    float4 *o = reinterpret_cast<float4 *>(a.buf<float>(a.cellrec) + slot * CR_N);
     o[rec_vec_pos<float>(2, t)] = make_float4((float)r8, (float)r9, (float)r10, (float)MR[0]);
     o[rec_vec_pos<float>(3, t)] = make_float4((float)MR[1], (float)MR[2], (float)MR[3], (float)MR[4]);
   } else {
-    double2 *o = reinterpret_cast<double2 *>(a.cellrec + slot * CR_N);
+    double2 *o = reinterpret_cast<double2 *>(a.buf<double>(a.cellrec) + slot * CR_N);
     (void)r8;
     (void)r9;
     o[rec_vec_pos<double>(5, t)] = make_double2(r10, MR[0]);
@@ -144,14 +138,13 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
     cell_metrics<CH>(d, a, j, c, mm);
     Diag<double> dd = diag<double>(q, mm, d.dxi, d.det, d.dzt, deltaT);
     double n5[5] = {dd.d11 * MR[0], dd.d22 * MR[1], dd.d22 * MR[2], dd.d22 * MR[3], dd.d51 * MR[0] + dd.d22 * MR[4]};
-    long long h = (long long)j * d.dj + k;
-    for (int n = 0; n < 5; n++) {
-      if (MIXED) {
-        if (i == ie) a.halo_ff[n][h] = (float)n5[n];
-        if (i == 3) a.halo_bf[n][h] = (float)n5[n];
-      } else {
-        if (i == ie) a.halo_f[n][h] = n5[n];
-        if (i == 3) a.halo_b[n][h] = n5[n];
+    const long long h = halo_slot(d, j, k);
+#pragma unroll
+    for (int side = 0; side < 2; side++) {   // plane ie feeds the forward pass, plane 3 the backward pass
+      if (i != (side ? 3 : ie)) continue;
+      for (int n = 0; n < 5; n++) {
+        if (MIXED) a.buf<float>(a.halo[side])[h + n * SWEEP_TJ] = (float)n5[n];
+        else a.buf<double>(a.halo[side])[h + n * SWEEP_TJ] = n5[n];
       }
     }
   }

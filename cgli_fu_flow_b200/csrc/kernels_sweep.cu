@@ -1,126 +1,94 @@
-// LU-SGS forward / backward sweeps as persistent tile wavefronts.
+// LU-SGS forward / backward sweeps as a systolic wavefront of warps.
 //
 // The reference visits the cells of one x-slab hyperplane by hyperplane
 // (i+j+k = m, Dual_time_stepping.cpp:983-1664), one OpenMP barrier per
 // plane.  A cell's update depends only on its three upwind neighbours, so
 // any order that respects that dependency graph gives the same numbers.
-// Here each CTA owns a TI x TJ tile of (i, j) columns and marches along k.
-// Thread (il, jl) handles cell k = 2 + s - il - jl at step s of the forward
-// pass: its i- and j-neighbours were handled by the neighbouring threads one
-// step earlier and hand over their products A.dQ through shared memory; its
-// k-neighbour is its own previous step.  The backward pass runs the mirror
-// image, and its step s visits exactly the cells of forward step S-1-s.
+// Here one warp owns one x row (i) of 32 j columns, one column per lane, and
+// marches along k: at step s of the forward pass lane jl handles cell
+// k = 2 + s - jl.  Its k neighbour is its own previous step (registers), its
+// j neighbour is the lane below at the previous step (a warp shuffle), and
+// its i neighbour is the same lane of the warp of row i - 1 at the same step,
+// which hands its products A.dQ over through a ring of shared-memory slots,
+// one mbarrier per slot and direction.  The backward pass runs the mirror
+// image, its steps visiting the forward steps in descending order.
+//
+// What bounds it: a pass is a chain of Nx + Ny + Nz dependent steps, and in
+// the middle of the chain the HBM traffic of about 1200 active warps.  There
+// is no block barrier: a warp waits only for the slot it needs next, so the
+// chain runs at the latency of one warp's step (load the slot, about ten
+// dependent FP64 operations, store the slot) and slower warps are absorbed
+// by the rings.
+// Measured (ms per forward / backward pass): 256x192x192 FP64 0.49 / 0.46,
+// FP32 0.36 / 0.35 (a tile of 16x16 or 8x16 columns with one thread per column
+// and a block barrier per step: 0.96 / 0.95 and 0.79 / 0.92); 64^3 FP64 0.118
+// / 0.115 (0.248 / 0.242).  One CTA alone takes 0.55 us per step in FP64 (0.83
+// before), 0.37 with four rows instead of eight: at eight rows, two warps per
+// scheduler, the shared-memory traffic of the steps (about 110 wavefronts a
+// row) adds up.
+//
+// A CTA holds TI rows (one warp each) of one 32-column block plus helper
+// warps that bring in what the rows read: XH warps fetch the x products of
+// the row before the CTA's first one (each every XH-th step, so XH round
+// trips to L2 are in flight), one warp fetches the y products of the
+// neighbouring column block for every row (a few lanes per row, each every
+// QY-th step).  They post into the same rings the rows use among themselves,
+// so the rows have no special cases; the slab's periodic x halo comes through
+// the x helpers as well (products formed by k_halo_products).
 //
 // Storage.  Everything the sweeps read per cell -- the split-Jacobian /
-// diagonal record, the residual MR and dQ -- lives in a tile-skewed layout,
-// slot (tile, forward step, thread), so at every step the threads of a tile
-// read and write consecutive words (the residual kernel writes it).  Only the
-// final update touches the reference layout.
+// diagonal record with the residual MR, and dQ -- lives in per-row streams
+// in the order the rows visit it: block (row, column block, forward step) of
+// 32 slots.  A row's block of one step arrives by asynchronous copies of the
+// row's own lanes, issued R steps ahead into the row's ring (only the lanes
+// with a cell at that step are copied).  The residual kernel writes the records, the final
+// update reads dQ; only these two touch the reference layout.
 //
-// Hand-over between tiles.  Tiles pass the products of their last row /
-// column through global buffers filled with a sentinel bit pattern before the
-// pass; the consumer spins (bounded) on the values themselves until none is
-// the sentinel, so a hand-over needs no fence and no counter (4- and 8-byte
-// stores are single-copy atomic).  A wait on another tile gives up after
-// SweepArgs::spin_limit polls, or at once when its CTA or any tile has
-// already given up (the CTA's dead flag, the status word): it records the
-// timeout code in the status word and the tile carries on to the end of the
-// pass without waiting, computing values nobody will use.  So no wait is
-// ever repeated at full length, every bulk copy is still awaited in order
-// (those waits have a fixed bound: the copies complete on their own), the
-// fast path carries no exit test, the update kernel leaves the state alone
-// and the host reports CGLI_ETIMEOUT.
-// Tiles take tickets in an order where every dependency holds a smaller
-// ticket, so a waiting CTA only ever waits on CTAs that are already running.
-//
-// Thread-block clusters (SweepArgs::cluster_x > 1, the CL instantiation):
-// the CTAs of a cluster are consecutive tiles along x, launched together.
-// Inside a cluster the x hand-over is pushed, not pulled: the producing
-// tile writes the products of its edge row straight into the consuming
-// tile's shared-memory ring with st.async, which counts the bytes on that
-// slot's mbarrier in the consumer (armed by the consumer with the bytes it
-// expects); the consumer waits on its own barrier and gives the slot back
-// with a relaxed arrival on the producer's "empty" barrier.  No fence is on
-// either path.  The first (last) tile of a cluster still receives (sends)
-// through the global buffers.  A cluster takes one ticket for its whole row
-// of tiles.  A CTA must not leave while a push into its shared memory is
-// still in flight, and a slot must not be re-armed before its phase has
-// completed, so the receiving lanes wait on every hand-over step, whether
-// their own cell is inside the slab or not, and these waits do not give up
-// at the tile wait limit or on the dead flag: the producer always pushes
-// every step (it is co-scheduled with the consumer and its own waits are
-// bounded), so they have the fixed bound of a copy wait, scaled by the wait
-// limit because the producer may itself sit in one wait of that length.
+// Hand-over between CTAs.  Products cross through global buffers that hold a
+// sentinel bit pattern wherever no value is waiting; the consumer polls the
+// values themselves, so a hand-over needs no fence and no counter (4- and
+// 8-byte stores are single-copy atomic), and puts the sentinel back once it
+// has read a value, so the buffers are ready for the next pass without a
+// fill.  A poll gives up after SweepArgs::spin_limit tries, or at once when
+// its CTA or any other has given up (the CTA's dead flag, the status word):
+// it records the timeout code in the status word and posts what it has, so
+// that every warp runs to the end of the pass without waiting, computing
+// values nobody will use; the ring waits inside a CTA follow the dead flag
+// too.  The update kernel then leaves the state alone, the host reports CGLI_ETIMEOUT and refills the
+// buffers with the sentinel.
+// CTAs take tickets in the order in which the wavefront reaches their tiles,
+// where every dependency holds a smaller ticket, so a waiting CTA only ever
+// waits on CTAs that are already running.
 //
 // The periodic x halo keeps the reference's lag: the forward pass at i = 3
-// uses dQ of plane Nx+2 as it was at the start of the sweep (halo_f), the
-// backward pass at i = Nx+2 uses dQ of plane 3 (halo_b).  The backward pass of
-// the first sweep writes both halos for the second sweep; after the final
-// backward pass a separate, fully parallel kernel applies the primitive
-// update of Dual_time_stepping.cpp:1702-1743 and accumulates the squared
-// increments of the residual norms.
+// uses dQ of plane Nx+2 as it was at the start of the sweep, the backward
+// pass at i = Nx+2 uses dQ of plane 3.  The backward pass of the first sweep
+// writes both halos for the second sweep.  (Its dQ elsewhere is used by
+// nothing: the second forward pass starts from MR, Dual_time_stepping.cpp:
+// 1289-1293 with the lagged plane of :942-976; so only the halo planes of
+// that pass are stored.)  After the final backward pass a separate, fully
+// parallel kernel applies the primitive update of
+// Dual_time_stepping.cpp:1702-1743 and accumulates the squared increments of
+// the residual norms.
 //
 // T is the arithmetic type of the sweep (double, or float for CGLI_MIXED).
+#include <algorithm>
+#include <type_traits>
+
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
 #include "tc_sm100.cuh"
 
-// steps ahead that a tile loads the products its neighbouring tiles hand over
-#ifndef CGLI_SWEEP_PREFETCH
-#define CGLI_SWEEP_PREFETCH 2
-#endif
-// tiles per SM the wavefront kernel is compiled for (a register cap)
-#ifndef CGLI_SWEEP_MINBLOCKS
-#define CGLI_SWEEP_MINBLOCKS 1
-#endif
-// backward pass: the forward result dQ of each step arrives with the
-// records' bulk copy (five rows of one value per thread)
-
 namespace cgli {
 
-using F64 = SweepTile<double>;
-using F32 = SweepTile<float>;
-
-template <typename T> struct SweepPtrs;
-template <> struct SweepPtrs<double> {
-  __device__ __forceinline__ static double *const *dq(const SweepArgs &a) { return a.dq; }
-  __device__ __forceinline__ static const double *cellrec(const SweepArgs &a) { return a.cellrec; }
-  __device__ __forceinline__ static double *const *hf(const SweepArgs &a) { return a.halo_f; }
-  __device__ __forceinline__ static double *const *hb(const SweepArgs &a) { return a.halo_b; }
-  __device__ __forceinline__ static double *const *hrec(const SweepArgs &a, bool b) { return b ? a.hrec_b : a.hrec_f; }
-  __device__ __forceinline__ static double *xb(const SweepArgs &a) { return a.xbuf; }
-  __device__ __forceinline__ static double *yb(const SweepArgs &a) { return a.ybuf; }
-  __device__ __forceinline__ static double *const *hxp(const SweepArgs &a) { return a.hxp; }
-};
-template <> struct SweepPtrs<float> {
-  __device__ __forceinline__ static float *const *dq(const SweepArgs &a) { return a.dqf; }
-  __device__ __forceinline__ static const float *cellrec(const SweepArgs &a) { return a.cellrecf; }
-  __device__ __forceinline__ static float *const *hf(const SweepArgs &a) { return a.halo_ff; }
-  __device__ __forceinline__ static float *const *hb(const SweepArgs &a) { return a.halo_bf; }
-  __device__ __forceinline__ static float *const *hrec(const SweepArgs &a, bool b) { return b ? a.hrecf_b : a.hrecf_f; }
-  __device__ __forceinline__ static float *xb(const SweepArgs &a) { return a.xbuff; }
-  __device__ __forceinline__ static float *yb(const SweepArgs &a) { return a.ybuff; }
-  __device__ __forceinline__ static float *const *hxp(const SweepArgs &a) { return a.hxpf; }
-};
-
-// face-direction metrics of a cell: general 3-D arrays, or a grid uniform in
-// x and z (channel) whose only varying term is etdy(j), held in shared memory
+// face-direction metrics of a cell: general (a row's nine terms per cell in
+// the step-ordered metric stream), or a grid uniform in x and z (channel)
+// whose only varying term is etdy(j)
 struct MetricsGeneral {
   static constexpr bool kChannel = false;
-  template <typename T>
-  __device__ __forceinline__ static void dirs(const Dev &d, const double *, long long c, int, T mm[9]) {
-#pragma unroll
-    for (int v = 0; v < 9; v++) mm[v] = (T)d.m[v][c];
-  }
 };
 struct MetricsChannel {
   static constexpr bool kChannel = true;
-  template <typename T>
-  __device__ __forceinline__ static void dirs(const Dev &, const double *et, long long, int jl, T mm[9]) {
-    mm[0] = 1; mm[1] = 0; mm[2] = 0;
-    mm[3] = 0; mm[4] = (T)et[jl]; mm[5] = 0;
-    mm[6] = 0; mm[7] = 0; mm[8] = 1;
-  }
 };
 
 __device__ __forceinline__ double ld_gpu(const double *p) {
@@ -135,6 +103,8 @@ __device__ __forceinline__ float ld_gpu(const float *p) {
 }
 __device__ __forceinline__ bool is_sentinel(double v) { return __double_as_longlong(v) == -1ll; }
 __device__ __forceinline__ bool is_sentinel(float v) { return __float_as_int(v) == -1; }
+__device__ __forceinline__ void put_sentinel(double *p) { *p = __longlong_as_double(-1ll); }
+__device__ __forceinline__ void put_sentinel(float *p) { *p = __int_as_float(-1); }
 
 // a wait on another tile has given up somewhere: this CTA's dead flag or
 // the grid's status word
@@ -146,50 +116,34 @@ __device__ __forceinline__ void give_up(volatile int *dead, int *status) {
   *dead = 1;
 }
 
-// bounded spin on five values handed over by a neighbouring tile; false when
-// it gives up (after `limit` polls, or at once once anything gave up)
-template <typename T>
-__device__ __forceinline__ bool recv5(const T *src, T out[5], int *status, int limit, volatile int *dead) {
-  for (int it = 0;; it++) {
-    bool ok = true;
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-      out[v] = ld_gpu(src + v);
-      ok = ok && !is_sentinel(out[v]);
-    }
-    if (ok) return true;
-    if (it >= limit || given_up(dead, status)) {
-      give_up(dead, status);
-      return false;
-    }
-    __nanosleep(20);
+// a thread's 16-byte asynchronous copy into shared memory (not kept in L1)
+// and the groups of such copies
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// Wait on a ring slot of this CTA (a phase completed by another of its
+// warps).  Those warps wait on nothing but such slots and on polls that give
+// up after the wait limit, and all of them follow the dead flag, so this
+// ends with theirs; `polls` bounds it by itself as well.
+__device__ __noinline__ void ring_wait_slow(uint32_t bar, uint32_t parity, int polls, volatile int *dead, int *status) {
+  for (int n = 0; n < polls; n++) {
+    if (tc::mbar_try(bar, parity)) return;
+    if (*dead) return;
   }
+  give_up(dead, status);
+}
+__device__ __forceinline__ void ring_wait(uint32_t bar, uint32_t parity, int polls, volatile int *dead, int *status) {
+  if (!tc::mbar_try(bar, parity)) ring_wait_slow(bar, parity, polls, dead, status);
 }
 
-// polls of the wait on a tile's own bulk copy of records (the copies complete
-// on their own; this only bounds the wait against a failing device)
-constexpr int kCopyPolls = 1 << 20;
-
-// REC_N record words and (mr non-null) the 5 MR words of one slot, through
-// the read-only path (CGLI_SWEEP_LDG) or plain loads
-#ifndef CGLI_SWEEP_LDG
-#define CGLI_SWEEP_LDG 0
-#endif
-__device__ __forceinline__ double2 ld_rec(const double2 *q) {
-#if CGLI_SWEEP_LDG
-  return __ldg(q);
-#else
-  return *q;
-#endif
-}
-__device__ __forceinline__ float4 ld_rec(const float4 *q) {
-#if CGLI_SWEEP_LDG
-  return __ldg(q);
-#else
-  return *q;
-#endif
-}
-// The 16-byte vectors of a slot are stored in an order rotated by the
+// REC_N record words and (mr non-null) the 5 MR words of one slot.  The
+// 16-byte vectors of a slot are stored in an order rotated by the
 // slot's position t in its step block (rec_vec_pos): a warp's vector loads
 // of its slots (one per lane, consecutive slots 128 B (FP64) or 64 B (FP32)
 // apart) then fall on distinct shared-memory banks in every phase of eight
@@ -199,479 +153,510 @@ __device__ __forceinline__ void load_cellrec(const double *p, int t, double rec[
   const double2 *q = reinterpret_cast<const double2 *>(p);
 #pragma unroll
   for (int u = 0; u < 5; u++) {
-    const double2 v = ld_rec(q + rec_vec_pos<double>(u, t));
+    const double2 v = q[rec_vec_pos<double>(u, t)];
     rec[2 * u] = v.x;
     rec[2 * u + 1] = v.y;
   }
-  const double2 a = ld_rec(q + rec_vec_pos<double>(5, t));
+  const double2 a = q[rec_vec_pos<double>(5, t)];
   rec[10] = a.x;
   if (mr) {
-    const double2 b = ld_rec(q + rec_vec_pos<double>(6, t)), c = ld_rec(q + rec_vec_pos<double>(7, t));
+    const double2 b = q[rec_vec_pos<double>(6, t)], c = q[rec_vec_pos<double>(7, t)];
     mr[0] = a.y; mr[1] = b.x; mr[2] = b.y; mr[3] = c.x; mr[4] = c.y;
   }
 }
 __device__ __forceinline__ void load_cellrec(const float *p, int t, float rec[REC_N], float *mr) {
   const float4 *q = reinterpret_cast<const float4 *>(p);
-  const float4 a = ld_rec(q + rec_vec_pos<float>(0, t)), b = ld_rec(q + rec_vec_pos<float>(1, t)),
-               c = ld_rec(q + rec_vec_pos<float>(2, t));
+  const float4 a = q[rec_vec_pos<float>(0, t)], b = q[rec_vec_pos<float>(1, t)],
+               c = q[rec_vec_pos<float>(2, t)];
   rec[0] = a.x; rec[1] = a.y; rec[2] = a.z; rec[3] = a.w;
   rec[4] = b.x; rec[5] = b.y; rec[6] = b.z; rec[7] = b.w;
   rec[8] = c.x; rec[9] = c.y; rec[10] = c.z;
   if (mr) {
-    const float4 e = ld_rec(q + rec_vec_pos<float>(3, t));
+    const float4 e = q[rec_vec_pos<float>(3, t)];
     mr[0] = c.w; mr[1] = e.x; mr[2] = e.y; mr[3] = e.z; mr[4] = e.w;
   }
 }
 
 // The x neighbour of the slab's first plane (forward) / last plane
 // (backward) is the periodic halo plane 2 / ie+1, a copy of plane ie / 3 made
-// by the Q halo exchange; its record and the lagged dQ are kept per (j, k).
-// Its product A+.dQ (forward) / A-.dQ (backward) is formed here once per
-// pass for every (j, k), off the wavefront's critical path.
+// by the Q halo exchange; its record is kept per (j, k), the lagged dQ of
+// that plane in the rows' step order.  The products A+.dQ (forward,
+// blockIdx.z = 0) and A-.dQ (backward, 1) are formed here once per sweep for
+// every (j, k), off the wavefront's critical path, in step order for the
+// rows' x helpers.  Both passes' products come from one launch: both inputs
+// are known before the sweep's first pass.  The launch also resets the two
+// passes' tickets.
 template <class Met, bool BACKWARD, typename T>
-__global__ void k_halo_products(Dev d, SweepArgs a) {
-  const int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = 2 + blockIdx.y;
-  if (k > d.nz + 1) return;
+__device__ __noinline__ void halo_product(const Dev &d, const SweepArgs &a, int j, int k) {
   const long long h = (long long)j * d.dj + k;
-  T rn[REC_N], mm[9];
+  T rn[REC_N], mx = 1, my = 0, mz = 0;
 #pragma unroll
-  for (int v = 0; v < REC_N; v++) rn[v] = SweepPtrs<T>::hrec(a, BACKWARD)[v][h];
-  Met::template dirs<T>(d, a.etdytab, h + (BACKWARD ? (long long)(d.nx + 3) : 2LL) * d.di, j, mm);
-  Split<T> An = split_from_record<T>(rn, 0, mm[0], mm[1], mm[2]);
+  for (int v = 0; v < REC_N; v++) rn[v] = a.buf<T>(a.hrec[BACKWARD])[v * d.di + h];
+  if (!Met::kChannel) {
+    const long long c = h + (BACKWARD ? (long long)(d.nx + 3) : 2LL) * d.di;
+    mx = (T)d.m[0][c]; my = (T)d.m[1][c]; mz = (T)d.m[2][c];
+  }
+  const Split<T> An = split_from_record<T>(rn, 0, mx, my, mz);
+  const long long s = halo_slot(d, j, k);
   T nh[5], o[5];
 #pragma unroll
-  for (int v = 0; v < 5; v++) nh[v] = BACKWARD ? SweepPtrs<T>::hb(a)[v][h] : SweepPtrs<T>::hf(a)[v][h];
+  for (int v = 0; v < 5; v++) nh[v] = a.buf<T>(a.halo[BACKWARD])[s + v * SWEEP_TJ];
   if (BACKWARD) upper_terms<T>(An, nh, o); else lower_terms<T>(An, nh, o);
 #pragma unroll
-  for (int v = 0; v < 5; v++) SweepPtrs<T>::hxp(a)[v][h] = o[v];
+  for (int v = 0; v < 5; v++) a.buf<T>(a.hx[BACKWARD])[s + v * SWEEP_TJ] = o[v];
 }
+template <class Met, typename T>
+__global__ void k_halo_products(const __grid_constant__ Dev d, const __grid_constant__ SweepArgs a) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.ticket[blockIdx.z] = 0;
+  const int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
+  if (k > d.nz + 1) return;
+  if (blockIdx.z == 0) halo_product<Met, false, T>(d, a, 2 + blockIdx.y, k);
+  else halo_product<Met, true, T>(d, a, 2 + blockIdx.y, k);
+}
+
+// the nine metric terms of every interior cell in step order (general grids;
+// once per change of the metrics)
+template <typename T>
+__global__ void k_metric_stream(Dev d, T *out) {
+  const int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = 2 + blockIdx.y, i = 3 + blockIdx.z;
+  if (k > d.nz + 1) return;
+  const long long slot = skew_slot(d, i, j, k), c = ix(d, i, j, k);
+  T *o = out + slot / SWEEP_TJ * (9 * SWEEP_TJ) + slot % SWEEP_TJ;
+#pragma unroll
+  for (int v = 0; v < 9; v++) o[v * SWEEP_TJ] = (T)d.m[v][c];
+}
+void launch_metric_stream(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed) {
+  const dim3 g((d.nz + 63) / 64, d.ny, d.nx);
+  if (mixed) k_metric_stream<float><<<g, 64, 0, s>>>(d, (float *)a.met);
+  else k_metric_stream<double><<<g, 64, 0, s>>>(d, (double *)a.met);
+}
+
+// a*b + c and a*b as written: the sums of products of a step are spelled out
+// in these, so that their rounding does not depend on which of two products
+// the compiler happens to fuse (it decides by the products' other uses, and
+// the steps of the ramps and of the middle would round differently)
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 // The split products of one direction for a face metric with a single
 // nonzero component m on momentum component q = DIR + 1 (the channel grid:
 // xi = (1,0,0), eta = (0,etdy,0), zeta = (0,0,1)): lower_terms / upper_terms
-// of split_from_record with the zero entries left out.
+// of split_from_record with the zero entries left out.  (Forward, the x and z
+// directions share the product hr n[0].)
 template <typename T, int DIR, bool BACKWARD>
 __device__ __forceinline__ void channel_products(const T r[REC_N], T m, const T n[5], T o[5]) {
   constexpr int q = DIR + 1;
-  const T U = r[R_UX + DIR], lam = r[R_LX + DIR], beta = r[R_BETA];
-  const T p1q = r[R_H] * m, pq1 = r[R_HR] * m, p5q = rec_hbt<T>(r) * m, p51 = rec_g<T>(r) * U;
-  if (!BACKWARD) {
-    const T p11 = (T)0.5 * (beta * U + lam), p22 = (T)0.5 * (U + lam);
-    o[0] = -p11 * n[0] - p1q * n[q];
+  const T U = r[R_UX + DIR], lam = BACKWARD ? -r[R_LX + DIR] : r[R_LX + DIR], beta = r[R_BETA];
+  const T sign = BACKWARD ? (T)1 : (T)-1;
+  const T p1q = sign * mul_rn(r[R_H], m), pq1 = sign * mul_rn(r[R_HR], m), p5q = sign * mul_rn(rec_hbt<T>(r), m);
+  const T p51 = sign * mul_rn(rec_g<T>(r), U);
+  const T p11 = sign * mul_rn((T)0.5, fma_rn(beta, U, lam)), p22 = sign * mul_rn((T)0.5, U + lam);
+  o[0] = fma_rn(p11, n[0], mul_rn(p1q, n[q]));
 #pragma unroll
-    for (int v = 1; v <= 3; v++) o[v] = v == q ? -pq1 * n[0] - p22 * n[v] : -p22 * n[v];
-    o[4] = -p51 * n[0] - p5q * n[q] - p22 * n[4];
-  } else {
-    const T m11 = (T)0.5 * (beta * U - lam), m22 = (T)0.5 * (U - lam);
-    o[0] = +m11 * n[0] + p1q * n[q];
-#pragma unroll
-    for (int v = 1; v <= 3; v++) o[v] = v == q ? +pq1 * n[0] + m22 * n[v] : m22 * n[v];
-    o[4] = +p51 * n[0] + p5q * n[q] + m22 * n[4];
-  }
+  for (int v = 1; v <= 3; v++)
+    o[v] = v != q ? mul_rn(p22, n[v])
+           : !BACKWARD && DIR != 1 ? fma_rn(p22, n[v], mul_rn(pq1, n[0]))
+                                   : fma_rn(pq1, n[0], mul_rn(p22, n[v]));
+  o[4] = fma_rn(p22, n[4], fma_rn(p51, n[0], mul_rn(p5q, n[q])));
 }
 
-template <int TI, int TJ, class Met, bool BACKWARD, typename T, bool CL>
-__global__ void __launch_bounds__(TI *TJ, CGLI_SWEEP_MINBLOCKS) k_sweep(Dev d, SweepArgs a) {
-  __shared__ T sx[2][TI][TJ][5];   // i-direction products, double-buffered by step parity
-  __shared__ T sy[2][TI][TJ][5];   // j-direction products
-  __shared__ double s_jt[TJ], s_et[TJ];
-  __shared__ int s_tile;
-  __shared__ int s_dead;       // a wait of this CTA gave up: no more waiting
-  // x hand-over ring inside a cluster: RX steps x TJ lanes x XW words
-  constexpr int RX = 8, XW = sizeof(T) == 8 ? 6 : 8;
-  __shared__ __align__(8) uint64_t s_full[CL ? RX : 1], s_empty[CL ? RX : 1];
-  // steps of records in flight: the ring holds RING steps' blocks, the copy
-  // of step s + RING - 1 is issued at step s
-  constexpr int RING = SweepTile<T>::RING;
-  constexpr bool DQB = BACKWARD;
-  __shared__ __align__(8) uint64_t s_bar[RING];
-  // the CTA's records of RING steps: step s's TI*TJ slots are one contiguous
-  // block of TI*TJ*CR_N words in the tile-skewed layout, brought in with one
-  // bulk copy RING - 1 steps ahead (backward, optionally followed by the five
-  // rows of the step's forward result dQ)
+// Geometry of a pass: TI row warps, XH x helpers and one y helper per CTA.
+// R: slots of a row's rings (x products, y products, records), so steps of
+// records on their way into shared memory.
+constexpr int SWEEP_XH = 3;
+template <typename T, bool GEN, bool BACKWARD>
+struct SweepShape {
+  static constexpr int TI = SweepTile<T>::TI, TJ = SWEEP_TJ;
+  static constexpr int R = GEN ? SweepTile<T>::RING_GENERAL : SweepTile<T>::RING;
+  static constexpr int THREADS = 32 * (TI + SWEEP_XH + 1);
+  static constexpr int QY = 32 / TI < R ? 32 / TI : R;   // y helper lanes per row
+  // words of one ring stage: 32 slots, the forward result (backward pass),
+  // the metric terms (general grids)
+  static constexpr int REC = TJ * CR_N, DQ = BACKWARD ? TJ * 5 : 0, MET = GEN ? TJ * 9 : 0;
+  static constexpr int STAGE = REC + DQ + MET;
+  static constexpr int WORDS = TI * R * (STAGE + 5 * TJ + 8) + R * 5 * TJ;   // (x slots of one more row)
+  static constexpr int SMEM = WORDS * (int)sizeof(T);
+  static_assert(32 % TI == 0, "helper lanes per row");
+  // a producer that takes every n-th step must not run two uses of a slot
+  // ahead of the row (the parity of a phase would be ambiguous): n <= R
+  static_assert(SWEEP_XH <= R && QY <= R, "ring depth");
+  static_assert(SMEM + 8 * (TI + 1) * R * 2 + 64 <= 227 * 1024, "shared memory of a pass");
+};
+
+template <class Met, bool BACKWARD, typename T>
+__global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREADS, 1)
+    k_sweep(Dev d, SweepArgs a, int last) {
+  using G = SweepShape<T, !Met::kChannel, BACKWARD>;
+  constexpr int TI = G::TI, TJ = G::TJ, R = G::R, XH = SWEEP_XH, QY = G::QY;
   extern __shared__ __align__(128) unsigned char s_dyn[];
-  T *const s_rec = reinterpret_cast<T *>(s_dyn);
-  constexpr int kStage = TI * TJ * (CR_N + (DQB ? 5 : 0));   // words per ring stage
-  T *const s_rx = s_rec + RING * kStage;   // the cluster ring follows the record ring
-  const int il = threadIdx.x / TJ, jl = threadIdx.x % TJ;
+  T *const s_rec = reinterpret_cast<T *>(s_dyn);             // [TI][R][STAGE]
+  T *const s_x = s_rec + TI * R * G::STAGE;                  // [TI + 1][R][5][TJ]
+  T *const s_y = s_x + (TI + 1) * R * 5 * TJ;                // [TI][R][8]
+  // per row and slot: the step's x (and y) products are posted; the row is
+  // done with them.  Row TI stands for no row: the last row of the flow posts
+  // there what nobody reads, so that all rows run the same instructions.
+  __shared__ __align__(8) uint64_t b_in[TI + 1][R], b_done[TI][R];
+  __shared__ int s_tile, s_dead;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nti = (d.nx + TI - 1) / TI, ntj = (d.ny + TJ - 1) / TJ;
-  // cluster of ncl consecutive x tiles (1 without clusters): one ticket per
-  // cluster, taken by its first CTA and written into every CTA's s_tile
-  const uint32_t ncl = CL ? tc::cluster_nctarank() : 1u, crank = CL ? tc::cluster_ctarank() : 0u;
-  const int nunits = (nti / (int)ncl) * ntj;
   if (threadIdx.x == 0) {
-    if (!CL) {
-      s_tile = (int)atomicAdd(a.ticket, 1u);
-    } else if (crank == 0) {
-      const uint32_t t = atomicAdd(a.ticket, 1u);
-      for (uint32_t r = 0; r < ncl; r++) tc::st_cluster_u32(tc::mapa(tc::smem_addr(&s_tile), r), t);
-    }
+    s_tile = (int)atomicAdd(a.ticket + (BACKWARD ? 1 : 0), 1u);
     s_dead = 0;
-    if (CL) {
-#pragma unroll
-      for (int r = 0; r < RX; r++) {
-        tc::mbar_init(tc::smem_addr(&s_full[r]), 1);    // the consumer's own arm per use
-        tc::mbar_init(tc::smem_addr(&s_empty[r]), 1);   // the consumer's release per use
-      }
-      // a receiving CTA arms its first RX slots with the bytes of one push
-      // before its producer can start (the cluster barrier below)
-      if (ncl > 1 && (BACKWARD ? crank + 1 < ncl : crank > 0))
-        for (int r = 0; r < RX && r < d.nz + TJ - 1; r++)
-          tc::mbar_expect_tx(tc::smem_addr(&s_full[r]), TJ * 5 * sizeof(T));
-    }
-#pragma unroll
-    for (int r = 0; r < RING; r++) tc::mbar_init(tc::smem_addr(&s_bar[r]), 1);
-    tc::mbar_fence_init();
-  }
-  // tickets and barriers visible cluster-wide before any remote access
-  if (CL) tc::cluster_sync(); else __syncthreads();
-  const int ticket = s_tile;
-  if (!CL && ticket >= nunits) return;   // (a cluster's ticket is always in range)
-  const int unit = a.order[BACKWARD ? nunits - 1 - ticket : ticket];
-  const int ta = (unit / ntj) * (int)ncl + (int)crank, tb = unit % ntj;
-  const int tile = ta * ntj + tb;
-  const int ie = d.nx + 2, jn = d.ny + 1;
-  const int i = 3 + ta * TI + il, j = 2 + tb * TJ + jl;
-  const bool inside = (i <= ie) && (j <= jn);
-  if (threadIdx.x < TJ) {
-    int jj = 2 + tb * TJ + threadIdx.x;
-    s_jt[threadIdx.x] = (Met::kChannel && jj <= jn) ? a.Jtab[jj] : 1.0;
-    s_et[threadIdx.x] = (Met::kChannel && jj <= jn) ? a.etdytab[jj] : 0.0;
   }
   __syncthreads();
-  const int Nz = d.nz;
-  const int S = Nz + TI - 1 + TJ - 1;
-  const long long tile_base = (long long)tile * S * (TI * TJ);
-  constexpr uint32_t kBlock = TI * TJ * CR_N * sizeof(T);
-  constexpr uint32_t kRow = TI * TJ * sizeof(T);
-  const T *const crec = SweepPtrs<T>::cellrec(a);
-  auto issue = [&](int step) {   // one thread
-    const int sf = BACKWARD ? S - 1 - step : step;
-    const int b = step % RING;
-    const uint32_t bar = tc::smem_addr(&s_bar[b]);
-    T *const dst = s_rec + b * kStage;
-    const long long slot0 = tile_base + (long long)sf * (TI * TJ);
-    tc::mbar_expect_tx(bar, kBlock + (DQB ? 5 * kRow : 0));
-    tc::bulk_load(tc::smem_addr(dst), crec + slot0 * CR_N, kBlock, bar);
-    if (DQB)
-#pragma unroll
-      for (int v = 0; v < 5; v++)
-        tc::bulk_load(tc::smem_addr(dst + TI * TJ * CR_N + v * TI * TJ), SweepPtrs<T>::dq(a)[v] + slot0, kRow, bar);
-  };
-  if (threadIdx.x == 0)
-    for (int r = 0; r < RING - 1 && r < S; r++) issue(r);
+  if (s_tile >= nti * ntj) return;
+  const int tile = a.order[BACKWARD ? nti * ntj - 1 - s_tile : s_tile];
+  const int ta = tile / ntj, tb = tile % ntj;
+  const int Nz = d.nz, S = sweep_steps(d);
+  const int ni = min(TI, d.nx - ta * TI), nj = min(TJ, d.ny - tb * TJ);   // rows and columns with cells
+  const int Se = Nz + nj - 1;                                              // steps of a row
   const int pa = BACKWARD ? ta + 1 : ta - 1, pb = BACKWARD ? tb + 1 : tb - 1;
-  const int tile_pa = pa * ntj + tb, tile_pb = ta * ntj + pb;
-  const bool halo_edge = BACKWARD ? (i == ie) : (i == 3);
-  const bool recv_x = !halo_edge && (BACKWARD ? il == TI - 1 : il == 0);
-  const bool recv_y = BACKWARD ? (jl == TJ - 1 || j == jn) : (jl == 0);
-  const bool wall_y = BACKWARD ? (j == jn) : (j == 2);
-  const bool send_x = BACKWARD ? (il == 0) : (il == TI - 1);
-  const bool send_y = BACKWARD ? (jl == 0) : (jl == TJ - 1);
-  // x hand-over inside the cluster: received from / sent to the neighbouring
-  // CTA's shared memory; at the cluster's ends through the global buffers
-  const bool dsm_recv = CL && ncl > 1 && (BACKWARD ? crank + 1 < ncl : crank > 0);
-  const bool dsm_send = CL && ncl > 1 && (BACKWARD ? crank > 0 : crank + 1 < ncl);
-  const uint32_t producer = BACKWARD ? crank + 1 : crank - 1, consumer = BACKWARD ? crank - 1 : crank + 1;
-  // the step q of the consumer's wait is the producer's step q + TI - 1
-  const int QN = S - TI + 1;   // hand-over steps per pass
-  constexpr uint32_t kPush = TJ * 5 * sizeof(T);   // bytes pushed per hand-over step (armed above for the first RX)
-  // the lanes that wait on the pushes: the tile's receiving edge, all of them
-  const bool wait_x = dsm_recv && (BACKWARD ? il == TI - 1 : il == 0);
-  const int push_polls = a.spin_limit > (0x7fffffff - kCopyPolls) / 64 ? 0x7fffffff : 64 * a.spin_limit + kCopyPolls;
-  const T rdx = (T)d.rdxi, rdy = (T)d.rdet, rdz = (T)d.rdzt, rdt = (T)(1.0 / d.dt);
-  T *xb = SweepPtrs<T>::xb(a), *yb = SweepPtrs<T>::yb(a);
-  T *const *dq = SweepPtrs<T>::dq(a);
-  T carry_z[5] = {0, 0, 0, 0, 0};
-
-  // hand-over values of the next PD steps, loaded ahead: a neighbouring
-  // tile runs just far enough ahead for its value to exist when needed, so
-  // a load issued then would wait one L2 round trip per step; loaded PD
-  // steps early it is usually there (a sentinel falls back to the bounded
-  // poll)
-  constexpr int PD = CGLI_SWEEP_PREFETCH;
-  auto kl_of = [&](int step) {
-    const int r = BACKWARD ? step - (TI - 1 - il) - (TJ - 1 - jl) : step - il - jl;
-    return (inside && r >= 0 && r < Nz) ? (BACKWARD ? Nz - 1 - r : r) : -1;
-  };
-  const T *xsrc = xb + ((long long)tile_pa * TJ + jl) * Nz * 5;
-  const T *ysrc = yb + ((long long)tile_pb * TI + il) * Nz * 5;
-  const bool pre_x = recv_x && !dsm_recv, pre_y = recv_y && !wall_y;
-  T px[PD][5], py[PD][5];
-  auto preload = [&](int step, T *qx, T *qy) {
-    const int k2 = kl_of(step);
-#pragma unroll
-    for (int v = 0; v < 5; v++) { qx[v] = (T)0; qy[v] = (T)0; }
-    if (k2 < 0) return;
-    if (pre_x)
-#pragma unroll
-      for (int v = 0; v < 5; v++) qx[v] = ld_gpu(xsrc + (long long)k2 * 5 + v);
-    if (pre_y)
-#pragma unroll
-      for (int v = 0; v < 5; v++) qy[v] = ld_gpu(ysrc + (long long)k2 * 5 + v);
-  };
-#pragma unroll
-  for (int p = 0; p < PD; p++) preload(p, px[p], py[p]);
-
-  // the periodic lagged halo of the slab's x edge: the x neighbour's product,
-  // formed before the pass (k_halo_products), loaded a step ahead by the
-  // edge lanes
-  T hx_cur[5], hx_nxt[5];
-  auto load_hx = [&](int step, T *out) {
-    const int k2 = kl_of(step);
-    if (k2 < 0) return;
-    const long long h = (long long)j * d.dj + 2 + k2;
-#pragma unroll
-    for (int v = 0; v < 5; v++) out[v] = SweepPtrs<T>::hxp(a)[v][h];
-  };
-  if (halo_edge) load_hx(0, hx_cur);
-  // this thread's slot of step s: slot0 + (forward step) * TI * TJ
-  const long long slot0 = tile_base + threadIdx.x;
-  const int rel0 = BACKWARD ? -(TI - 1 - il) - (TJ - 1 - jl) : -il - jl;
-
-  // unrolled twice: the ring and buffer indices of the two halves are
-  // constants, and the compiler overlaps the halves' independent work
-#pragma unroll 2
-  for (int s = 0; s < S; s++) {
-    const int rel = rel0 + s;
-    const int kl = BACKWARD ? Nz - 1 - rel : rel;
-    const bool active = inside && rel >= 0 && rel < Nz;
-    // the slot read in step s - 1 is free again (every receiving lane read it
-    // before the barrier that ended that step): arm it for its next use, then
-    // give it back to the producer
-    if (dsm_recv && threadIdx.x == 0 && s >= 1 && s - 1 < QN) {
-      if (s - 1 + RX < QN) tc::mbar_expect_tx(tc::smem_addr(&s_full[(s - 1) % RX]), kPush);
-      tc::mbar_arrive_cluster_relaxed(tc::mapa(tc::smem_addr(&s_empty[(s - 1) % RX]), producer));
-    }
-    // loads of the next cell go out first and land during the dependent part
-    // stage (s + RING - 1) % RING was last read at step s - 1, before the previous barrier
-    if (threadIdx.x == 0 && s + RING - 1 < S) issue(s + RING - 1);
-    if (halo_edge && s + 1 < S) load_hx(s + 1, hx_nxt);
-    // this step's records (bounded wait; a timeout is reported like a tile's)
-    if (!tc::mbar_wait(tc::smem_addr(&s_bar[s % RING]), (s / RING) & 1, kCopyPolls)) give_up(&s_dead, d.status);
-    // the cluster neighbour's push of this step (every receiving lane, so
-    // that every push has landed before the slot is re-armed or the CTA leaves)
-    if (wait_x && s < QN &&
-        !tc::mbar_wait_cluster(tc::smem_addr(&s_full[s % RX]), (s / RX) & 1, push_polls))
-      give_up(&s_dead, d.status);
-    // the record and MR (forward) or this cell's forward result (backward)
-    T rec[REC_N], mr[5];
-    if (active) {
-      const T *st = s_rec + (s % RING) * kStage;
-      load_cellrec(st + threadIdx.x * CR_N, (int)threadIdx.x, rec, BACKWARD ? (T *)nullptr : mr);
-      if (DQB)
-#pragma unroll
-        for (int v = 0; v < 5; v++) mr[v] = st[TI * TJ * CR_N + v * TI * TJ + threadIdx.x];
-    }
-    T ox[5];
-    if (active) {
-      const int pbuf = (s - 1) & 1;
-      T tx[5], ty[5];
-      if (halo_edge) {
-#pragma unroll
-        for (int v = 0; v < 5; v++) tx[v] = hx_cur[v];
-      } else if (!recv_x) {
-        const int sil = BACKWARD ? il + 1 : il - 1;
-#pragma unroll
-        for (int v = 0; v < 5; v++) tx[v] = sx[pbuf][sil][jl][v];
-      } else if (dsm_recv) {
-        // pushed by the producing CTA of the cluster (step s < QN here; the
-        // wait above has seen it land)
-        const T *src = s_rx + ((s % RX) * TJ + jl) * XW;
-#pragma unroll
-        for (int v = 0; v < 5; v++) tx[v] = src[v];
-      } else {
-        bool ok = true;
-#pragma unroll
-        for (int v = 0; v < 5; v++) { tx[v] = px[0][v]; ok = ok && !is_sentinel(px[0][v]); }
-        if (!ok) recv5<T>(xsrc + (long long)kl * 5, tx, d.status, a.spin_limit, &s_dead);
-      }
-      if (!recv_y) {
-        const int sjl = BACKWARD ? jl + 1 : jl - 1;
-#pragma unroll
-        for (int v = 0; v < 5; v++) ty[v] = sy[pbuf][il][sjl][v];
-      } else if (!wall_y) {
-        bool ok = true;
-#pragma unroll
-        for (int v = 0; v < 5; v++) { ty[v] = py[0][v]; ok = ok && !is_sentinel(py[0][v]); }
-        if (!ok) recv5<T>(ysrc + (long long)kl * 5, ty, d.status, a.spin_limit, &s_dead);
-      } else {
-#pragma unroll
-        for (int v = 0; v < 5; v++) ty[v] = 0;  // wall ghost row: dQ = 0 there
-      }
-      const bool zedge = rel == 0;             // z ghost row: dQ = 0 there
-      T L[5];
-#pragma unroll
-      for (int v = 0; v < 5; v++) L[v] = tx[v] * rdx + ty[v] * rdy + (zedge ? (T)0 : carry_z[v]) * rdz;
-      const T d11 = rec[R_D11], d22 = rec[R_D22], d51 = rec_d51<T>(rec, rdt);
-      T n[5];
-      if (!BACKWARD) {
-        // Dual_time_stepping.cpp:1289-1293
-        T r1 = mr[0] - L[0];
-        n[0] = d11 * r1;
-        n[1] = d22 * (mr[1] - L[1]);
-        n[2] = d22 * (mr[2] - L[2]);
-        n[3] = d22 * (mr[3] - L[3]);
-        n[4] = d51 * r1 + d22 * (mr[4] - L[4]);
-      } else {
-        // Dual_time_stepping.cpp:1651-1655 (mr holds this cell's forward result)
-        n[0] = mr[0] - d11 * L[0];
-        n[1] = mr[1] - d22 * L[1];
-        n[2] = mr[2] - d22 * L[2];
-        n[3] = mr[3] - d22 * L[3];
-        n[4] = mr[4] - (d51 * L[0] + d22 * L[4]);
-      }
-      const long long c = Met::kChannel ? 0 : ix(d, i, j, 2 + kl);
-      T mm[9];
-      Met::template dirs<T>(d, s_et, c, jl, mm);
-      T oy[5];
-      if (Met::kChannel) {
-        // the channel's face metrics have one nonzero component per
-        // direction (1, etdy, 1 on the x, y, z components), so only the
-        // nonzero split entries are formed and applied
-        channel_products<T, 0, BACKWARD>(rec, (T)1, n, ox);
-        channel_products<T, 1, BACKWARD>(rec, mm[4], n, oy);
-        channel_products<T, 2, BACKWARD>(rec, (T)1, n, carry_z);
-      } else {
-        Split<T> Ax = split_from_record<T>(rec, 0, mm[0], mm[1], mm[2]);
-        Split<T> Ay = split_from_record<T>(rec, 1, mm[3], mm[4], mm[5]);
-        Split<T> Az = split_from_record<T>(rec, 2, mm[6], mm[7], mm[8]);
-        if (BACKWARD) {
-          upper_terms<T>(Ax, n, ox);
-          upper_terms<T>(Ay, n, oy);
-          upper_terms<T>(Az, n, carry_z);
-        } else {
-          lower_terms<T>(Ax, n, ox);
-          lower_terms<T>(Ay, n, oy);
-          lower_terms<T>(Az, n, carry_z);
-        }
-      }
-      const int cb = s & 1;
-#pragma unroll
-      for (int v = 0; v < 5; v++) { sx[cb][il][jl][v] = ox[v]; sy[cb][il][jl][v] = oy[v]; }
-      if (send_x && !dsm_send) {
-        T *dst = xb + (((long long)tile * TJ + jl) * Nz + kl) * 5;
-#pragma unroll
-        for (int v = 0; v < 5; v++) __stcg(dst + v, ox[v]);
-      }
-      if (send_y) {
-        T *dst = yb + (((long long)tile * TI + il) * Nz + kl) * 5;
-#pragma unroll
-        for (int v = 0; v < 5; v++) __stcg(dst + v, oy[v]);
-      }
-      {
-#pragma unroll
-        for (int v = 0; v < 5; v++) dq[v][slot0 + (long long)(BACKWARD ? S - 1 - s : s) * (TI * TJ)] = n[v];
-        if (BACKWARD && !d.x_open) {
-          // lagged halos of the next sweep: plane ie feeds its forward pass,
-          // plane 3 its backward pass (an open slab's halos stay zero)
-          const long long h = (long long)j * d.dj + 2 + kl;
-          if (i == ie)
-            for (int v = 0; v < 5; v++) SweepPtrs<T>::hf(a)[v][h] = n[v];
-          if (i == 3)
-            for (int v = 0; v < 5; v++) SweepPtrs<T>::hb(a)[v][h] = n[v];
-        }
-      }
-    }
-    if (dsm_send && send_x && s >= TI - 1) {
-      const int q = s - (TI - 1);
-      // the slot's previous use must have been read by the consumer (after
-      // a give-up the push goes ahead regardless: its values are unused, and
-      // an early push only counts its bytes ahead on the consumer's next
-      // phase, which the consumer arms once it has seen the previous one)
-      const uint32_t eb = tc::smem_addr(&s_empty[q % RX]);
-      if (q >= RX && !tc::mbar_wait_cluster(eb, ((q / RX) - 1) & 1, 1) &&
-          !tc::mbar_wait_cluster(eb, ((q / RX) - 1) & 1, given_up(&s_dead, d.status) ? 0 : a.spin_limit))
-        give_up(&s_dead, d.status);
-      {
-        // every lane pushes its five words each step (zeros for a cell
-        // outside the slab), so the consumer's byte count always completes
-        T o5[5];
-#pragma unroll
-        for (int v = 0; v < 5; v++) o5[v] = active ? ox[v] : (T)0;
-        const uint32_t dst = tc::mapa(tc::smem_addr(s_rx + ((q % RX) * TJ + jl) * XW), consumer);
-        const uint32_t bar = tc::mapa(tc::smem_addr(&s_full[q % RX]), consumer);
-        if (sizeof(T) == 8) {
-          tc::st_async_v2(dst, (double)o5[0], (double)o5[1], bar);
-          tc::st_async_v2(dst + 16, (double)o5[2], (double)o5[3], bar);
-          tc::st_async(dst + 32, (double)o5[4], bar);
-        } else {
-          tc::st_async_v4(dst, (float)o5[0], (float)o5[1], (float)o5[2], (float)o5[3], bar);
-          tc::st_async(dst + 16, (float)o5[4], bar);
-        }
-      }
-    }
-    if (pre_x || pre_y) {
-#pragma unroll
-      for (int p = 0; p + 1 < PD; p++)
-#pragma unroll
-        for (int v = 0; v < 5; v++) { px[p][v] = px[p + 1][v]; py[p][v] = py[p + 1][v]; }
-      if (s + PD < S) preload(s + PD, px[PD - 1], py[PD - 1]);
-    }
-    if (halo_edge)
-#pragma unroll
-      for (int v = 0; v < 5; v++) hx_cur[v] = hx_nxt[v];
-    __syncthreads();
+  const bool halo = BACKWARD ? ta == nti - 1 : ta == 0;                    // the x products are the periodic halo's
+  const bool from_y = BACKWARD ? tb + 1 < ntj : tb > 0;
+  const int row0 = BACKWARD ? ni - 1 : 0;                                  // first row of the flow
+  const int polls = a.spin_limit > (1 << 28) ? 0x7fffffff : 4 * a.spin_limit + 4096;
+  T *const xbuf = a.buf<T>(a.xbuf), *const ybuf = a.buf<T>(a.ybuf);
+  if (threadIdx.x < TI * R) {
+    const int w = threadIdx.x / R, r = threadIdx.x % R;
+    tc::mbar_init(tc::smem_addr(&b_in[w][r]), from_y ? 2 : 1);
+    tc::mbar_init(tc::smem_addr(&b_done[w][r]), 1);
+    if (w == 0) tc::mbar_init(tc::smem_addr(&b_in[TI][r]), 1);
   }
-  // the cluster's CTAs leave together: none while another can still write
-  // into its shared memory
-  if (CL) tc::cluster_sync();
+  tc::mbar_fence_init();
+  __syncthreads();
+
+  if (warp == TI + XH) {
+    // ---- y helper: lane (row w, q) posts the receiving lane's values of
+    // the row's steps q, q + QY, ...; the steps past its last cell are empty
+    if (!from_y) return;
+    const int w = lane / (32 / TI), q = lane % (32 / TI);
+    int r = q, idle = 0;
+    T *const src = ybuf + ((long long)(ta * TI + w) * ntj + pb) * Nz * 5;
+    const bool mine = w < ni && q < QY;
+    while (__any_sync(0xffffffffu, mine && r < Se)) {
+      bool posted = false;
+      if (mine && r < Se) {
+        T *const p = src + (long long)(BACKWARD ? Nz - 1 - r : r) * 5;
+        T v5[5];
+        bool ok = true;
+        if (r < Nz)
+#pragma unroll
+          for (int v = 0; v < 5; v++) {
+            v5[v] = ld_gpu(p + v);
+            ok = ok && !is_sentinel(v5[v]);
+          }
+        const bool gone = !ok && given_up(&s_dead, d.status);
+        const bool room = r < R || tc::mbar_test(tc::smem_addr(&b_done[w][r % R]), ((r / R) - 1) & 1) || s_dead;
+        if ((ok || gone) && room) {
+          if (r < Nz) {
+            T *const dst = s_y + (w * R + r % R) * 8;
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+              dst[v] = v5[v];
+              if (ok) put_sentinel(p + v);
+            }
+          }
+          tc::mbar_arrive(tc::smem_addr(&b_in[w][r % R]));
+          r += QY;
+          idle = 0;
+          posted = true;
+        } else if (!ok) {
+          // (room is awaited without a count: the row empties its slots as
+          // long as its other inputs come, whose waits are counted)
+          if (idle++ >= a.spin_limit) give_up(&s_dead, d.status);
+        }
+      }
+      if (!__any_sync(0xffffffffu, posted)) __nanosleep(20);
+    }
+    return;
+  }
+  if (warp >= TI) {
+    // ---- x helper: every XH-th step of the first row's x products
+    T *const src = halo ? a.buf<T>(a.hx[BACKWARD]) + (long long)tb * S * (5 * TJ)
+                        : xbuf + ((long long)pa * ntj + tb) * S * (5 * TJ);
+    const int h = warp - TI;
+    bool active = false;
+    T v5[5] = {0, 0, 0, 0, 0};
+    auto fetch = [&](int s) {   // the lanes' values of step s, as they are now
+      const int k = (BACKWARD ? Se - 1 - s : s) - lane;
+      active = lane < nj && k >= 0 && k < Nz;
+      if (active)
+#pragma unroll
+        for (int v = 0; v < 5; v++) v5[v] = ld_gpu(src + (long long)(BACKWARD ? Se - 1 - s : s) * (5 * TJ) + v * TJ + lane);
+    };
+    auto missing = [&]() {
+      bool m = false;
+#pragma unroll
+      for (int v = 0; v < 5; v++) m = m || is_sentinel(v5[v]);
+      return active && !halo && m;
+    };
+    if (h < Se) fetch(h);
+    for (int s = h; s < Se; s += XH) {
+      for (int it = 0; __any_sync(0xffffffffu, missing()); it++) {
+        const bool stop = it >= a.spin_limit || given_up(&s_dead, d.status);
+        if (__any_sync(0xffffffffu, stop)) {
+          if (lane == 0) give_up(&s_dead, d.status);
+          break;
+        }
+        fetch(s);
+      }
+      if (s >= R) ring_wait(tc::smem_addr(&b_done[row0][s % R]), ((s / R) - 1) & 1, polls, &s_dead, d.status);
+      T *const dst = s_x + (row0 * R + s % R) * (5 * TJ) + lane;
+#pragma unroll
+      for (int v = 0; v < 5; v++) dst[v * TJ] = v5[v];
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(tc::smem_addr(&b_in[row0][s % R]));
+      if (active && !halo && !missing())
+#pragma unroll
+        for (int v = 0; v < 5; v++) put_sentinel(src + (long long)(BACKWARD ? Se - 1 - s : s) * (5 * TJ) + v * TJ + lane);
+      if (s + XH < Se) fetch(s + XH);   // under way while the other helpers post
+    }
+    return;
+  }
+  // ---- a row.  Its step is the serial chain of the pass, so it is kept to
+  // one wait for the products, the arithmetic, one store of the products and
+  // one arrival instruction (lane 0 on the receiving row's slot, lane 1 on
+  // its own); the records come by the lanes' own asynchronous copies, R steps
+  // ahead.  The loop is unrolled by the ring depth, so that every slot is a
+  // compile-time offset, and a group of steps in which every lane has a cell
+  // runs without the tests that the ramps need: at one warp per scheduler a
+  // branch costs as much as several arithmetic instructions.
+  const int w = warp;
+  if (w >= ni) return;
+  const int i = 3 + ta * TI + w, j = 2 + tb * TJ + lane, ie = d.nx + 2;
+  const bool next_row = BACKWARD ? w > 0 : w + 1 < ni;
+  const int dst_w = next_row ? (BACKWARD ? w - 1 : w + 1) : TI;     // the row that receives this row's x products
+  const bool send_x = !next_row && (BACKWARD ? ta > 0 : ta + 1 < nti);
+  const bool y_out = BACKWARD ? tb > 0 : tb + 1 < ntj;
+  const int recv_lane = BACKWARD ? nj - 1 : 0, send_lane = BACKWARD ? 0 : TJ - 1;
+  // the lane that holds this lane's j neighbour; the edge lane's neighbour is
+  // the wall ghost row (dQ = 0: weight 0) unless the y helper posts one
+  const int src_lane = lane == recv_lane ? lane : (BACKWARD ? min(lane + 1, TJ - 1) : max(lane - 1, 0));
+  const T rdx = (T)d.rdxi, rdz = (T)d.rdzt, rdt = (T)(1.0 / d.dt);
+  const T rdy = lane == recv_lane && !from_y ? (T)0 : (T)d.rdet;
+  const bool column = lane < nj;
+  const T et = Met::kChannel && column ? (T)a.etdytab[j] : (T)1;
+  const long long stream = (long long)(i - 3) * ntj + tb;
+  // the block of step s is sf = s or Se - 1 - s
+  constexpr int DIR = BACKWARD ? -1 : 1;
+  const int sf0 = BACKWARD ? Se - 1 : 0;
+  // dQ out: into the row's stream, or (first backward pass) only planes ie
+  // and 3, the lagged halos of the second sweep's passes (an open slab's stay
+  // zero)
+  const bool to_halo = BACKWARD && !last;
+  const bool store = !to_halo || (!d.x_open && (i == ie || i == 3));
+  T *dq = (to_halo ? a.buf<T>(a.halo[i == ie ? 0 : 1]) + (long long)tb * S * (5 * TJ)
+                   : a.buf<T>(a.dq) + stream * S * (5 * TJ)) + (long long)sf0 * (5 * TJ) + lane;
+  T *xout = xbuf + ((long long)ta * ntj + tb) * S * (5 * TJ) + (long long)sf0 * (5 * TJ) + lane;
+  T *const yout = ybuf + (stream * Nz + (BACKWARD ? Nz - 1 : 0)) * 5;
+  const T *const x_in = s_x + w * R * 5 * TJ + lane;
+  T *const x_out = s_x + dst_w * R * 5 * TJ + lane;
+  const T *const y_in = s_y + w * R * 8;
+  const T *const rec_in = s_rec + w * R * G::STAGE;
+  const uint32_t bar_in = tc::smem_addr(&b_in[w][0]), bar_dst = tc::smem_addr(&b_done[next_row ? dst_w : w][0]),
+                 bar_arrive = lane == 0 ? tc::smem_addr(&b_in[dst_w][0]) : tc::smem_addr(&b_done[w][0]);
+  // the copies of a step into its stage, one group: this lane's 16 bytes of
+  // every 512 of the step's blocks
+  constexpr int REC_B = G::REC * sizeof(T), DQ_B = 5 * TJ * sizeof(T), MET_B = 9 * TJ * sizeof(T);
+  const char *rec_src = (const char *)(a.buf<T>(a.cellrec) + stream * S * G::REC) + (long long)sf0 * REC_B + lane * 16;
+  const char *dq_src = (const char *)(a.buf<T>(a.dq) + stream * S * (5 * TJ)) + (long long)sf0 * DQ_B + lane * 16;
+  const char *met_src = nullptr;
+  if (!Met::kChannel) met_src = (const char *)(a.buf<T>(a.met) + stream * S * (9 * TJ)) + (long long)sf0 * MET_B + lane * 16;
+  const uint32_t stage0 = tc::smem_addr(rec_in) + lane * 16;
+  auto copy = [&](auto steady, int s, int stage) {   // called for s = 0, 1, 2, ...
+    if (decltype(steady)::value || s < Se) {
+      const uint32_t to = stage0 + stage * (uint32_t)(G::STAGE * sizeof(T));
+      if (decltype(steady)::value) {
+#pragma unroll
+        for (int o = 0; o < REC_B; o += 512) cp_async16(to + o, rec_src + o);
+      } else {
+        const int sf = BACKWARD ? Se - 1 - s : s, l0 = max(0, sf - Nz + 1), l1 = min(nj - 1, sf);   // lanes with a cell
+#pragma unroll
+        for (int o = 0; o < REC_B; o += 512) {
+          const int l = (o + lane * 16) / (int)(CR_N * sizeof(T));
+          if (l >= l0 && l <= l1) cp_async16(to + o, rec_src + o);
+        }
+      }
+      if (BACKWARD)
+#pragma unroll
+        for (int o = 0; o < DQ_B; o += 512)
+          if (o + 512 <= DQ_B || o + lane * 16 < DQ_B) cp_async16(to + REC_B + o, dq_src + o);
+      if (!Met::kChannel)
+#pragma unroll
+        for (int o = 0; o < MET_B; o += 512)
+          if (o + 512 <= MET_B || o + lane * 16 < MET_B)
+            cp_async16(to + G::DQ * (uint32_t)sizeof(T) + REC_B + o, met_src + o);
+      rec_src += DIR * REC_B;
+      if (BACKWARD) dq_src += DIR * DQ_B;
+      if (!Met::kChannel) met_src += DIR * MET_B;
+    }
+    cp_async_commit();
+  };
+  T rec[REC_N], mr[5], mm[Met::kChannel ? 1 : 9];
+  auto load = [&](int stage) {   // the oldest step under way, into registers
+    cp_async_wait<R - 1>();
+    __syncwarp();
+    const T *const st = rec_in + stage * G::STAGE;
+    load_cellrec(st + lane * CR_N, lane, rec, BACKWARD ? (T *)nullptr : mr);
+    if (BACKWARD)
+#pragma unroll
+      for (int v = 0; v < 5; v++) mr[v] = st[G::REC + v * TJ + lane];
+    if (!Met::kChannel)
+#pragma unroll
+      for (int v = 0; v < 9; v++) mm[v] = st[G::REC + G::DQ + v * TJ + lane];
+  };
+#pragma unroll
+  for (int u = 0; u < R; u++) copy(std::false_type(), u, u);
+  load(0);
+  T ty[5] = {0, 0, 0, 0, 0}, cz[5] = {0, 0, 0, 0, 0};
+  int kf = BACKWARD ? lane - (nj - 1) : -lane;    // the lane's cell, counted in the order of the pass
+  uint32_t parity = 0;                            // of the slots' current use
+  // one step; `steady`: every column has a cell at this step and R steps on
+  auto step = [&](auto steady, int s, int u) {
+    constexpr bool STEADY = decltype(steady)::value;
+    // lanes without a cell carry arbitrary values along, which reach no lane
+    // with a cell: an i, j or k neighbour without a cell is masked here or at
+    // the lane's edge
+    const bool active = STEADY ? column : column && (unsigned)kf < (unsigned)Nz;
+    ring_wait(bar_in + 8 * u, parity, polls, &s_dead, d.status);
+    T tx[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) tx[v] = x_in[(u * 5 + v) * TJ];
+    if (from_y && lane == recv_lane)
+#pragma unroll
+      for (int v = 0; v < 5; v++) ty[v] = y_in[u * 8 + v];
+    if (!STEADY && kf == 0)   // its z neighbour is the ghost row: dQ = 0
+#pragma unroll
+      for (int v = 0; v < 5; v++) cz[v] = (T)0;
+    T L[5];
+#pragma unroll
+    for (int v = 0; v < 5; v++) L[v] = fma_rn(cz[v], rdz, fma_rn(tx[v], rdx, mul_rn(ty[v], rdy)));
+    const T d11 = rec[R_D11], d22 = rec[R_D22], d51 = rec_d51<T>(rec, rdt);
+    T n[5];
+    if (!BACKWARD) {
+      // Dual_time_stepping.cpp:1289-1293
+      T r1 = mr[0] - L[0];
+      n[0] = d11 * r1;
+      n[1] = d22 * (mr[1] - L[1]);
+      n[2] = d22 * (mr[2] - L[2]);
+      n[3] = d22 * (mr[3] - L[3]);
+      n[4] = fma_rn(d22, mr[4] - L[4], mul_rn(d51, r1));
+    } else {
+      // Dual_time_stepping.cpp:1651-1655 (mr holds this cell's forward result)
+      n[0] = fma_rn(-d11, L[0], mr[0]);
+      n[1] = fma_rn(-d22, L[1], mr[1]);
+      n[2] = fma_rn(-d22, L[2], mr[2]);
+      n[3] = fma_rn(-d22, L[3], mr[3]);
+      n[4] = mr[4] - fma_rn(d22, L[4], mul_rn(d51, L[0]));
+    }
+    T ox[5], oy[5];
+    if (Met::kChannel) {
+      // the channel's face metrics have one nonzero component per direction
+      // (1, etdy, 1 on the x, y, z components), so only the nonzero split
+      // entries are formed and applied
+      channel_products<T, 0, BACKWARD>(rec, (T)1, n, ox);
+      channel_products<T, 1, BACKWARD>(rec, et, n, oy);
+      channel_products<T, 2, BACKWARD>(rec, (T)1, n, cz);
+    } else {
+      const Split<T> Ax = split_from_record<T>(rec, 0, mm[0], mm[1], mm[2]);
+      const Split<T> Ay = split_from_record<T>(rec, 1, mm[3], mm[4], mm[5]);
+      const Split<T> Az = split_from_record<T>(rec, 2, mm[6], mm[7], mm[8]);
+      if (BACKWARD) {
+        upper_terms<T>(Ax, n, ox);
+        upper_terms<T>(Ay, n, oy);
+        upper_terms<T>(Az, n, cz);
+      } else {
+        lower_terms<T>(Ax, n, ox);
+        lower_terms<T>(Ay, n, oy);
+        lower_terms<T>(Az, n, cz);
+      }
+    }
+    // hand the x products on (room is awaited for two steps at a time)
+    const int room = u % 2 ? -1 : min(u + 1, R - 1);
+    if (room >= 0 && next_row && (STEADY || s + (room - u) >= R))
+      ring_wait(bar_dst + 8 * room, parity ^ 1, polls, &s_dead, d.status);
+#pragma unroll
+    for (int v = 0; v < 5; v++) x_out[(u * 5 + v) * TJ] = ox[v];
+    if (send_x && active)
+#pragma unroll
+      for (int v = 0; v < 5; v++) __stcg(xout + v * TJ, ox[v]);
+    __syncwarp();
+    // every lane has read its inputs and written its products
+    if (lane < 2) tc::mbar_arrive(bar_arrive + 8 * u);
+#pragma unroll
+    for (int v = 0; v < 5; v++) ty[v] = __shfl_sync(0xffffffffu, oy[v], src_lane);
+    copy(steady, s + R, u);
+    if (store && active)
+#pragma unroll
+      for (int v = 0; v < 5; v++) dq[v * TJ] = n[v];
+    if (y_out && lane == send_lane && active)
+#pragma unroll
+      for (int v = 0; v < 5; v++) __stcg(yout + DIR * 5 * kf + v, oy[v]);
+    dq += DIR * 5 * TJ;
+    xout += DIR * 5 * TJ;
+    kf++;
+    if (STEADY || s + 1 < Se) load((u + 1) % R);
+  };
+  for (int s0 = 0; s0 < Se; s0 += R, parity ^= 1) {
+    if (s0 >= max(nj, R) && s0 + 2 * R <= Nz) {
+#pragma unroll
+      for (int u = 0; u < R; u++) step(std::true_type(), s0 + u, u);
+    } else {
+#pragma unroll
+      for (int u = 0; u < R; u++)
+        if (s0 + u < Se) step(std::false_type(), s0 + u, u);
+    }
+  }
 }
 
 // Dual_time_stepping.cpp:1702-1743 after the last backward pass: the
 // primitive update of every interior cell from its final dQ (read from the
-// tile-skewed layout), fully parallel rather than inside the wavefront's
-// chain of dependent steps, with per-block partial sums of the squared
-// increments (:1761-1776).  The divisions by q1, rho, T and J are
-// Newton-refined reciprocals (1/J from the table).
+// rows' streams), fully parallel rather than inside the wavefront's chain of
+// dependent steps, with per-block partial sums of the squared increments
+// (:1761-1776).  The divisions by q1, rho, T and J are Newton-refined
+// reciprocals (1/J from the table).
 //
-// A block owns one row il of one tile's TJ columns and UPD_KC consecutive k
-// of them.  In the tile-skewed layout those cells lie in UPD_KC + TJ - 1
-// consecutive steps, each holding the row's TJ slots side by side: the block
-// reads them whole (TJ consecutive words per step and variable) into shared
-// memory, then each warp updates 32 consecutive k of one column, so the
-// reads and writes of the state in the reference layout are coalesced too.
-constexpr int UPD_KC = 32;
-template <typename T>
-inline unsigned sweep_update_grid_x(const Dev &d) {
-  constexpr int TI = SweepTile<T>::TI, TJ = SweepTile<T>::TJ;
-  return (unsigned)(((d.nx + TI - 1) / TI) * ((d.ny + TJ - 1) / TJ) * TI);
-}
-template <typename T>
+// A block owns UPD_TJ columns of one row and UPD_KC consecutive k of them.
+// In the row's stream those cells lie in UPD_KC + UPD_TJ - 1 consecutive
+// steps, each holding the columns' values side by side: the block reads them
+// whole into shared memory, then each warp updates 32 consecutive k of one
+// column, so the reads and writes of the state in the reference layout are
+// coalesced too.
+constexpr int UPD_KC = 32, UPD_TJ = 16;
+inline unsigned sweep_update_grid_x(const Dev &d) { return (unsigned)(d.nx * ((d.ny + UPD_TJ - 1) / UPD_TJ)); }
 inline unsigned sweep_update_grid_y(const Dev &d) { return (unsigned)((d.nz + UPD_KC - 1) / UPD_KC); }
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_update_skewed(Dev d, SweepArgs a) {
-  constexpr int TI = SweepTile<T>::TI, TJ = SweepTile<T>::TJ;
-  constexpr int NS = UPD_KC + TJ - 1;   // steps holding the block's cells
-  static_assert(256 % TJ == 0 && TJ % 8 == 0, "row staging");
-  __shared__ T sdq[5][NS][TJ + 1];       // (+1: the update reads a column down the steps)
+  constexpr int NS = UPD_KC + UPD_TJ - 1;   // steps holding the block's cells
+  static_assert(SWEEP_TJ % UPD_TJ == 0 && 256 % UPD_TJ == 0, "column staging");
+  __shared__ T sdq[5][NS][UPD_TJ + 1];       // (+1: the update reads a column down the steps)
   // a wavefront pass that gave up left dQ incomplete: keep the state
   if (*(volatile int *)d.status) return;
-  const int ntj = (d.ny + TJ - 1) / TJ, S = d.nz + TI + TJ - 2;
-  const int tile = blockIdx.x / TI, il = blockIdx.x % TI;
-  const int ta = tile / ntj, tb = tile % ntj;
-  const int k0 = blockIdx.y * UPD_KC;    // first k of the block (0-based)
-  const int s0 = k0 + il;                // step of the cell (il, jl = 0, k0)
-  const long long base = (long long)tile * S * (TI * TJ) + il * TJ;
-  T *const *dq = SweepPtrs<T>::dq(a);
-  for (int e = threadIdx.x; e < NS * TJ; e += blockDim.x) {
-    const int ls = e / TJ, jl = e % TJ, st = s0 + ls;
+  const int ntu = (d.ny + UPD_TJ - 1) / UPD_TJ, S = sweep_steps(d);
+  const int row = blockIdx.x / ntu, j0 = blockIdx.x % ntu * UPD_TJ;   // 0-based row and first column
+  const int ntj = (d.ny + SWEEP_TJ - 1) / SWEEP_TJ, l0 = j0 % SWEEP_TJ;
+  const int k0 = blockIdx.y * UPD_KC;        // first k of the block (0-based)
+  const int s0 = k0 + l0;                    // step of the cell (first column, k0)
+  const T *const dq = a.buf<T>(a.dq) + ((long long)row * ntj + j0 / SWEEP_TJ) * S * (5 * SWEEP_TJ) + l0;
+  for (int e = threadIdx.x; e < NS * UPD_TJ; e += blockDim.x) {
+    const int ls = e / UPD_TJ, jl = e % UPD_TJ, st = s0 + ls;
     if (st < S) {
-      const long long g = base + (long long)st * (TI * TJ) + jl;
 #pragma unroll
-      for (int v = 0; v < 5; v++) sdq[v][ls][jl] = dq[v][g];
+      for (int v = 0; v < 5; v++) sdq[v][ls][jl] = dq[(long long)st * (5 * SWEEP_TJ) + v * SWEEP_TJ + jl];
     }
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int i = 3 + ta * TI + il;
+  const int i = 3 + row;
   double acc[5] = {0, 0, 0, 0, 0};
-  for (int jl = warp; jl < TJ; jl += nw) {
-    const int j = 2 + tb * TJ + jl, kl = k0 + lane;
-    if (i > d.nx + 2 || j > d.ny + 1 || kl >= d.nz) continue;
-    const int ls = lane + jl;            // step kl + il + jl, relative to s0
+  for (int jl = warp; jl < UPD_TJ; jl += nw) {
+    const int j = 2 + j0 + jl, kl = k0 + lane;
+    if (j > d.ny + 1 || kl >= d.nz) continue;
+    const int ls = lane + jl;            // step of the cell, relative to s0
     const long long c = ix(d, i, j, 2 + kl);
     const double J = d.J[c], iJ = d.iJ[c];
     const double q1 = d.U_[0][c], iq1 = nr_rcp(q1);
@@ -700,144 +685,54 @@ __global__ void __launch_bounds__(256) k_update_skewed(Dev d, SweepArgs a) {
 
 template <typename T>
 static void launch_update_skewed(const Dev &d, const SweepArgs &a, cudaStream_t s) {
-  k_update_skewed<T><<<dim3(sweep_update_grid_x<T>(d), sweep_update_grid_y<T>(d)), 256, 0, s>>>(d, a);
+  k_update_skewed<T><<<dim3(sweep_update_grid_x(d), sweep_update_grid_y(d)), 256, 0, s>>>(d, a);
 }
-int sweep_update_blocks(const Dev &d, bool mixed) {
-  return mixed ? (int)(sweep_update_grid_x<float>(d) * sweep_update_grid_y<float>(d))
-               : (int)(sweep_update_grid_x<double>(d) * sweep_update_grid_y<double>(d));
+int sweep_update_blocks(const Dev &d) { return (int)(sweep_update_grid_x(d) * sweep_update_grid_y(d)); }
+
+// tickets follow the step at which the wavefront reaches a tile, TI steps
+// per tile along x and 32 along y
+void sweep_tile_order(int nti, int ntj, int ti, std::vector<int> &order) {
+  order.resize((size_t)nti * ntj);
+  for (int t = 0; t < nti * ntj; t++) order[t] = t;
+  std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
+    return p / ntj * ti + p % ntj * SWEEP_TJ < q / ntj * ti + q % ntj * SWEEP_TJ;
+  });
 }
 
-// dynamic shared memory of a wavefront pass: the ring of record stages
-template <int TI, int TJ, typename T>
-constexpr int sweep_smem_bytes(bool backward, bool cluster) {
-  return SweepTile<T>::RING * TI * TJ * (CR_N + (backward ? 5 : 0)) * (int)sizeof(T) +
-         (cluster ? 8 * TJ * (sizeof(T) == 8 ? 6 : 8) * (int)sizeof(T) : 0);   // the cluster's x hand-over ring
+template <class Met, typename T>
+static void run_halo_products(const Dev &d, const SweepArgs &a, cudaStream_t s) {
+  k_halo_products<Met, T><<<dim3((d.nz + 63) / 64, d.ny, 2), 64, 0, s>>>(d, a);
+}
+template <class Met, typename T>
+static void run_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool backward, bool last) {
+  const int ntiles = sweep_tiles_x<T>(d.nx) * sweep_tiles_y(d.ny);
+  using F = SweepShape<T, !Met::kChannel, false>;
+  using B = SweepShape<T, !Met::kChannel, true>;
+  if (!backward) k_sweep<Met, false, T><<<ntiles, F::THREADS, F::SMEM, s>>>(d, a, last);
+  else k_sweep<Met, true, T><<<ntiles, B::THREADS, B::SMEM, s>>>(d, a, last);
+}
+// one symmetric sweep; its backward dQ is stored only when the update follows
+template <class Met, typename T>
+static void run_sweep(const Dev &d, const SweepArgs &a, cudaStream_t s, bool last) {
+  run_halo_products<Met, T>(d, a, s);
+  run_pass<Met, T>(d, a, s, false, last);
+  run_pass<Met, T>(d, a, s, true, last);
 }
 
-// tickets follow the anti-diagonals ta + tb of the tile grid
-void sweep_tile_order(int nti, int ntj, std::vector<int> &order) {
-  order.clear();
-  for (int dsum = 0; dsum <= nti + ntj - 2; dsum++)
-    for (int ta = 0; ta < nti; ta++) {
-      int tb = dsum - ta;
-      if (tb >= 0 && tb < ntj) order.push_back(ta * ntj + tb);
-    }
-}
+#define SWEEP_DISPATCH(fn, ...)                                        \
+  do {                                                                 \
+    if (mixed) {                                                       \
+      if (a.channel_metrics) fn<MetricsChannel, float>(__VA_ARGS__);   \
+      else fn<MetricsGeneral, float>(__VA_ARGS__);                     \
+    } else {                                                           \
+      if (a.channel_metrics) fn<MetricsChannel, double>(__VA_ARGS__);  \
+      else fn<MetricsGeneral, double>(__VA_ARGS__);                    \
+    }                                                                  \
+  } while (0)
 
-// One wavefront pass: ticket reset and sentinel fill of the hand-over
-// buffers, the halo products, then the pass itself (with the cluster
-// dimension a.cluster_x along x when it is above 1).
-template <int TI, int TJ, class Met, typename T>
-static void run_one_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool backward, bool final_pass) {
-  const int nti = (d.nx + TI - 1) / TI, ntj = (d.ny + TJ - 1) / TJ, ntiles = nti * ntj;
-  const size_t xbytes = (size_t)ntiles * TJ * d.nz * 5 * sizeof(T), ybytes = (size_t)ntiles * TI * d.nz * 5 * sizeof(T);
-  T *xb = sizeof(T) == 8 ? (T *)a.xbuf : (T *)a.xbuff;
-  T *yb = sizeof(T) == 8 ? (T *)a.ybuf : (T *)a.ybuff;
-  cudaMemsetAsync(a.ticket, 0, sizeof(unsigned int), s);
-  cudaMemsetAsync(xb, 0xff, xbytes, s);
-  cudaMemsetAsync(yb, 0xff, ybytes, s);
-  const dim3 hg((d.nz + 63) / 64, d.ny);
-  if (!backward) k_halo_products<Met, false, T><<<hg, 64, 0, s>>>(d, a);
-  else k_halo_products<Met, true, T><<<hg, 64, 0, s>>>(d, a);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ntiles);
-  cfg.blockDim = dim3(TI * TJ);
-  cfg.dynamicSmemBytes = sweep_smem_bytes<TI, TJ, T>(backward, a.cluster_x > 1);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  if (a.cluster_x > 1) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.cluster_x;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-  }
-  if (a.cluster_x > 1) {
-    if (!backward) cudaLaunchKernelEx(&cfg, k_sweep<TI, TJ, Met, false, T, true>, d, a);
-    else cudaLaunchKernelEx(&cfg, k_sweep<TI, TJ, Met, true, T, true>, d, a);
-  } else {
-    if (!backward) cudaLaunchKernelEx(&cfg, k_sweep<TI, TJ, Met, false, T, false>, d, a);
-    else cudaLaunchKernelEx(&cfg, k_sweep<TI, TJ, Met, true, T, false>, d, a);
-  }
-  if (final_pass) launch_update_skewed<T>(d, a, s);
-}
-
-template <int TI, int TJ, class Met, typename T>
-static void run_sweeps(const Dev &d, const SweepArgs &a, cudaStream_t s) {
-  for (int sweep = 0; sweep < 2; sweep++)
-    for (int pass = 0; pass < 2; pass++) run_one_pass<TI, TJ, Met, T>(d, a, s, pass == 1, false);
-}
-
-void launch_sweep_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed, bool backward, bool final_pass) {
-  if (mixed) {
-    if (a.channel_metrics) run_one_pass<F32::TI, F32::TJ, MetricsChannel, float>(d, a, s, backward, final_pass);
-    else run_one_pass<F32::TI, F32::TJ, MetricsGeneral, float>(d, a, s, backward, final_pass);
-  } else {
-    if (a.channel_metrics) run_one_pass<F64::TI, F64::TJ, MetricsChannel, double>(d, a, s, backward, final_pass);
-    else run_one_pass<F64::TI, F64::TJ, MetricsGeneral, double>(d, a, s, backward, final_pass);
-  }
-}
-
-// the wavefront kernels' shared memory (static products plus the dynamic
-// two-step record buffer) exceeds 48 KB: opt in once, outside any capture
-template <class Met, typename T, bool CL>
-static cudaError_t opt_in() {
-  constexpr int TI = SweepTile<T>::TI, TJ = SweepTile<T>::TJ;
-  cudaError_t e = cudaFuncSetAttribute(k_sweep<TI, TJ, Met, false, T, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       sweep_smem_bytes<TI, TJ, T>(false, CL));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sweep<TI, TJ, Met, true, T, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             sweep_smem_bytes<TI, TJ, T>(true, CL));
-  return e;
-}
-cudaError_t sweep_kernel_attributes() {
-  cudaError_t e = opt_in<MetricsChannel, double, false>();
-  if (e == cudaSuccess) e = opt_in<MetricsGeneral, double, false>();
-  if (e == cudaSuccess) e = opt_in<MetricsChannel, float, false>();
-  if (e == cudaSuccess) e = opt_in<MetricsGeneral, float, false>();
-  if (SweepTile<double>::CLUSTER_MAX > 1) {
-    if (e == cudaSuccess) e = opt_in<MetricsChannel, double, true>();
-    if (e == cudaSuccess) e = opt_in<MetricsGeneral, double, true>();
-  }
-  if (SweepTile<float>::CLUSTER_MAX > 1) {
-    if (e == cudaSuccess) e = opt_in<MetricsChannel, float, true>();
-    if (e == cudaSuccess) e = opt_in<MetricsGeneral, float, true>();
-  }
-  return e;
-}
-
-// The cluster size along x of the passes in type T for a grid of nti x ntj
-// tiles: the largest of CLUSTER_MAX, CLUSTER_MAX/2, ... (at least 2) that
-// divides nti and of which the device can hold at least one cluster of the
-// largest wavefront kernel; 1 (no clusters) otherwise.
-template <typename T>
-static int cluster_x_for(int nti, int ntj) {
-  constexpr int TI = SweepTile<T>::TI, TJ = SweepTile<T>::TJ;
-  for (int cx = SweepTile<T>::CLUSTER_MAX; cx >= 2; cx /= 2) {
-    if (nti % cx) continue;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nti * ntj);
-    cfg.blockDim = dim3(TI * TJ);
-    cfg.dynamicSmemBytes = sweep_smem_bytes<TI, TJ, T>(true, true);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cx;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_sweep<TI, TJ, MetricsGeneral, true, T, true>, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      continue;
-    }
-    if (n >= 1) return cx;
-  }
-  return 1;
-}
-int sweep_cluster_x(int nti, int ntj, bool mixed) {
-  return mixed ? cluster_x_for<float>(nti, ntj) : cluster_x_for<double>(nti, ntj);
+void launch_sweep_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed, bool backward, bool last) {
+  if (!backward) SWEEP_DISPATCH(run_halo_products, d, a, s);
+  SWEEP_DISPATCH(run_pass, d, a, s, backward, last);
 }
 
 void launch_sweep_update(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed) {
@@ -846,13 +741,25 @@ void launch_sweep_update(const Dev &d, const SweepArgs &a, cudaStream_t s, bool 
 }
 
 void launch_sweeps(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed) {
-  if (mixed) {
-    if (a.channel_metrics) run_sweeps<F32::TI, F32::TJ, MetricsChannel, float>(d, a, s);
-    else run_sweeps<F32::TI, F32::TJ, MetricsGeneral, float>(d, a, s);
-  } else {
-    if (a.channel_metrics) run_sweeps<F64::TI, F64::TJ, MetricsChannel, double>(d, a, s);
-    else run_sweeps<F64::TI, F64::TJ, MetricsGeneral, double>(d, a, s);
-  }
+  for (int sweep = 0; sweep < 2; sweep++) SWEEP_DISPATCH(run_sweep, d, a, s, sweep == 1);
+}
+
+// the wavefront kernels' rings exceed 48 KB: opt in once, outside any capture
+template <class Met, typename T>
+static cudaError_t opt_in() {
+  cudaError_t e = cudaFuncSetAttribute(k_sweep<Met, false, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       SweepShape<T, !Met::kChannel, false>::SMEM);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_sweep<Met, true, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SweepShape<T, !Met::kChannel, true>::SMEM);
+  return e;
+}
+cudaError_t sweep_kernel_attributes() {
+  cudaError_t e = opt_in<MetricsChannel, double>();
+  if (e == cudaSuccess) e = opt_in<MetricsGeneral, double>();
+  if (e == cudaSuccess) e = opt_in<MetricsChannel, float>();
+  if (e == cudaSuccess) e = opt_in<MetricsGeneral, float>();
+  return e;
 }
 
 }  // namespace cgli
