@@ -332,7 +332,7 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
     const bool mixed = p->precision == CGLI_MIXED;
     const size_t es = mixed ? sizeof(float) : sizeof(double);
     const size_t nsk = (size_t)cgli::skew_size(d), plane = (size_t)d.Y * d.Z;
-    // the wavefront's tile grid for this context's precision
+    // the wavefront's tile grid
     const int nti = mixed ? cgli::sweep_tiles_x<float>(p->nx) : cgli::sweep_tiles_x<double>(p->nx);
     const int ntj = cgli::sweep_tiles_y(p->ny);
     const size_t block = (size_t)cgli::sweep_steps(d) * 5 * cgli::SWEEP_TJ * es;   // one column block's five values, every step
@@ -356,17 +356,24 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
     if (rc == CGLI_OK) rc = alloc(c, sizeof(double) * d.Y, (void **)&et);
     a.Jtab = jt; a.etdytab = et;
     a.spin_limit = CGLI_WAIT_LIMIT_DEFAULT;
-    // the tickets' order of the tiles
-    std::vector<int> order;
-    cgli::sweep_tile_order(nti, ntj, mixed ? cgli::SweepTile<float>::TI : cgli::SweepTile<double>::TI, order);
-    int *dorder = nullptr;
-    if (rc == CGLI_OK) rc = alloc(c, sizeof(int) * order.size(), (void **)&dorder);
-    if (rc == CGLI_OK) cudaMemcpy(dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice);
-    a.order = dorder;
   }
   if (rc == CGLI_OK) {
     cudaError_t e = cgli::sweep_kernel_attributes();
     if (e != cudaSuccess) rc = fail(CGLI_ECUDA, std::string("sweep kernel attributes: ") + cudaGetErrorString(e));
+  }
+  if (rc == CGLI_OK) {
+    // the wavefront's clusters along x and the tickets' order of them
+    cgli::SweepArgs &a = c->sw;
+    const bool mixed = p->precision == CGLI_MIXED;
+    const int nti = mixed ? cgli::sweep_tiles_x<float>(p->nx) : cgli::sweep_tiles_x<double>(p->nx);
+    const int ti = mixed ? cgli::SweepTile<float>::TI : cgli::SweepTile<double>::TI;
+    a.cluster_x = cgli::sweep_cluster_x(nti, mixed);
+    std::vector<int> order;
+    cgli::sweep_tile_order((nti + a.cluster_x - 1) / a.cluster_x, cgli::sweep_tiles_y(p->ny), ti * a.cluster_x, order);
+    int *dorder = nullptr;
+    rc = alloc(c, sizeof(int) * order.size(), (void **)&dorder);
+    if (rc == CGLI_OK) cudaMemcpy(dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice);
+    a.order = dorder;
   }
   if (rc == CGLI_OK && cudaMallocHost(&c->h_norms, 16 * sizeof(double)) != cudaSuccess)
     rc = fail(CGLI_ENOMEM, "cudaMallocHost");

@@ -23,18 +23,15 @@ __host__ __device__ __forceinline__ int rec_vec_pos(int u, int t) {
 }
 
 // Wavefront geometry per arithmetic type of the passes: a CTA holds TI x rows
-// of SWEEP_TJ = 32 j columns (a warp per row, a lane per column); the steps of
-// records in flight per row on the channel grid and on general grids (what
-// shared memory holds).  TI = 4 with two CTAs per SM has faster steps but
-// twice the hand-overs between CTAs: 0.104 / 0.108 against 0.118 / 0.116 ms a
-// pass at 64^3, 0.55 / 0.53 against 0.49 / 0.46 at 256x192x192 (FP64).
+// of SWEEP_TJ = 32 j columns (a warp per row, a lane per column); the slots of
+// a row's rings, by which the rows' loop is unrolled (even).
 constexpr int SWEEP_TJ = 32;
 template <typename T> struct SweepTile;
 template <> struct SweepTile<double> {
-  static constexpr int TI = 8, TJ = SWEEP_TJ, RING = 4, RING_GENERAL = 3;
+  static constexpr int TI = 4, TJ = SWEEP_TJ, RING = 4;
 };
 template <> struct SweepTile<float> {
-  static constexpr int TI = 8, TJ = SWEEP_TJ, RING = 4, RING_GENERAL = 4;
+  static constexpr int TI = 4, TJ = SWEEP_TJ, RING = 4;
 };
 constexpr int CGLI_TIMEOUT_CODE = 6;
 
@@ -61,6 +58,7 @@ struct SweepArgs {
   const double *Jtab, *etdytab;   // per-j metrics of a grid uniform in x and z
   int channel_metrics;            // 1: use Jtab / etdytab instead of the 3-D arrays
   int spin_limit;                 // bounded wait (polls) for a neighbouring tile
+  int cluster_x;                  // wavefront CTAs per cluster along x
   template <typename T>
   __host__ __device__ __forceinline__ T *buf(void *p) const { return static_cast<T *>(p); }
 };
@@ -81,11 +79,13 @@ __host__ __device__ __forceinline__ long long halo_slot(const Dev &d, int j, int
   const int jl = (j - 2) % SWEEP_TJ;
   return ((long long)((j - 2) / SWEEP_TJ) * sweep_steps(d) + (k - 2) + jl) * (5 * SWEEP_TJ) + jl;
 }
-// tiles of the wavefront in x and y for the passes in type T
+// tiles of the wavefront in x and y
 template <typename T> inline int sweep_tiles_x(int nx) { return (nx + SweepTile<T>::TI - 1) / SweepTile<T>::TI; }
 inline int sweep_tiles_y(int ny) { return (ny + SWEEP_TJ - 1) / SWEEP_TJ; }
 
-void sweep_tile_order(int nti, int ntj, int ti, std::vector<int> &order);
+void sweep_tile_order(int ncx, int ntj, int rows, std::vector<int> &order);
+// CTAs per cluster along x of the passes over nti x tiles
+int sweep_cluster_x(int nti, bool mixed);
 // shared-memory opt-in of the wavefront kernels (once per process and device)
 cudaError_t sweep_kernel_attributes();
 // a.met from the metrics of every interior cell

@@ -19,30 +19,40 @@
 // chain runs at the latency of one warp's step (load the slot, about ten
 // dependent FP64 operations, store the slot) and slower warps are absorbed
 // by the rings.
-// Measured (ms per forward / backward pass): 256x192x192 FP64 0.49 / 0.46,
+// Measured (ms per forward / backward pass): 256x192x192 FP64 0.46 / 0.44,
 // FP32 0.36 / 0.35 (a tile of 16x16 or 8x16 columns with one thread per column
-// and a block barrier per step: 0.96 / 0.95 and 0.79 / 0.92); 64^3 FP64 0.118
-// / 0.115 (0.248 / 0.242).  One CTA alone takes 0.55 us per step in FP64 (0.83
-// before), 0.37 with four rows instead of eight: at eight rows, two warps per
-// scheduler, the shared-memory traffic of the steps (about 110 wavefronts a
-// row) adds up.
+// and a block barrier per step: 0.96 / 0.95 and 0.79 / 0.92); 64^3 FP64 0.084
+// / 0.082 (0.248 / 0.242).  One CTA alone takes 0.36 us per step in FP64 (0.83
+// before).
 //
-// A CTA holds TI rows (one warp each) of one 32-column block plus helper
-// warps that bring in what the rows read: XH warps fetch the x products of
-// the row before the CTA's first one (each every XH-th step, so XH round
-// trips to L2 are in flight), one warp fetches the y products of the
-// neighbouring column block for every row (a few lanes per row, each every
-// QY-th step).  They post into the same rings the rows use among themselves,
-// so the rows have no special cases; the slab's periodic x halo comes through
-// the x helpers as well (products formed by k_halo_products).
+// A CTA holds TI = 4 rows (one warp per scheduler) of one 32-column block plus
+// helper warps: XH x helpers fetch the x products of the row before the CTA's
+// first one (each every XH-th step, so XH round trips to L2 are in flight; with
+// two of them they set the pace of the FP32 passes), the y helper fetches the y
+// products of the neighbouring column block for every row (a few lanes per
+// row, each every QY-th step), the sender passes on what the last row posts.
+// All post into the same rings the rows use among themselves, so the rows have
+// no special cases; the slab's periodic x halo comes through the x helpers as
+// well (products formed by k_halo_products).  Eight rows per CTA, two warps per
+// scheduler, take 0.55 us per step: the shared-memory traffic of the steps
+// (about 100 wavefronts a row) fills the load / store pipe; at 64^3 that made
+// a pass 0.12 ms, at 256x192x192 0.51 / 0.49.
+//
+// Up to eight CTAs along x form a cluster.  Inside it the sender pushes the x
+// products into the next CTA's ring with st.async, which counts the bytes on
+// that slot's mbarrier; the receiving CTA arms the slot and returns the room
+// (the receiver, a warp that takes an x helper's place).  That hop takes about
+// 0.3 us; through L2 (clusters' ends, and everything along y) 1.2-1.5 us,
+// which cost 0.10 against 0.084 ms a pass at 64^3.
 //
 // Storage.  Everything the sweeps read per cell -- the split-Jacobian /
 // diagonal record with the residual MR, and dQ -- lives in per-row streams
 // in the order the rows visit it: block (row, column block, forward step) of
 // 32 slots.  A row's block of one step arrives by asynchronous copies of the
 // row's own lanes, issued R steps ahead into the row's ring (only the lanes
-// with a cell at that step are copied).  The residual kernel writes the records, the final
-// update reads dQ; only these two touch the reference layout.
+// with a cell at that step are copied).  The residual kernel writes the
+// records, the final update reads dQ; only these two touch the reference
+// layout.
 //
 // Hand-over between CTAs.  Products cross through global buffers that hold a
 // sentinel bit pattern wherever no value is waiting; the consumer polls the
@@ -54,9 +64,10 @@
 // it records the timeout code in the status word and posts what it has, so
 // that every warp runs to the end of the pass without waiting, computing
 // values nobody will use; the ring waits inside a CTA follow the dead flag
-// too.  The update kernel then leaves the state alone, the host reports CGLI_ETIMEOUT and refills the
+// too (but not those on pushed products, push_wait).  The update kernel then
+// leaves the state alone, the host reports CGLI_ETIMEOUT and refills the
 // buffers with the sentinel.
-// CTAs take tickets in the order in which the wavefront reaches their tiles,
+// Clusters take tickets in the order in which the wavefront reaches them,
 // where every dependency holds a smaller ticket, so a waiting CTA only ever
 // waits on CTAs that are already running.
 //
@@ -107,13 +118,29 @@ __device__ __forceinline__ void put_sentinel(double *p) { *p = __longlong_as_dou
 __device__ __forceinline__ void put_sentinel(float *p) { *p = __int_as_float(-1); }
 
 // a wait on another tile has given up somewhere: this CTA's dead flag or
-// the grid's status word
+// the grid's status word (a trip to L2: polls look there now and then only)
 __device__ __forceinline__ bool given_up(const volatile int *dead, const int *status) {
   return *dead || *(const volatile int *)status;
 }
 __device__ __forceinline__ void give_up(volatile int *dead, int *status) {
   atomicExch(status, CGLI_TIMEOUT_CODE);
   *dead = 1;
+}
+
+// Wait on a slot that counts pushed bytes, on the room for a push, and of the
+// sender and the row before it.  These do not follow the dead flag: the other
+// end always goes on (it is co-scheduled, and its own inputs come or are given
+// up), every byte must have landed before the CTA ends, and a slot armed or
+// filled ahead of its phase would leave the barrier's counts wrong.  The count
+// bounds the wait against a failing device only.
+constexpr int PUSH_POLLS = 1 << 26;
+__device__ __noinline__ void push_wait_slow(uint32_t bar, uint32_t parity, volatile int *dead, int *status) {
+  for (int n = 0; n < PUSH_POLLS; n++)
+    if (tc::mbar_try(bar, parity)) return;
+  give_up(dead, status);
+}
+__device__ __forceinline__ void push_wait(uint32_t bar, uint32_t parity, volatile int *dead, int *status) {
+  if (!tc::mbar_try(bar, parity)) push_wait_slow(bar, parity, dead, status);
 }
 
 // a thread's 16-byte asynchronous copy into shared memory (not kept in L1)
@@ -263,15 +290,16 @@ __device__ __forceinline__ void channel_products(const T r[REC_N], T m, const T 
   o[4] = fma_rn(p22, n[4], fma_rn(p51, n[0], mul_rn(p5q, n[q])));
 }
 
-// Geometry of a pass: TI row warps, XH x helpers and one y helper per CTA.
+// Geometry of a pass: TI row warps, XH x helpers, the sender and the y helper
+// per CTA.
 // R: slots of a row's rings (x products, y products, records), so steps of
 // records on their way into shared memory.
 constexpr int SWEEP_XH = 3;
 template <typename T, bool GEN, bool BACKWARD>
 struct SweepShape {
   static constexpr int TI = SweepTile<T>::TI, TJ = SWEEP_TJ;
-  static constexpr int R = GEN ? SweepTile<T>::RING_GENERAL : SweepTile<T>::RING;
-  static constexpr int THREADS = 32 * (TI + SWEEP_XH + 1);
+  static constexpr int R = SweepTile<T>::RING;
+  static constexpr int THREADS = 32 * (TI + SWEEP_XH + 2);
   static constexpr int QY = 32 / TI < R ? 32 / TI : R;   // y helper lanes per row
   // words of one ring stage: 32 slots, the forward result (backward pass),
   // the metric terms (general grids)
@@ -282,8 +310,8 @@ struct SweepShape {
   static_assert(32 % TI == 0, "helper lanes per row");
   // a producer that takes every n-th step must not run two uses of a slot
   // ahead of the row (the parity of a phase would be ambiguous): n <= R
-  static_assert(SWEEP_XH <= R && QY <= R, "ring depth");
-  static_assert(SMEM + 8 * (TI + 1) * R * 2 + 64 <= 227 * 1024, "shared memory of a pass");
+  static_assert(SWEEP_XH <= R && QY <= R && R % 2 == 0, "ring depth");
+  static_assert(SMEM + 8 * (TI + 2) * R * 2 + 64 <= 227 * 1024, "shared memory of a pass");
 };
 
 template <class Met, bool BACKWARD, typename T>
@@ -296,39 +324,54 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
   T *const s_x = s_rec + TI * R * G::STAGE;                  // [TI + 1][R][5][TJ]
   T *const s_y = s_x + (TI + 1) * R * 5 * TJ;                // [TI][R][8]
   // per row and slot: the step's x (and y) products are posted; the row is
-  // done with them.  Row TI stands for no row: the last row of the flow posts
-  // there what nobody reads, so that all rows run the same instructions.
-  __shared__ __align__(8) uint64_t b_in[TI + 1][R], b_done[TI][R];
-  __shared__ int s_tile, s_dead;
+  // done with them.  Row TI is the sender, so that all rows run the same
+  // instructions.  b_room: the next CTA of the cluster is done with the slot
+  // of its first row
+  __shared__ __align__(8) uint64_t b_in[TI + 1][R], b_done[TI + 1][R], b_room[R];
+  __shared__ int s_ticket, s_dead, s_never;   // (s_never stays 0)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nti = (d.nx + TI - 1) / TI, ntj = (d.ny + TJ - 1) / TJ;
+  // one ticket per cluster of consecutive x tiles, taken by its first CTA
+  const int cx = (int)tc::cluster_nctarank(), rank = (int)tc::cluster_ctarank();
+  const int units = (nti + cx - 1) / cx * ntj;
   if (threadIdx.x == 0) {
-    s_tile = (int)atomicAdd(a.ticket + (BACKWARD ? 1 : 0), 1u);
-    s_dead = 0;
+    s_dead = s_never = 0;
+    if (rank == 0) s_ticket = (int)atomicAdd(a.ticket + (BACKWARD ? 1 : 0), 1u);
   }
-  __syncthreads();
-  if (s_tile >= nti * ntj) return;
-  const int tile = a.order[BACKWARD ? nti * ntj - 1 - s_tile : s_tile];
-  const int ta = tile / ntj, tb = tile % ntj;
+  tc::cluster_sync();
+  const int ticket = (int)tc::ld_cluster_u32(tc::mapa(tc::smem_addr(&s_ticket), 0));
+  const int unit = a.order[BACKWARD ? units - 1 - ticket : ticket];
+  const int ta = unit / ntj * cx + rank, tb = unit % ntj;
   const int Nz = d.nz, S = sweep_steps(d);
   const int ni = min(TI, d.nx - ta * TI), nj = min(TJ, d.ny - tb * TJ);   // rows and columns with cells
   const int Se = Nz + nj - 1;                                              // steps of a row
   const int pa = BACKWARD ? ta + 1 : ta - 1, pb = BACKWARD ? tb + 1 : tb - 1;
   const bool halo = BACKWARD ? ta == nti - 1 : ta == 0;                    // the x products are the periodic halo's
   const bool from_y = BACKWARD ? tb + 1 < ntj : tb > 0;
+  // x products from / to the neighbouring CTA of the cluster
+  const bool pushed = !halo && (BACKWARD ? rank + 1 < cx : rank > 0);
+  const bool push = BACKWARD ? rank > 0 : rank + 1 < cx && ta + 1 < nti;
   const int row0 = BACKWARD ? ni - 1 : 0;                                  // first row of the flow
   const int polls = a.spin_limit > (1 << 28) ? 0x7fffffff : 4 * a.spin_limit + 4096;
+  constexpr uint32_t PUSH_B = 5 * TJ * sizeof(T);
   T *const xbuf = a.buf<T>(a.xbuf), *const ybuf = a.buf<T>(a.ybuf);
   if (threadIdx.x < TI * R) {
     const int w = threadIdx.x / R, r = threadIdx.x % R;
     tc::mbar_init(tc::smem_addr(&b_in[w][r]), from_y ? 2 : 1);
     tc::mbar_init(tc::smem_addr(&b_done[w][r]), 1);
-    if (w == 0) tc::mbar_init(tc::smem_addr(&b_in[TI][r]), 1);
+    if (w == 0) {
+      tc::mbar_init(tc::smem_addr(&b_in[TI][r]), 1);
+      tc::mbar_init(tc::smem_addr(&b_done[TI][r]), 1);
+      tc::mbar_init(tc::smem_addr(&b_room[r]), 1);
+    }
+    // pushed products count their bytes on the slot; the row arms it
+    if (pushed && w == row0 && r < Se) tc::mbar_expect_tx(tc::smem_addr(&b_in[w][r]), PUSH_B);
   }
   tc::mbar_fence_init();
-  __syncthreads();
+  tc::cluster_sync();
+  if (ta >= nti) return;
 
-  if (warp == TI + XH) {
+  if (warp == TI + XH + 1) {
     // ---- y helper: lane (row w, q) posts the receiving lane's values of
     // the row's steps q, q + QY, ...; the steps past its last cell are empty
     if (!from_y) return;
@@ -348,8 +391,12 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
             v5[v] = ld_gpu(p + v);
             ok = ok && !is_sentinel(v5[v]);
           }
-        const bool gone = !ok && given_up(&s_dead, d.status);
-        const bool room = r < R || tc::mbar_test(tc::smem_addr(&b_done[w][r % R]), ((r / R) - 1) & 1) || s_dead;
+        const bool gone = !ok && (*(volatile int *)&s_dead || (idle % 16 == 15 && given_up(&s_dead, d.status)));
+        // (once the CTA has given up, its rows no longer wait, and neither
+        // does this; but a row with pushed products goes on waiting, and its
+        // slots, which count bytes, must not be posted ahead of it)
+        const bool room = r < R || tc::mbar_test(tc::smem_addr(&b_done[w][r % R]), ((r / R) - 1) & 1) ||
+                          (*(volatile int *)&s_dead && !(pushed && w == row0));
         if ((ok || gone) && room) {
           if (r < Nz) {
             T *const dst = s_y + (w * R + r % R) * 8;
@@ -373,8 +420,58 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
     }
     return;
   }
+  if (warp == TI + XH) {
+    // ---- sender: the last row's x products, to the next CTA of the cluster
+    // (pushed into its first row's slots, every lane's, so that the bytes
+    // are always the same), to the next cluster's through the global buffer,
+    // or (the end of the slab) nowhere
+    const bool send = !push && (BACKWARD ? ta > 0 : ta + 1 < nti);
+    const int up = BACKWARD ? rank - 1 : rank + 1, up_row0 = BACKWARD ? TI - 1 : 0;   // (backward, it is a whole CTA)
+    const uint32_t to = push ? tc::mapa(tc::smem_addr(s_x + up_row0 * R * 5 * TJ + lane), up) : 0,
+                   to_bar = push ? tc::mapa(tc::smem_addr(&b_in[up_row0][0]), up) : 0;
+    T *const out = xbuf + ((long long)ta * ntj + tb) * S * (5 * TJ) + lane;
+    for (int s = 0; s < Se; s++) {
+      const int u = s % R;
+      const uint32_t ph = (s / R) & 1;
+      push_wait(tc::smem_addr(&b_in[TI][u]), ph, &s_dead, d.status);
+      T v5[5];
+#pragma unroll
+      for (int v = 0; v < 5; v++) v5[v] = s_x[(TI * R + u) * (5 * TJ) + v * TJ + lane];
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(tc::smem_addr(&b_done[TI][u]));
+      if (push) {
+        if (s >= R) push_wait(tc::smem_addr(&b_room[u]), ph ^ 1, &s_dead, d.status);
+#pragma unroll
+        for (int v = 0; v < 5; v++) tc::st_async(to + (u * 5 + v) * (uint32_t)(TJ * sizeof(T)), v5[v], to_bar + 8 * u);
+      } else if (send) {
+        const int sf = BACKWARD ? Se - 1 - s : s, k = sf - lane;
+        if (lane < nj && k >= 0 && k < Nz)
+#pragma unroll
+          for (int v = 0; v < 5; v++) __stcg(out + (long long)sf * (5 * TJ) + v * TJ, v5[v]);
+      }
+    }
+    if (cx > 1) tc::cluster_sync();
+    return;
+  }
+  if (warp == TI && pushed) {
+    // ---- receiver: arms the first row's slots for the products pushed into
+    // them and returns the room
+    if (lane == 0) {
+      const uint32_t room = tc::mapa(tc::smem_addr(&b_room[0]), BACKWARD ? rank + 1 : rank - 1);
+      for (int s = 0; s + R < Se; s++) {
+        const int u = s % R;
+        push_wait(tc::smem_addr(&b_done[row0][u]), (s / R) & 1, &s_dead, d.status);
+        tc::mbar_expect_tx(tc::smem_addr(&b_in[row0][u]), PUSH_B);
+        tc::mbar_arrive_cluster_relaxed(room + 8 * u);
+      }
+    }
+    __syncwarp();
+    tc::cluster_sync();
+    return;
+  }
   if (warp >= TI) {
     // ---- x helper: every XH-th step of the first row's x products
+    if (pushed) return;
     T *const src = halo ? a.buf<T>(a.hx[BACKWARD]) + (long long)tb * S * (5 * TJ)
                         : xbuf + ((long long)pa * ntj + tb) * S * (5 * TJ);
     const int h = warp - TI;
@@ -396,8 +493,7 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
     if (h < Se) fetch(h);
     for (int s = h; s < Se; s += XH) {
       for (int it = 0; __any_sync(0xffffffffu, missing()); it++) {
-        const bool stop = it >= a.spin_limit || given_up(&s_dead, d.status);
-        if (__any_sync(0xffffffffu, stop)) {
+        if (it >= a.spin_limit || (it % 16 == 15 && given_up(&s_dead, d.status))) {
           if (lane == 0) give_up(&s_dead, d.status);
           break;
         }
@@ -429,7 +525,11 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
   const int i = 3 + ta * TI + w, j = 2 + tb * TJ + lane, ie = d.nx + 2;
   const bool next_row = BACKWARD ? w > 0 : w + 1 < ni;
   const int dst_w = next_row ? (BACKWARD ? w - 1 : w + 1) : TI;     // the row that receives this row's x products
-  const bool send_x = !next_row && (BACKWARD ? ta > 0 : ta + 1 < nti);
+  // what lets a wait end early: the dead flag; but not for slots that count
+  // pushed bytes, and not ahead of the sender (see push_wait)
+  volatile int *const dead_in = pushed && w == row0 ? &s_never : &s_dead;
+  volatile int *const dead_out = next_row ? &s_dead : &s_never;
+  const int polls_in = pushed && w == row0 ? PUSH_POLLS : polls, polls_out = next_row ? polls : PUSH_POLLS;
   const bool y_out = BACKWARD ? tb > 0 : tb + 1 < ntj;
   const int recv_lane = BACKWARD ? nj - 1 : 0, send_lane = BACKWARD ? 0 : TJ - 1;
   // the lane that holds this lane's j neighbour; the edge lane's neighbour is
@@ -450,13 +550,12 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
   const bool store = !to_halo || (!d.x_open && (i == ie || i == 3));
   T *dq = (to_halo ? a.buf<T>(a.halo[i == ie ? 0 : 1]) + (long long)tb * S * (5 * TJ)
                    : a.buf<T>(a.dq) + stream * S * (5 * TJ)) + (long long)sf0 * (5 * TJ) + lane;
-  T *xout = xbuf + ((long long)ta * ntj + tb) * S * (5 * TJ) + (long long)sf0 * (5 * TJ) + lane;
   T *const yout = ybuf + (stream * Nz + (BACKWARD ? Nz - 1 : 0)) * 5;
   const T *const x_in = s_x + w * R * 5 * TJ + lane;
   T *const x_out = s_x + dst_w * R * 5 * TJ + lane;
   const T *const y_in = s_y + w * R * 8;
   const T *const rec_in = s_rec + w * R * G::STAGE;
-  const uint32_t bar_in = tc::smem_addr(&b_in[w][0]), bar_dst = tc::smem_addr(&b_done[next_row ? dst_w : w][0]),
+  const uint32_t bar_in = tc::smem_addr(&b_in[w][0]), bar_dst = tc::smem_addr(&b_done[dst_w][0]),
                  bar_arrive = lane == 0 ? tc::smem_addr(&b_in[dst_w][0]) : tc::smem_addr(&b_done[w][0]);
   // the copies of a step into its stage, one group: this lane's 16 bytes of
   // every 512 of the step's blocks
@@ -521,7 +620,7 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
     // with a cell: an i, j or k neighbour without a cell is masked here or at
     // the lane's edge
     const bool active = STEADY ? column : column && (unsigned)kf < (unsigned)Nz;
-    ring_wait(bar_in + 8 * u, parity, polls, &s_dead, d.status);
+    ring_wait(bar_in + 8 * u, parity, polls_in, dead_in, d.status);
     T tx[5];
 #pragma unroll
     for (int v = 0; v < 5; v++) tx[v] = x_in[(u * 5 + v) * TJ];
@@ -575,14 +674,10 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
       }
     }
     // hand the x products on (room is awaited for two steps at a time)
-    const int room = u % 2 ? -1 : min(u + 1, R - 1);
-    if (room >= 0 && next_row && (STEADY || s + (room - u) >= R))
-      ring_wait(bar_dst + 8 * room, parity ^ 1, polls, &s_dead, d.status);
+    if (u % 2 == 0 && (STEADY || s + 1 >= R))
+      ring_wait(bar_dst + 8 * (u + 1), parity ^ 1, polls_out, dead_out, d.status);
 #pragma unroll
     for (int v = 0; v < 5; v++) x_out[(u * 5 + v) * TJ] = ox[v];
-    if (send_x && active)
-#pragma unroll
-      for (int v = 0; v < 5; v++) __stcg(xout + v * TJ, ox[v]);
     __syncwarp();
     // every lane has read its inputs and written its products
     if (lane < 2) tc::mbar_arrive(bar_arrive + 8 * u);
@@ -596,7 +691,6 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
 #pragma unroll
       for (int v = 0; v < 5; v++) __stcg(yout + DIR * 5 * kf + v, oy[v]);
     dq += DIR * 5 * TJ;
-    xout += DIR * 5 * TJ;
     kf++;
     if (STEADY || s + 1 < Se) load((u + 1) % R);
   };
@@ -610,6 +704,8 @@ __global__ void __launch_bounds__(SweepShape<T, !Met::kChannel, BACKWARD>::THREA
         if (s0 + u < Se) step(std::false_type(), s0 + u, u);
     }
   }
+  // a CTA stays until its neighbours have sent it their last signals
+  if (cx > 1) tc::cluster_sync();
 }
 
 // Dual_time_stepping.cpp:1702-1743 after the last backward pass: the
@@ -689,15 +785,41 @@ static void launch_update_skewed(const Dev &d, const SweepArgs &a, cudaStream_t 
 }
 int sweep_update_blocks(const Dev &d) { return (int)(sweep_update_grid_x(d) * sweep_update_grid_y(d)); }
 
-// tickets follow the step at which the wavefront reaches a tile, TI steps
-// per tile along x and 32 along y
-void sweep_tile_order(int nti, int ntj, int ti, std::vector<int> &order) {
-  order.resize((size_t)nti * ntj);
-  for (int t = 0; t < nti * ntj; t++) order[t] = t;
+// tickets follow the step at which the wavefront reaches a cluster, `rows`
+// steps per cluster along x and 32 per column block along y
+void sweep_tile_order(int ncx, int ntj, int rows, std::vector<int> &order) {
+  order.resize((size_t)ncx * ntj);
+  for (int t = 0; t < ncx * ntj; t++) order[t] = t;
   std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
-    return p / ntj * ti + p % ntj * SWEEP_TJ < q / ntj * ti + q % ntj * SWEEP_TJ;
+    return p / ntj * rows + p % ntj * SWEEP_TJ < q / ntj * rows + q % ntj * SWEEP_TJ;
   });
 }
+
+// CTAs per cluster along x for nti tiles: enough for all of them, at most 8,
+// if the device holds such a cluster of the largest wavefront kernel
+template <typename T>
+static int cluster_x_for(int nti) {
+  using B = SweepShape<T, true, true>;
+  int cx = 1;
+  while (cx < 8 && cx < nti) cx *= 2;
+  for (; cx > 1; cx /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cx);
+    cfg.blockDim = dim3(B::THREADS);
+    cfg.dynamicSmemBytes = B::SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cx;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_sweep<MetricsGeneral, true, T>, &cfg) == cudaSuccess && n >= 1) return cx;
+    cudaGetLastError();
+  }
+  return 1;
+}
+int sweep_cluster_x(int nti, bool mixed) { return mixed ? cluster_x_for<float>(nti) : cluster_x_for<double>(nti); }
 
 template <class Met, typename T>
 static void run_halo_products(const Dev &d, const SweepArgs &a, cudaStream_t s) {
@@ -705,11 +827,22 @@ static void run_halo_products(const Dev &d, const SweepArgs &a, cudaStream_t s) 
 }
 template <class Met, typename T>
 static void run_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool backward, bool last) {
-  const int ntiles = sweep_tiles_x<T>(d.nx) * sweep_tiles_y(d.ny);
+  const int cx = a.cluster_x, ncx = (sweep_tiles_x<T>(d.nx) + cx - 1) / cx;
   using F = SweepShape<T, !Met::kChannel, false>;
   using B = SweepShape<T, !Met::kChannel, true>;
-  if (!backward) k_sweep<Met, false, T><<<ntiles, F::THREADS, F::SMEM, s>>>(d, a, last);
-  else k_sweep<Met, true, T><<<ntiles, B::THREADS, B::SMEM, s>>>(d, a, last);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncx * cx * sweep_tiles_y(d.ny));
+  cfg.blockDim = dim3(F::THREADS);
+  cfg.dynamicSmemBytes = backward ? B::SMEM : F::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cx;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (!backward) cudaLaunchKernelEx(&cfg, k_sweep<Met, false, T>, d, a, (int)last);
+  else cudaLaunchKernelEx(&cfg, k_sweep<Met, true, T>, d, a, (int)last);
 }
 // one symmetric sweep; its backward dQ is stored only when the update follows
 template <class Met, typename T>

@@ -56,6 +56,54 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
   return false;
 }
 
+// ------------------------------------------- thread-block clusters (DSMEM)
+// A CTA's rank in its cluster and the cluster's size (1 without clusters).
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// The shared::cluster address of the variable at shared::cta address `local`
+// in the shared memory of cluster CTA `rank`.
+__device__ __forceinline__ uint32_t mapa(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+// Asynchronous stores into another cluster CTA's shared memory that count
+// their bytes on that CTA's mbarrier (complete_tx): the consumer arms the
+// barrier with the bytes it expects and waits on it; no fence is needed on
+// the producing side.
+__device__ __forceinline__ void st_async(uint32_t addr, double x, uint32_t remote_bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr), "d"(x),
+               "r"(remote_bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t addr, float x, uint32_t remote_bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(addr), "f"(x),
+               "r"(remote_bar)
+               : "memory");
+}
+// Arrival on another cluster CTA's mbarrier without ordering this thread's
+// earlier memory operations (a flow-control signal that carries no data).
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t remote_bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+}
+// The cluster-wide barrier of every thread of the cluster that has not exited.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 // ------------------------------------------------------------------ TMA
 // Tiled 2-D / 4-D loads into this CTA's shared memory, completing on an
 // mbarrier; `map` is the generic address of a __grid_constant__ CUtensorMap.
