@@ -256,7 +256,7 @@ def run_gpu(a, dist: Dist) -> dict | None:
         return None
     from cgli_fu_flow_b200 import roofline
     # the roofline kernel's mean launch: the wavefront passes of every inner
-    # iteration of the timed steps, from events around them in the graph
+    # iteration of the timed steps, from the device clock around them
     roof = roofline.sweep_roofline(ch, sweep_ms / max(sweep_passes, 1), a.precision)
     roof["launches_timed"] = sweep_passes
     out = {

@@ -61,14 +61,18 @@ struct cgli_ctx {
   cgli::SweepArgs sw;
   bool metrics_checked = false;
   cudaGraphExec_t iter_graph = nullptr;
-  cudaGraphExec_t dts_graph = nullptr;
   cudaEvent_t events[8] = {};
   double Emax[5] = {0, 0, 0, 0, 0};   // running maximum of the norms over the run
   int history = 0;                    // completed steps since the state was set
   int predictor = 0;                  // 0 previous level, 1 extrapolation, 2 learned
   int inner_solver = CGLI_LUSGS;      // CGLI_LUSGS or CGLI_DPLUR
-  cudaEvent_t sweep_ev[2] = {};       // recorded around the wavefront passes inside the iteration graph
-  double sweep_ms = 0;                // their accumulated device time since the last reset
+  // results of the last kRing inner iterations, written by the iterations
+  // themselves (pinned host memory), and how many were launched so far
+  cgli::IterResult *ring = nullptr;
+  long long launched = 0;
+  cudaStream_t side[3] = {};          // branches of the iteration graph (fluxes, viscous terms)
+  cudaEvent_t fork = nullptr, join[3] = {};
+  double sweep_ms = 0;                // accumulated device time of the wavefront passes since the last reset
   long long sweep_passes = 0;
   cgli_cnn *cnn = nullptr;            // learned initial guess (not owned)
   std::vector<double> step_norms;     // the five norms of every inner iteration of the last step
@@ -79,6 +83,8 @@ struct cgli_ctx {
 };
 
 namespace {
+
+constexpr int kRing = 32;
 
 int alloc(cgli_ctx *c, size_t bytes, void **out) {
   void *p = nullptr;
@@ -189,19 +195,43 @@ int read_norms(cgli_ctx *c, double er[5], int nblocks) {
   cgli::launch_norms(c->d, c->stream, nblocks, scale, c->d_out);
   CUDA_TRY(cudaMemcpyAsync(c->h_norms, c->d_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
-  int status = 0;
-  CUDA_TRY(cudaMemcpy(&status, c->d.status, sizeof(int), cudaMemcpyDeviceToHost));
-  if (status) {
-    int zero = 0;
-    cudaMemcpy(c->d.status, &zero, sizeof(int), cudaMemcpyHostToDevice);
-    // products that were never read are left behind: only the sentinel again
-    cudaMemset(c->sw.xbuf, 0xff, c->sw.hand_bytes);
-    return fail(CGLI_ETIMEOUT, "a wavefront tile gave up waiting for its neighbour (bounded spin)");
-  }
   for (int v = 0; v < 5; v++) er[v] = c->h_norms[v];
   for (int v = 0; v < 5; v++)
     if (!std::isfinite(er[v])) return fail(CGLI_EDIVERGED, "update norm is not finite");
   return CGLI_OK;
+}
+
+// Launches the iteration graph n (<= kRing) times and waits; the iterations
+// need nothing from the host in between.  Returns how many of them are good
+// and their results; a failed one (its successors leave the state alone) sets
+// *rc and clears what it left behind.
+int run_iterations(cgli_ctx *c, int n, const cgli::IterResult *res[kRing], int *rc) {
+  const long long first = c->launched;
+  *rc = CGLI_OK;
+  for (int it = 0; it < n; it++) {
+    const cudaError_t e = cudaGraphLaunch(c->iter_graph, c->stream);
+    if (e != cudaSuccess) { *rc = fail(CGLI_ECUDA, std::string("cudaGraphLaunch: ") + cudaGetErrorString(e)); n = it; break; }
+    c->launched++;
+  }
+  const cudaError_t e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) { *rc = fail(CGLI_ECUDA, std::string("cudaStreamSynchronize: ") + cudaGetErrorString(e)); return 0; }
+  for (int it = 0; it < n; it++) {
+    const cgli::IterResult &r = c->ring[(first + it) % kRing];
+    bool finite = true;
+    for (int v = 0; v < 5; v++) finite = finite && std::isfinite(r.norm[v]);
+    if (r.status == 0 && finite) {
+      res[it] = &r;
+      if (r.sweep_ms > 0) { c->sweep_ms += r.sweep_ms; c->sweep_passes += 4; }
+      continue;
+    }
+    cudaMemset(c->d.status, 0, sizeof(int));
+    // products that were never read are left behind: only the sentinel again
+    cudaMemset(c->sw.xbuf, 0xff, c->sw.hand_bytes);
+    *rc = r.status ? fail(CGLI_ETIMEOUT, "a wavefront tile gave up waiting for its neighbour (bounded spin)")
+                   : fail(CGLI_EDIVERGED, "update norm is not finite");
+    return it;
+  }
+  return n;
 }
 
 void drop_graph(cgli_ctx *c) {
@@ -351,6 +381,7 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
       if (cudaMemset(a.xbuf, 0xff, a.hand_bytes) != cudaSuccess) rc = fail(CGLI_ECUDA, "cudaMemset");   // the sentinel
     }
     if (rc == CGLI_OK) rc = alloc(c, 64, (void **)&a.ticket);
+    if (rc == CGLI_OK) rc = alloc(c, 64, (void **)&a.clock);
     double *jt = nullptr, *et = nullptr;
     if (rc == CGLI_OK) rc = alloc(c, sizeof(double) * d.Y, (void **)&jt);
     if (rc == CGLI_OK) rc = alloc(c, sizeof(double) * d.Y, (void **)&et);
@@ -375,7 +406,8 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
     if (rc == CGLI_OK) cudaMemcpy(dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice);
     a.order = dorder;
   }
-  if (rc == CGLI_OK && cudaMallocHost(&c->h_norms, 16 * sizeof(double)) != cudaSuccess)
+  if (rc == CGLI_OK && (cudaMallocHost(&c->h_norms, 16 * sizeof(double)) != cudaSuccess ||
+                        cudaMallocHost(&c->ring, kRing * sizeof(cgli::IterResult)) != cudaSuccess))
     rc = fail(CGLI_ENOMEM, "cudaMallocHost");
   if (rc == CGLI_OK && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
     rc = fail(CGLI_ECUDA, "cudaStreamCreate");
@@ -387,8 +419,12 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
   }
   for (auto &e : c->events)
     if (rc == CGLI_OK && cudaEventCreate(&e) != cudaSuccess) rc = fail(CGLI_ECUDA, "cudaEventCreate");
-  for (auto &e : c->sweep_ev)
-    if (rc == CGLI_OK && cudaEventCreate(&e) != cudaSuccess) rc = fail(CGLI_ECUDA, "cudaEventCreate");
+  for (int q = 0; q < 3; q++)
+    if (rc == CGLI_OK && (cudaStreamCreateWithFlags(&c->side[q], cudaStreamNonBlocking) != cudaSuccess ||
+                          cudaEventCreateWithFlags(&c->join[q], cudaEventDisableTiming) != cudaSuccess))
+      rc = fail(CGLI_ECUDA, "cudaStreamCreate");
+  if (rc == CGLI_OK && cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) != cudaSuccess)
+    rc = fail(CGLI_ECUDA, "cudaEventCreate");
   if (rc != CGLI_OK) {
     std::string keep = g_err;
     cgli_destroy(c);
@@ -406,11 +442,14 @@ int cgli_destroy(cgli_ctx *c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->iter_graph) cudaGraphExecDestroy(c->iter_graph);
-  if (c->dts_graph) cudaGraphExecDestroy(c->dts_graph);
   for (auto &e : c->events)
     if (e) cudaEventDestroy(e);
-  for (auto &e : c->sweep_ev)
+  for (auto &e : c->join)
     if (e) cudaEventDestroy(e);
+  if (c->fork) cudaEventDestroy(c->fork);
+  for (auto &q : c->side)
+    if (q) cudaStreamDestroy(q);
+  if (c->ring) cudaFreeHost(c->ring);
   for (void *p : c->allocs) cudaFree(p);
   if (c->h_norms) cudaFreeHost(c->h_norms);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -733,46 +772,51 @@ int cgli_set_inner_solver(cgli_ctx *c, int solver) {
   return CGLI_OK;
 }
 
+// the graph of one inner iteration, its results into the ring
+static int ensure_graph(cgli_ctx *c) {
+  if (c->iter_graph) return CGLI_OK;
+  const bool dplur = c->inner_solver == CGLI_DPLUR, mixed = c->p.precision == CGLI_MIXED;
+  cudaStream_t s = c->stream;
+  cudaGraph_t g;
+  CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  // the three fluxes and the viscous terms depend on the boundaries only:
+  // parallel branches of the graph
+  cgli::launch_halo_bc(c->d, s);
+  cudaEventRecord(c->fork, s);
+  for (cudaStream_t q : c->side) cudaStreamWaitEvent(q, c->fork, 0);
+  cgli::launch_viscous(c->d, s);
+  cgli::launch_flux_x(c->d, c->side[0]);
+  cgli::launch_flux_y(c->d, c->side[1]);
+  cgli::launch_flux_z(c->d, c->side[2]);
+  if (!dplur) cgli::launch_target_u(c->d, c->side[0]);
+  for (int q = 0; q < 3; q++) {
+    cudaEventRecord(c->join[q], c->side[q]);
+    cudaStreamWaitEvent(s, c->join[q], 0);
+  }
+  if (dplur) {
+    cgli::launch_dplur(c->d, c->sw, s);
+  } else {
+    cgli::launch_residual_fast(c->d, c->sw, s, mixed);
+    cgli::launch_sweeps(c->d, c->sw, s, mixed);
+    cgli::launch_sweep_update(c->d, c->sw, s, mixed);
+  }
+  cgli::launch_iteration_result(c->d, c->sw, s, dplur ? c->update_blocks : c->sweep_update_blocks,
+                                1.0 / ((double)c->p.nx * c->p.ny * c->p.nz), c->ring, kRing, !dplur);
+  cudaError_t e = cudaStreamEndCapture(s, &g);
+  if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+  e = cudaGraphInstantiate(&c->iter_graph, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  return CGLI_OK;
+}
+
 int cgli_inner_iteration(cgli_ctx *c, double er[5]) {
   int rc = check(c); if (rc) return rc;
   rc = need_ready(c); if (rc) return rc;
   if (!er) return fail(CGLI_EINVAL, "null er");
-  if (!c->metrics_checked) {
-    rc = check_channel_metrics(c); if (rc) return rc;
-  }
-  const bool dplur = c->inner_solver == CGLI_DPLUR;
-  if (!c->iter_graph) {
-    cudaGraph_t g;
-    CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    if (dplur) {
-      cgli::launch_dplur_iteration(c->d, c->sw, c->stream);
-    } else {
-      // the four wavefront passes are bracketed by two events, so that their
-      // device time is known for every iteration the graph runs
-      cgli::launch_fused_residual(c->d, c->sw, c->stream, c->p.precision);
-      // (external records: event-record nodes of the graph, not capture-internal dependencies)
-      cudaEventRecordWithFlags(c->sweep_ev[0], c->stream, cudaEventRecordExternal);
-      cgli::launch_sweeps(c->d, c->sw, c->stream, c->p.precision == CGLI_MIXED);
-      cudaEventRecordWithFlags(c->sweep_ev[1], c->stream, cudaEventRecordExternal);
-      cgli::launch_sweep_update(c->d, c->sw, c->stream, c->p.precision == CGLI_MIXED);
-    }
-    cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-    if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&c->iter_graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-  }
-  CUDA_TRY(cudaGraphLaunch(c->iter_graph, c->stream));
-  rc = read_norms(c, er, dplur ? c->update_blocks : c->sweep_update_blocks);   // synchronises the stream
-  if (rc == CGLI_OK && !dplur) {
-    float ms = 0;
-    if (cudaEventElapsedTime(&ms, c->sweep_ev[0], c->sweep_ev[1]) == cudaSuccess) {
-      c->sweep_ms += ms;
-      c->sweep_passes += 4;
-    } else {
-      cudaGetLastError();   // timing unavailable: leave no error behind for the next call
-    }
-  }
+  rc = ensure_graph(c); if (rc) return rc;
+  const cgli::IterResult *res[kRing];
+  if (run_iterations(c, 1, res, &rc) == 1) std::copy(res[0]->norm, res[0]->norm + 5, er);
   return rc;
 }
 
@@ -924,22 +968,26 @@ int cgli_step(cgli_ctx *c, int fixed_iters, double drop, int cap, int *iters, do
   }
   int it = 0;
   c->step_norms.clear();
-  while (true) {
-    it++;
-    rc = cgli_inner_iteration(c, er);
+  rc = ensure_graph(c); if (rc) return rc;
+  bool stop = false;
+  while (!stop) {
+    // a fixed number of iterations needs no norms on the way
+    const int n = fixed_iters > 0 ? std::min(fixed_iters - it, kRing) : 1;
+    const cgli::IterResult *res[kRing];
+    const int good = run_iterations(c, n, res, &rc);
+    for (int q = 0; q < good; q++) {
+      it++;
+      std::copy(res[q]->norm, res[q]->norm + 5, er);
+      c->step_norms.insert(c->step_norms.end(), er, er + 5);
+      // main.cpp:287-304: norms divided by their running maximum over the run
+      bool done = true;
+      for (int v = 0; v < 5; v++) {
+        c->Emax[v] = std::max(c->Emax[v], er[v]);
+        done = done && (c->Emax[v] > 0 ? er[v] / c->Emax[v] < drop : true);
+      }
+      stop = fixed_iters > 0 ? it >= fixed_iters : done || it >= cap;
+    }
     if (rc) return rc;
-    c->step_norms.insert(c->step_norms.end(), er, er + 5);
-    // main.cpp:287-304: norms divided by their running maximum over the run
-    bool done = true;
-    for (int v = 0; v < 5; v++) {
-      c->Emax[v] = std::max(c->Emax[v], er[v]);
-      done = done && (c->Emax[v] > 0 ? er[v] / c->Emax[v] < drop : true);
-    }
-    if (fixed_iters > 0) {
-      if (it >= fixed_iters) break;
-    } else if (done || it >= cap) {
-      break;
-    }
   }
   *iters = it;
   rc = cgli_end_step(c);

@@ -33,7 +33,7 @@ template <> struct SweepTile<double> {
 template <> struct SweepTile<float> {
   static constexpr int TI = 4, TJ = SWEEP_TJ, RING = 4;
 };
-constexpr int CGLI_TIMEOUT_CODE = 6;
+constexpr int CGLI_TIMEOUT_CODE = 6, CGLI_DIVERGED_CODE = 7;   // of the status word
 
 // Buffers of the wavefront sweeps (kernels_sweep.cu), in the arithmetic type
 // of the passes (double, or float for CGLI_MIXED).  A row's stream holds the
@@ -54,6 +54,7 @@ struct SweepArgs {
   void *xbuf, *ybuf;
   size_t hand_bytes;
   unsigned int *ticket;           // tile ticket counters of the two passes
+  unsigned long long *clock;      // [0] %globaltimer at the first pass, [1] at the update; [2] iterations run
   const int *order;               // tile visiting order
   const double *Jtab, *etdytab;   // per-j metrics of a grid uniform in x and z
   int channel_metrics;            // 1: use Jtab / etdytab instead of the 3-D arrays
@@ -96,8 +97,6 @@ void launch_sweeps(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed)
 void launch_sweep_update(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed);
 // partial sums (blocks) the update after the wavefront passes writes
 int sweep_update_blocks(const Dev &d);
-// everything of a fused inner iteration before the sweeps
-void launch_fused_residual(const Dev &d, const SweepArgs &a, cudaStream_t s, int precision);
 // one pass of the first or the last sweep (a forward one with both passes'
 // halo products)
 void launch_sweep_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed, bool backward, bool last);
@@ -111,8 +110,6 @@ void launch_dts_residual(const Dev &d, cudaStream_t s);
 void launch_dplur(const Dev &d, const SweepArgs &sw, cudaStream_t s);
 // one relaxation NR -> NL (from_nr) or NL -> NR
 void launch_dplur_relax(const Dev &d, const SweepArgs &sw, cudaStream_t s, bool from_nr);
-// halo, boundaries, fluxes, viscous terms, then launch_dplur
-void launch_dplur_iteration(const Dev &d, const SweepArgs &sw, cudaStream_t s);
 // residual assembly writing MR and the first sweep's lagged halo planes
 void launch_residual_fast(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed);
 
@@ -142,6 +139,18 @@ void launch_viscous(const Dev &d, cudaStream_t s);
 void launch_dts(const Dev &d, cudaStream_t s, int update_blocks_x);
 // reduces d.partial (nblocks x 5) into out[5] = sqrt(sum) * scale
 void launch_norms(const Dev &d, cudaStream_t s, int nblocks, double scale, double *out);
+// what an inner iteration leaves for the host
+struct IterResult {
+  double norm[5];
+  double sweep_ms;   // device time of the wavefront passes (0: none)
+  int status;        // the status word: a pass that gave up
+};
+// the norms from d.partial (as launch_norms), the status word and the passes'
+// time of this iteration into ring[iteration % slots] (host memory); a norm
+// that is not finite sets the status word, so that iterations launched behind
+// this one leave the state alone
+void launch_iteration_result(const Dev &d, const SweepArgs &a, cudaStream_t s, int nblocks, double scale,
+                             IterResult *ring, int slots, bool timed);
 // bulk mass flux (Driven_force.cpp:38-62) into out[0]; out holds 8 + 296
 // doubles (per-block partial sums at out + 8)
 void launch_bulk_flux(const Dev &d, cudaStream_t s, double *out);

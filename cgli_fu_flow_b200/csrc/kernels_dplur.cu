@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(128, 8) k_dplur_update(Dev d, RelaxPtrs a) {
   int i = 3 + blockIdx.y;
   const double *const *nr = a.src;
   double acc[5] = {0, 0, 0, 0, 0};
+  if (*(volatile int *)d.status) return;   // an iteration before this one failed: keep the state
   for (int kk = k; kk <= d.nz + 1; kk += blockDim.x) {
     long long c = ix(d, i, j, kk);
     // the divisions by q1, rho, T and J as reciprocals (1/J from the table)
@@ -341,15 +342,6 @@ void launch_dplur(const Dev &d, const SweepArgs &sw, cudaStream_t s) {
   for (int sweep = 0; sweep < 4; sweep++) launch_dplur_relax(d, sw, s, sweep % 2 == 0);
   RelaxPtrs a = ptrs(d.NR, d.NL, sw);
   k_dplur_update<<<dim3(d.ny, d.nx), 128, 0, s>>>(d, a);
-}
-
-void launch_dplur_iteration(const Dev &d, const SweepArgs &sw, cudaStream_t s) {
-  launch_halo_bc(d, s);
-  launch_flux_x(d, s);
-  launch_flux_y(d, s);
-  launch_flux_z(d, s);
-  launch_viscous(d, s);
-  launch_dplur(d, sw, s);
 }
 
 }  // namespace cgli

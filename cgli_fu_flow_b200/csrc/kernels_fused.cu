@@ -1,6 +1,5 @@
-// Fast path of one inner iteration: halo and boundaries, fluxes, viscous
-// terms, residual assembly, four wavefront sweep passes with the update
-// fused into the last one.
+// Residual assembly of the fast path of one inner iteration (between the
+// fluxes / viscous terms and the wavefront sweeps).
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
 
@@ -159,16 +158,6 @@ void launch_residual_fast(const Dev &d, const SweepArgs &a, cudaStream_t s, bool
     if (mixed) k_residual_fast<true, false><<<g, 64, 0, s>>>(d, a);
     else k_residual_fast<false, false><<<g, 64, 0, s>>>(d, a);
   }
-}
-
-void launch_fused_residual(const Dev &d, const SweepArgs &a, cudaStream_t s, int precision) {
-  launch_halo_bc(d, s);
-  launch_flux_x(d, s);
-  launch_flux_y(d, s);
-  launch_flux_z(d, s);
-  launch_viscous(d, s);
-  launch_target_u(d, s);
-  launch_residual_fast(d, a, s, precision == 1);
 }
 
 }  // namespace cgli

@@ -702,6 +702,34 @@ __global__ void k_norms(const double *partial, int nblocks, double scale, double
   if (threadIdx.x < 5) out[threadIdx.x] = sqrt(tot[threadIdx.x]) * scale;
 }
 
+// the same at the end of an inner iteration, with what else the host wants to
+// know of it, into a slot of a ring in host memory: the iteration graph needs
+// no copy nodes, and several iterations can run without the host in between.
+// a.clock[2] counts the iterations.
+__global__ void k_iteration_result(Dev d, SweepArgs a, int nblocks, double scale, IterResult *ring, int slots, int timed) {
+  double acc[5] = {0, 0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
+    for (int v = 0; v < 5; v++) acc[v] += d.partial[5 * (long long)b + v];
+  __shared__ double tot[5];
+  block_sum5(acc, tot);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  IterResult r;
+  bool finite = true;
+  for (int v = 0; v < 5; v++) {
+    r.norm[v] = sqrt(tot[v]) * scale;
+    finite = finite && isfinite(r.norm[v]);
+  }
+  r.sweep_ms = timed ? 1e-6 * (double)(a.clock[1] - a.clock[0]) : 0.0;
+  r.status = *(volatile int *)d.status;
+  if (!r.status && !finite) *d.status = CGLI_DIVERGED_CODE;
+  ring[a.clock[2]++ % slots] = r;
+}
+void launch_iteration_result(const Dev &d, const SweepArgs &a, cudaStream_t s, int nblocks, double scale,
+                             IterResult *ring, int slots, bool timed) {
+  k_iteration_result<<<1, 1024, 0, s>>>(d, a, nblocks, scale, ring, slots, timed);
+}
+
 // bulk mass flux, Driven_force.cpp:38-62: sum over interior cells of
 // (U2_*J)/J / Jsum with Jsum the column volume sum at (i,k) = (3,3)
 // bulk mass flux of Driven_force.cpp:38-62: sum over the interior of

@@ -212,7 +212,12 @@ __device__ __forceinline__ void load_cellrec(const float *p, int t, float rec[RE
 // every (j, k), off the wavefront's critical path, in step order for the
 // rows' x helpers.  Both passes' products come from one launch: both inputs
 // are known before the sweep's first pass.  The launch also resets the two
-// passes' tickets.
+// passes' tickets and (first sweep) notes the time.
+__device__ __forceinline__ unsigned long long globaltimer() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
 template <class Met, bool BACKWARD, typename T>
 __device__ __noinline__ void halo_product(const Dev &d, const SweepArgs &a, int j, int k) {
   const long long h = (long long)j * d.dj + k;
@@ -233,8 +238,11 @@ __device__ __noinline__ void halo_product(const Dev &d, const SweepArgs &a, int 
   for (int v = 0; v < 5; v++) a.buf<T>(a.hx[BACKWARD])[s + v * SWEEP_TJ] = o[v];
 }
 template <class Met, typename T>
-__global__ void k_halo_products(const __grid_constant__ Dev d, const __grid_constant__ SweepArgs a) {
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.ticket[blockIdx.z] = 0;
+__global__ void k_halo_products(const __grid_constant__ Dev d, const __grid_constant__ SweepArgs a, int first) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    a.ticket[blockIdx.z] = 0;
+    if (first && blockIdx.z == 0) a.clock[0] = globaltimer();
+  }
   const int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
   if (k > d.nz + 1) return;
   if (blockIdx.z == 0) halo_product<Met, false, T>(d, a, 2 + blockIdx.y, k);
@@ -730,6 +738,7 @@ __global__ void __launch_bounds__(256) k_update_skewed(Dev d, SweepArgs a) {
   constexpr int NS = UPD_KC + UPD_TJ - 1;   // steps holding the block's cells
   static_assert(SWEEP_TJ % UPD_TJ == 0 && 256 % UPD_TJ == 0, "column staging");
   __shared__ T sdq[5][NS][UPD_TJ + 1];       // (+1: the update reads a column down the steps)
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.clock[1] = globaltimer();
   // a wavefront pass that gave up left dQ incomplete: keep the state
   if (*(volatile int *)d.status) return;
   const int ntu = (d.ny + UPD_TJ - 1) / UPD_TJ, S = sweep_steps(d);
@@ -822,8 +831,8 @@ static int cluster_x_for(int nti) {
 int sweep_cluster_x(int nti, bool mixed) { return mixed ? cluster_x_for<float>(nti) : cluster_x_for<double>(nti); }
 
 template <class Met, typename T>
-static void run_halo_products(const Dev &d, const SweepArgs &a, cudaStream_t s) {
-  k_halo_products<Met, T><<<dim3((d.nz + 63) / 64, d.ny, 2), 64, 0, s>>>(d, a);
+static void run_halo_products(const Dev &d, const SweepArgs &a, cudaStream_t s, bool first) {
+  k_halo_products<Met, T><<<dim3((d.nz + 63) / 64, d.ny, 2), 64, 0, s>>>(d, a, first);
 }
 template <class Met, typename T>
 static void run_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool backward, bool last) {
@@ -847,7 +856,7 @@ static void run_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool back
 // one symmetric sweep; its backward dQ is stored only when the update follows
 template <class Met, typename T>
 static void run_sweep(const Dev &d, const SweepArgs &a, cudaStream_t s, bool last) {
-  run_halo_products<Met, T>(d, a, s);
+  run_halo_products<Met, T>(d, a, s, !last);
   run_pass<Met, T>(d, a, s, false, last);
   run_pass<Met, T>(d, a, s, true, last);
 }
@@ -864,7 +873,7 @@ static void run_sweep(const Dev &d, const SweepArgs &a, cudaStream_t s, bool las
   } while (0)
 
 void launch_sweep_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed, bool backward, bool last) {
-  if (!backward) SWEEP_DISPATCH(run_halo_products, d, a, s);
+  if (!backward) SWEEP_DISPATCH(run_halo_products, d, a, s, !last);
   SWEEP_DISPATCH(run_pass, d, a, s, backward, last);
 }
 

@@ -315,7 +315,7 @@ class Solver:
 
     def sweep_time(self, reset: bool = False) -> tuple[float, int]:
         """(ms, passes): device time of the wavefront passes of every inner
-        iteration since the last reset (events inside the iteration graph)."""
+        iteration since the last reset (the device clock around them)."""
         ms = ctypes.c_double()
         n = ctypes.c_longlong()
         self._rc(self.L.cgli_sweep_time(self.h, ctypes.byref(ms), ctypes.byref(n), int(reset)))
