@@ -26,7 +26,7 @@ namespace {
 
 constexpr int FTJ = 8, FTK = 32;                 // output tile (j, k)
 constexpr int FRJ = FTJ + 2, FRK = FTK + 2;      // tile with a one-cell halo
-constexpr int FCHUNK = 16;                       // x planes per CTA
+constexpr int FTHREADS = (FRJ * FRK + 31) / 32 * 32;   // a thread per cell of the tile with halo
 
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
@@ -53,12 +53,38 @@ struct LevelArgs {
   int wrap;             // read P through its periodic image: the 3-plane
                         // exchange of level 3 on a single periodic slab
                         // (Filter.cpp:447-466) without a copy
+  int chunk;            // x planes per CTA
 };
 
 __device__ __forceinline__ int wrap_plane(int p, int nx) { return p < 3 ? p + nx : (p > nx + 2 ? p - nx : p); }
 
+// The quotients a / b of one divisor, correctly rounded, from its correctly
+// rounded reciprocal: q <- q + (a - q b) (1 / b) with fused multiply-adds, the
+// second of which starts within half a unit in the last place and so rounds
+// correctly (P. Markstein, IBM J. Res. Dev. 34(1), 1990), for operands and
+// quotients far from over- and underflow; any other goes through the IEEE
+// division (a divisor out of range through its NaN for a reciprocal).
+__device__ __forceinline__ double divisor(double b) {
+  const double m = fabs(b);
+  return m > 1e-200 && m < 1e200 ? __drcp_rn(b) : __longlong_as_double(0x7ff8000000000000LL);
+}
+__device__ __forceinline__ double quotient(double a, double b, double rb) {
+  double q = mul(a, rb);
+  q = __fma_rn(__fma_rn(-q, b, a), rb, q);
+  q = __fma_rn(__fma_rn(-q, b, a), rb, q);
+  const double m = fabs(q), n = fabs(a);
+  return m > 1e-200 && m < 1e200 && n > 1e-200 && n < 1e200 ? q : dvd(a, b);
+}
+
+// One level.  Bound by the latency of its chain of planes (load, x, y and z
+// pass, a barrier each): every plane's loads (the next plane of the previous
+// level, the next J and Y, the running sum) are issued a plane ahead, a thread
+// per cell of the tile with halo keeps each pass to one round, and the x
+// chunk is chosen so that the CTAs fill the chip (launch_filter).  At
+// 96x72x72 a level takes 51.5 us; with chunks of 16 planes, a division where
+// the quotient stands and loads inside the passes it took 137.
 template <bool TWO_H>
-__global__ void __launch_bounds__(FTJ *FTK) k_filter_level(LevelArgs a) {
+__global__ void __launch_bounds__(FTHREADS, 2) k_filter_level(LevelArgs a) {
   extern __shared__ double sm[];
   double *ring = sm;                                // [3][4][FRJ*FRK]
   double *gx = ring + 3 * 4 * FRJ * FRK;            // [4][FRJ*FRK]
@@ -69,121 +95,128 @@ __global__ void __launch_bounds__(FTJ *FTK) k_filter_level(LevelArgs a) {
 
   const int tid = threadIdx.x;
   const int k0 = 2 + blockIdx.x * FTK, j0 = 2 + blockIdx.y * FTJ;
-  const int ia = a.i0 + blockIdx.z * FCHUNK;
-  const int ib = min(a.i1, ia + FCHUNK - 1);
+  const int ia = a.i0 + blockIdx.z * a.chunk;
+  const int ib = min(a.i1, ia + a.chunk - 1);
   const int ny = a.ny + 1, nz = a.nz + 1;           // the reference's ny, nz
   const long long di = (long long)a.Y * a.Z, dj = a.Z;
   const int gend = a.nx + 2;
 
-  auto load_plane = [&](int p) {
-    const int slot = p % 3;
-    const int src = a.wrap ? wrap_plane(p, a.nx) : p;
-    for (int t = tid; t < FRJ * FRK; t += FTJ * FTK) {
-      const int j = j0 - 1 + t / FRK, k = k0 - 1 + t % FRK;
-      if (j >= 2 && j <= ny && k >= 2 && k <= nz) {
-        const long long o = src * di + j * dj + k;
+  // this thread's cell of the tile with halo (x pass), of the tile with the
+  // z halo (y pass) and of the tile (z pass)
+  const int jh = j0 - 1 + tid / FRK, kh = k0 - 1 + tid % FRK;
+  const bool in_h = tid < FRJ * FRK;
+  const bool ring_cell = in_h && jh >= 2 && jh <= ny && kh >= 2 && kh <= nz;
+  const bool j_cell = in_h && jh >= 1 && jh <= ny + 1 && kh >= 1 && kh <= nz + 1;
+  const bool wall_cell = in_h && (jh == 1 || jh == ny + 1) && kh >= 2 && kh <= nz;
+  const int jy = j0 + tid / FRK, ky = k0 - 1 + tid % FRK;
+  const bool in_y = tid < FTJ * FRK && jy <= ny;
+  const bool y_cell = in_y && ky >= 2 && ky <= nz, z_ghost = in_y && (ky == 1 || ky == nz + 1);
+  const int rz = tid / FTK, cz = tid % FTK;
+  const bool z_cell = tid < FTJ * FTK && j0 + rz <= ny && k0 + cz <= nz;
+  const long long oh = jh * dj + kh, oy = jy * dj + ky, oz = (j0 + rz) * dj + k0 + cz;
+
+  double np[4], nj = 0, ym = 0, yc = 0, yp = 0, ac[4], ug[4];
+  auto fetch_plane = [&](int p) {
+    const long long o = (long long)(a.wrap ? wrap_plane(p, a.nx) : p) * di + oh;
+    if (ring_cell)
 #pragma unroll
-        for (int v = 0; v < 4; v++) ring[(slot * 4 + v) * FRJ * FRK + t] = a.P[v][o];
-      }
-    }
+      for (int v = 0; v < 4; v++) np[v] = a.P[v][o];
+  };
+  auto put_plane = [&](int p) {
+    if (ring_cell)
+#pragma unroll
+      for (int v = 0; v < 4; v++) ring[((p % 3) * 4 + v) * FRJ * FRK + tid] = np[v];
+  };
+  auto fetch_metric = [&](int i) {   // J on the tile with halo, Y for the weights of the y pass
+    if (j_cell) nj = a.J[i * di + oh];
+    if (y_cell) { ym = a.Yp[i * di + oy - dj]; yc = a.Yp[i * di + oy]; yp = a.Yp[i * di + oy + dj]; }
   };
 
-  load_plane(ia - 1);
-  load_plane(ia);
+  for (int p = ia - 1; p <= ia + 1; p++) {
+    fetch_plane(p);
+    put_plane(p);
+  }
+  fetch_metric(ia);
   for (int i = ia; i <= ib; i++) {
-    __syncthreads();
-    load_plane(i + 1);
-    // J of plane i on the tile with halo, y-pass weights (Filter.cpp:187-191)
-    for (int t = tid; t < FRJ * FRK; t += FTJ * FTK) {
-      const int j = j0 - 1 + t / FRK, k = k0 - 1 + t % FRK;
-      if (j >= 1 && j <= ny + 1 && k >= 1 && k <= nz + 1) jt[t] = a.J[i * di + j * dj + k];
-    }
-    for (int t = tid; t < FTJ * FRK; t += FTJ * FTK) {
-      const int j = j0 + t / FRK, k = k0 - 1 + t % FRK;
-      if (j <= ny && k >= 2 && k <= nz) {
-        const long long o = i * di + j * dj + k;
-        const double yp = a.Yp[o + dj], yc = a.Yp[o], ym = a.Yp[o - dj];
-        const double A = sub(yp, ym), B = sub(yp, yc), C = sub(yc, ym);
-        w1[t] = TWO_H ? dvd(B, A) : dvd(mul(2.0, B), A);
-        w3[t] = TWO_H ? dvd(C, A) : dvd(mul(2.0, C), A);
-      }
+    // J of plane i, y-pass weights (Filter.cpp:187-191)
+    if (j_cell) jt[tid] = nj;
+    if (y_cell) {
+      const double A = sub(yp, ym), B = sub(yp, yc), C = sub(yc, ym), rA = divisor(A);
+      w1[tid] = quotient(TWO_H ? B : mul(2.0, B), A, rA);
+      w3[tid] = quotient(TWO_H ? C : mul(2.0, C), A, rA);
     }
     __syncthreads();
+    const bool interior = i >= 3 && i <= gend;
+    if (i < ib) {
+      fetch_plane(i + 2);
+      fetch_metric(i + 1);
+    }
+    if (z_cell && interior && a.level > 0)
+#pragma unroll
+      for (int v = 0; v < 4; v++) ac[v] = a.acc[v][i * di + oz];
+    if (wall_cell)
+#pragma unroll
+      for (int v = 0; v < 4; v++) ug[v] = a.U[v][i * di + oh];
     // x pass; the wall rows keep U_ (the scratch arrays start as U_ copies,
     // Filter.cpp:121-138, and the passes only write j = 2..ny)
     const int sm1 = (i - 1) % 3, s0 = i % 3, sp1 = (i + 1) % 3;
-    for (int t = tid; t < FRJ * FRK; t += FTJ * FTK) {
-      const int j = j0 - 1 + t / FRK, k = k0 - 1 + t % FRK;
-      if (k < 2 || k > nz) continue;
-      if (j >= 2 && j <= ny) {
+    if (ring_cell) {
 #pragma unroll
-        for (int v = 0; v < 4; v++)
-          gx[v * FRJ * FRK + t] = smooth3<TWO_H>(ring[(sm1 * 4 + v) * FRJ * FRK + t], ring[(s0 * 4 + v) * FRJ * FRK + t],
-                                                 ring[(sp1 * 4 + v) * FRJ * FRK + t]);
-      } else if (j == 1 || j == ny + 1) {
-        const long long o = i * di + j * dj + k;
+      for (int v = 0; v < 4; v++)
+        gx[v * FRJ * FRK + tid] = smooth3<TWO_H>(ring[(sm1 * 4 + v) * FRJ * FRK + tid], ring[(s0 * 4 + v) * FRJ * FRK + tid],
+                                                 ring[(sp1 * 4 + v) * FRJ * FRK + tid]);
+    } else if (wall_cell) {
 #pragma unroll
-        for (int v = 0; v < 4; v++) gx[v * FRJ * FRK + t] = a.U[v][o];
-      }
+      for (int v = 0; v < 4; v++) gx[v * FRJ * FRK + tid] = ug[v];
     }
     __syncthreads();
     // y pass (Filter.cpp:193 for h, :875 for 2h); z ghosts keep U_
-    for (int t = tid; t < FTJ * FRK; t += FTJ * FTK) {
-      const int r = t / FRK, c = t % FRK;
-      const int j = j0 + r, k = k0 - 1 + c;
-      if (j > ny) continue;
-      if (k >= 2 && k <= nz) {
-        const int tm = r * FRK + c, tc = tm + FRK, tp = tc + FRK;
-        const double Jm = jt[tm], Jc = jt[tc], Jp = jt[tp];
-        const double wa = w1[t], wc = w3[t];
+    if (y_cell) {
+      const int tm = tid, tc = tm + FRK, tp = tc + FRK;   // rows jy - 1, jy, jy + 1 of the tile with halo
+      const double Jm = jt[tm], Jc = jt[tc], Jp = jt[tp], rJ = divisor(Jc);
+      const double wa = w1[tid], wc = w3[tid];
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const double *g = gx + v * FRJ * FRK;
-          const double s = add(add(mul(mul(wa, g[tm]), Jm), mul(mul(TWO_H ? 1.0 : 6.0, g[tc]), Jc)), mul(mul(wc, g[tp]), Jp));
-          gy[v * FTJ * FRK + t] = TWO_H ? dvd(mul(0.5, s), Jc) : dvd(mul(0.125, s), Jc);
-        }
-      } else if (k == 1 || k == nz + 1) {
-        const long long o = i * di + j * dj + k;
-#pragma unroll
-        for (int v = 0; v < 4; v++) gy[v * FTJ * FRK + t] = a.U[v][o];
+      for (int v = 0; v < 4; v++) {
+        const double *g = gx + v * FRJ * FRK;
+        const double s = add(add(mul(mul(wa, g[tm]), Jm), mul(mul(TWO_H ? 1.0 : 6.0, g[tc]), Jc)), mul(mul(wc, g[tp]), Jp));
+        gy[v * FTJ * FRK + tid] = quotient(mul(TWO_H ? 0.5 : 0.125, s), Jc, rJ);
       }
+    } else if (z_ghost) {
+#pragma unroll
+      for (int v = 0; v < 4; v++) gy[v * FTJ * FRK + tid] = a.U[v][i * di + oy];
     }
     __syncthreads();
     // z pass, high-pass accumulation, E on the last level
-    {
-      const int r = tid / FTK, c = tid % FTK;
-      const int j = j0 + r, k = k0 + c;
-      if (j <= ny && k <= nz) {
-        const long long o = i * di + j * dj + k;
-        const bool interior = i >= 3 && i <= gend;
-        double f[4];
+    if (z_cell) {
+      const long long o = i * di + oz;
+      double f[4];
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const double *g = gy + v * FTJ * FRK + r * FRK + c;
-          const double L = smooth3<TWO_H>(g[0], g[1], g[2]);
-          if (a.level < 5) a.L[v][o] = L;
-          if (interior) {
-            // Filter.cpp:769 / :1444, left to right
-            switch (a.level) {
-              case 0: a.acc[v][o] = mul(6.0, L); break;
-              case 1: a.acc[v][o] = sub(a.acc[v][o], mul(15.0, L)); break;
-              case 2: a.acc[v][o] = add(a.acc[v][o], mul(20.0, L)); break;
-              case 3: a.acc[v][o] = sub(a.acc[v][o], mul(15.0, L)); break;
-              case 4: a.acc[v][o] = add(a.acc[v][o], mul(6.0, L)); break;
-              default: f[v] = sub(a.acc[v][o], L); break;
-            }
+      for (int v = 0; v < 4; v++) {
+        const double *g = gy + v * FTJ * FRK + rz * FRK + cz;
+        const double L = smooth3<TWO_H>(g[0], g[1], g[2]);
+        if (a.level < 5) a.L[v][o] = L;
+        if (interior) {
+          // Filter.cpp:769 / :1444, left to right
+          switch (a.level) {
+            case 0: a.acc[v][o] = mul(6.0, L); break;
+            case 1: a.acc[v][o] = sub(ac[v], mul(15.0, L)); break;
+            case 2: a.acc[v][o] = add(ac[v], mul(20.0, L)); break;
+            case 3: a.acc[v][o] = sub(ac[v], mul(15.0, L)); break;
+            case 4: a.acc[v][o] = add(ac[v], mul(6.0, L)); break;
+            default: f[v] = sub(ac[v], L); break;
           }
         }
-        if (a.level == 5 && interior) {
-          // Filter.cpp:796-800 / :1471-1475
-          const double u1 = a.U[0][o];
-          const double ue = sub(dvd(a.U[1][o], u1), dvd(f[1], f[0]));
-          const double ve = sub(dvd(a.U[2][o], u1), dvd(f[2], f[0]));
-          const double we = sub(dvd(a.U[3][o], u1), dvd(f[3], f[0]));
-          a.E[o] = add(add(mul(ue, ue), mul(ve, ve)), mul(we, we));
-        }
+      }
+      if (a.level == 5 && interior) {
+        // Filter.cpp:796-800 / :1471-1475
+        const double u1 = a.U[0][o];
+        const double ue = sub(dvd(a.U[1][o], u1), dvd(f[1], f[0]));
+        const double ve = sub(dvd(a.U[2][o], u1), dvd(f[2], f[0]));
+        const double we = sub(dvd(a.U[3][o], u1), dvd(f[3], f[0]));
+        a.E[o] = add(add(mul(ue, ue), mul(ve, ve)), mul(we, we));
       }
     }
+    if (i < ib) put_plane(i + 2);   // over plane i - 1, last read by the x pass
   }
 }
 
@@ -245,6 +278,10 @@ cudaError_t launch_filter(const Dev &d, const FilterBufs &b, double crit, double
     err = cudaFuncSetAttribute(k_filter_level<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)level_smem());
   if (err != cudaSuccess) return err;
   const int gend = d.nx + 2;
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int slots = 2 * sms;   // CTAs the chip holds (registers and shared memory of two per SM)
   const int range[6][2] = {{1, gend + 2}, {2, gend + 1}, {3, gend}, {1, gend + 2}, {2, gend + 1}, {3, gend}};
   for (int sc = 0; sc < 2; sc++) {
     LevelArgs a{};
@@ -264,9 +301,17 @@ cudaError_t launch_filter(const Dev &d, const FilterBufs &b, double crit, double
       a.i1 = range[lev][1];
       a.level = lev;
       a.wrap = lev == 3;
-      dim3 grid((d.nz + FTK - 1) / FTK, (d.ny + FTJ - 1) / FTJ, (a.i1 - a.i0 + 1 + FCHUNK - 1) / FCHUNK);
-      if (sc == 0) k_filter_level<false><<<grid, FTJ * FTK, level_smem(), s>>>(a);
-      else k_filter_level<true><<<grid, FTJ * FTK, level_smem(), s>>>(a);
+      // planes per CTA: the fewest plane steps in a row on one of the chip's
+      // slots, waves x (chunk + 3, the three planes loaded before the first)
+      const int tiles = (d.nz + FTK - 1) / FTK * ((d.ny + FTJ - 1) / FTJ), planes = a.i1 - a.i0 + 1;
+      long long least = -1;
+      for (int x = 1; x <= planes; x++) {
+        const long long ctas = (long long)tiles * ((planes + x - 1) / x), cost = (ctas + slots - 1) / slots * (x + 3);
+        if (least < 0 || cost < least) { least = cost; a.chunk = x; }
+      }
+      dim3 grid((d.nz + FTK - 1) / FTK, (d.ny + FTJ - 1) / FTJ, (planes + a.chunk - 1) / a.chunk);
+      if (sc == 0) k_filter_level<false><<<grid, FTHREADS, level_smem(), s>>>(a);
+      else k_filter_level<true><<<grid, FTHREADS, level_smem(), s>>>(a);
     }
   }
   EpArgs e{};
