@@ -354,6 +354,8 @@ __global__ void __launch_bounds__(192, 1)
   const int xa = blockIdx.y * a.xchunk;
   const int n = min(a.xchunk, a.nx - xa);
   const size_t blk = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+  // this CTA's share of the nine (dx, dz) groups
+  const int g_lo = 9 * blockIdx.z / gridDim.z, g_hi = 9 * (blockIdx.z + 1) / gridDim.z;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 13; i++) tc::mbar_init(bar(i), 1);
@@ -415,6 +417,7 @@ __global__ void __launch_bounds__(192, 1)
         const uint64_t g_d = gdesc + (uint64_t)((t & 1) * (G_TILE >> 4));
 #pragma unroll
         for (int g = 0; g < 9; g++) {
+          if (g < g_lo || g >= g_hi) continue;
           const int dx = g / 3, dz = g % 3;
           const uint64_t x_d = xp[dx] + (uint64_t)((dz * WG_COPY) >> 4);
 #pragma unroll
@@ -435,7 +438,7 @@ __global__ void __launch_bounds__(192, 1)
     if (!warp_wait(bar(DONE), 0, a.spin, abort_flag)) ok = false;
     if (ok && !*abort_flag) {
       tc::fence_after_sync();
-      for (int g = 0; g < 9; g++) {
+      for (int g = g_lo; g < g_hi; g++) {
         float v[32];
         tc::tmem_ld_32x32(tmem + ((uint32_t)(ew * 32) << 16) + g * 32, v);
         const int dy = ew;
@@ -696,12 +699,20 @@ __global__ void k_bias_partial(const bf16 *g, float *part, int nx, int ny, int n
     part[blockIdx.x * 32 + threadIdx.x] = t;
   }
 }
-__global__ void k_bias_total(const float *part, int nblk, float *db) {
-  const int c = threadIdx.x;
-  if (c >= 32) return;
+// (1024 threads fetch 256 blocks' partial sums at a time for the 32 that add
+// them up in order: 4.2 us with one warp's dependent loads)
+__global__ void __launch_bounds__(1024) k_bias_total(const float *part, int nblk, float *db) {
+  __shared__ float v[256 * 32];
   float t = 0.f;
-  for (int b = 0; b < nblk; b++) t += part[b * 32 + c];
-  db[c] = t;
+  for (int b0 = 0; b0 < nblk; b0 += 256) {
+    const int n = min(256, nblk - b0) * 32;
+    for (int e = threadIdx.x; e < n; e += blockDim.x) v[e] = part[b0 * 32 + e];
+    __syncthreads();
+    if (threadIdx.x < 32)
+      for (int e = threadIdx.x; e < n; e += 32) t += v[e];
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) db[threadIdx.x] = t;
 }
 
 // BF16 copies of the float32 master weights: forward [27][cout][cin] and
@@ -711,26 +722,40 @@ __global__ void k_bias_total(const float *part, int nblk, float *db) {
 // 3 (3 dy + dz) + dx: the three dx taps of one (dy, dz) are 96 consecutive
 // rows (output channel, 32 input channels), the N = 96 B operand of k_conv
 __device__ __forceinline__ int wblock(int t) { return ((t / 3) % 3 * 3 + t % 3) * 3 + t / 9; }
-__global__ void k_prep_weights(const float *W, bf16 *wf, bf16 *wt) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 27 * 1024) return;
+__device__ __forceinline__ void prep_weight(int e, float w, bf16 *wf, bf16 *wt) {
   const int t = e / 1024, co = (e / 32) % 32, ci = e % 32;
-  const bf16 h = __float2bfloat16_rn(W[e]);
+  const bf16 h = __float2bfloat16_rn(w);
   wf[wblock(t) * 1024 + co * 32 + ci] = h;
   wt[wblock(26 - t) * 1024 + ci * 32 + co] = h;
 }
 
+// the five layers' parameters, gradients, moments and BF16 copies
+struct LayerPtrs {
+  float *W[NL], *b[NL], *dW[NL], *db[NL], *mW[NL], *vW[NL], *mb[NL], *vb[NL];
+  bf16 *wf[NL], *wt[NL];
+};
+__global__ void k_prep_weights(LayerPtrs p) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y;
+  if (e < 27 * 1024) prep_weight(e, p.W[l][e], p.wf[l], p.wt[l]);
+}
+
 // Adam (Kingma & Ba 2015), bias-corrected, float32
-__global__ void k_adam(float *p, const float *g, float *m, float *v, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const float gg = g[e];
-  const float mm = b1 * m[e] + (1.f - b1) * gg;
-  const float vv = b2 * v[e] + (1.f - b2) * gg * gg;
-  m[e] = mm;
-  v[e] = vv;
-  p[e] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+__device__ __forceinline__ float adam(float &p, float gg, float &m, float &v, float lr, float b1, float b2, float eps,
+                                      float c1, float c2) {
+  const float mm = b1 * m + (1.f - b1) * gg;
+  const float vv = b2 * v + (1.f - b2) * gg * gg;
+  m = mm;
+  v = vv;
+  p -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+  return p;
+}
+// one launch for every layer (blockIdx.y) and its biases, with the BF16
+// copies of the new weights
+__global__ void k_adam(LayerPtrs p, float lr, float b1, float b2, float eps, float c1, float c2) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y;
+  if (e < 27 * 1024)
+    prep_weight(e, adam(p.W[l][e], p.dW[l][e], p.mW[l][e], p.vW[l][e], lr, b1, b2, eps, c1, c2), p.wf[l], p.wt[l]);
+  if (e < 32) adam(p.b[l][e], p.db[l][e], p.mb[l][e], p.vb[l][e], lr, b1, b2, eps, c1, c2);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -790,7 +815,9 @@ struct cgli_cnn {
   float *out8 = nullptr, *t8 = nullptr, *partial = nullptr, *bpart = nullptr, *loss = nullptr;
   double *blk_loss = nullptr;
   int *status = nullptr;
-  int xchunk = 0, nblk_cols = 0, nblk_x = 0, nbias = 0;
+  // x planes per CTA of the convolutions and of the weight gradient, and the
+  // CTAs that share the weight gradient's nine (dx, dz) groups of a chunk
+  int xchunk = 0, wchunk = 0, wsplit = 1, nblk_cols = 0, nbias = 0;
   bool training = false;
   Scales sc{};
   int adam_step = 0;
@@ -829,12 +856,43 @@ int calloc_dev(cgli_cnn *n, size_t bytes, void **out) {
 
 int act_alloc(cgli_cnn *n, bf16 **p) { return calloc_dev(n, (size_t)n->padded * ROW, (void **)p); }
 
+dim3 conv_grid(const cgli_cnn *n) { return dim3(n->nblk_cols, (n->nx + n->xchunk - 1) / n->xchunk); }
+dim3 wgrad_grid(const cgli_cnn *n) { return dim3(n->nblk_cols, (n->nx + n->wchunk - 1) / n->wchunk, n->wsplit); }
+int wgrad_blocks(const cgli_cnn *n) { return (int)(wgrad_grid(n).x * wgrad_grid(n).y); }   // chunks
+
+// Planes per CTA of a kernel with `cols` columns and one CTA per SM: the
+// fewest plane loads in a row on one SM, waves x (chunk + 2 halo planes + 3,
+// the cost of a CTA's start: its weights, barriers and TMEM).  (One fixed
+// chunk of 32 left half the chip idle at 64^3, 64 CTAs; there 16 planes take
+// 30.4 against 52.3 us a hidden layer, 46.9 against 83 its input gradient.)
+int best_chunk(int nx, int cols, int sms) {
+  int best = 1;
+  long long least = -1;
+  for (int x = 1; x <= nx; x++) {
+    const long long ctas = (long long)cols * ((nx + x - 1) / x), cost = (ctas + sms - 1) / sms * (x + 5);
+    if (least < 0 || cost < least) { least = cost; best = x; }
+  }
+  return best;
+}
+// CTAs per chunk of the weight gradient: the fewest groups in a row on one SM,
+// 3 more per CTA for the planes that each of them loads (the chunk itself
+// stays, so that every sum keeps its order): at 64^3, 64 chunks, two CTAs a
+// chunk take 64.7 us, one 84, nine 140
+int best_split(int ctas, int sms) {
+  int best = 1, least = 1 << 30;
+  for (int z = 1; z <= 9; z++) {
+    const int cost = (ctas * z + sms - 1) / sms * ((9 + z - 1) / z + 3);
+    if (cost < least) { least = cost; best = z; }
+  }
+  return best;
+}
+
 int ensure_training(cgli_cnn *n) {
   if (n->training) return CGLI_OK;
   int rc = CGLI_OK;
   for (int l = 0; l < NL - 1 && !rc; l++) rc = act_alloc(n, &n->z[l]);
   for (int i = 0; i < 2 && !rc; i++) rc = act_alloc(n, &n->g[i]);
-  if (!rc) rc = calloc_dev(n, (size_t)n->nblk_cols * n->nblk_x * 27 * 1024 * sizeof(float), (void **)&n->partial);
+  if (!rc) rc = calloc_dev(n, (size_t)wgrad_blocks(n) * 27 * 1024 * sizeof(float), (void **)&n->partial);
   if (!rc) rc = calloc_dev(n, (size_t)n->cells * 8 * sizeof(float), (void **)&n->t8);
   if (rc) return rc;
   for (int i = 0; i < 2; i++)
@@ -854,8 +912,6 @@ int check_status(cgli_cnn *n, cudaStream_t s) {
   }
   return CGLI_OK;
 }
-
-dim3 conv_grid(const cgli_cnn *n) { return dim3(n->nblk_cols, n->nblk_x); }
 
 void launch_halo(cgli_cnn *n, bf16 *buf, cudaStream_t s) {
   const long long work = (long long)n->nx * n->ny * 2 + 2LL * n->ny * (n->nz + 2);
@@ -888,8 +944,17 @@ void forward(cgli_cnn *n, bool train, cudaStream_t s) {
   }
 }
 
+LayerPtrs layer_ptrs(const cgli_cnn *n) {
+  LayerPtrs p;
+  for (int l = 0; l < NL; l++) {
+    p.W[l] = n->W[l]; p.b[l] = n->b[l]; p.dW[l] = n->dW[l]; p.db[l] = n->db[l];
+    p.mW[l] = n->mW[l]; p.vW[l] = n->vW[l]; p.mb[l] = n->mb[l]; p.vb[l] = n->vb[l];
+    p.wf[l] = n->wf[l]; p.wt[l] = n->wt[l];
+  }
+  return p;
+}
 void prep_weights(cgli_cnn *n, cudaStream_t s) {
-  for (int l = 0; l < NL; l++) k_prep_weights<<<(27 * 1024 + 255) / 256, 256, 0, s>>>(n->W[l], n->wf[l], n->wt[l]);
+  k_prep_weights<<<dim3((27 * 1024 + 255) / 256, NL), 256, 0, s>>>(layer_ptrs(n));
 }
 
 // loss on out8 vs t8, gradients of every layer into dW/db
@@ -900,15 +965,15 @@ void backward(cgli_cnn *n, cudaStream_t s) {
   k_sum_loss<<<1, 256, 0, s>>>(n->blk_loss, lb, cells, n->loss);
   launch_halo(n, n->g[0], s);
   int cur = 0;
-  const int nblk = n->nblk_cols * n->nblk_x;
+  const int nblk = wgrad_blocks(n);
   for (int l = NL - 1; l >= 0; l--) {
     WgradArgs w{};
-    w.partial = n->partial; w.nx = n->nx; w.ny = n->ny; w.nz = n->nz; w.xchunk = n->xchunk; w.spin = SPIN;
+    w.partial = n->partial; w.nx = n->nx; w.ny = n->ny; w.nz = n->nz; w.xchunk = n->wchunk; w.spin = SPIN;
     w.status = n->status;
-    k_wgrad<<<conv_grid(n), 192, WGRAD_SMEM, s>>>(n->act7[l], n->g4[cur], w);
+    k_wgrad<<<wgrad_grid(n), 192, WGRAD_SMEM, s>>>(n->act7[l], n->g4[cur], w);
     k_reduce_wgrad<<<(27 * 1024 + 255) / 256, 256, 0, s>>>(n->partial, nblk, n->dW[l]);
     k_bias_partial<<<n->nbias, 256, 0, s>>>(n->g[cur], n->bpart, n->nx, n->ny, n->nz);
-    k_bias_total<<<1, 32, 0, s>>>(n->bpart, n->nbias, n->db[l]);
+    k_bias_total<<<1, 1024, 0, s>>>(n->bpart, n->nbias, n->db[l]);
     if (l > 0) {
       ConvArgs a = conv_args(n);
       a.act_out = n->g[cur ^ 1];
@@ -924,11 +989,7 @@ void adam_step(cgli_cnn *n, float lr, cudaStream_t s) {
   n->adam_step++;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const float c1 = 1.f - powf(b1, (float)n->adam_step), c2 = 1.f - powf(b2, (float)n->adam_step);
-  for (int l = 0; l < NL; l++) {
-    k_adam<<<(27 * 1024 + 255) / 256, 256, 0, s>>>(n->W[l], n->dW[l], n->mW[l], n->vW[l], 27 * 1024, lr, b1, b2, eps, c1, c2);
-    k_adam<<<1, 32, 0, s>>>(n->b[l], n->db[l], n->mb[l], n->vb[l], 32, lr, b1, b2, eps, c1, c2);
-  }
-  prep_weights(n, s);
+  k_adam<<<dim3((27 * 1024 + 255) / 256, NL), 256, 0, s>>>(layer_ptrs(n), lr, b1, b2, eps, c1, c2);
 }
 
 int set_smem_attrs() {
@@ -1005,9 +1066,12 @@ int cgli_cnn_create(int nx, int ny, int nz, cgli_cnn **out) {
   cudaGetDevice(&n->device);
   n->cells = (long long)nx * ny * nz;
   n->padded = (long long)(nx + 2) * (ny + 2) * (nz + 2);
-  n->xchunk = nx <= 32 ? nx : 32;
   n->nblk_cols = (ny / 4) * (nz / 32);
-  n->nblk_x = (nx + n->xchunk - 1) / n->xchunk;
+  int sms = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device);
+  n->xchunk = best_chunk(nx, n->nblk_cols, sms);
+  n->wchunk = nx <= 32 ? nx : 32;
+  n->wsplit = best_split(n->nblk_cols * ((nx + n->wchunk - 1) / n->wchunk), sms);
   n->nbias = 296;
   if (cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete n;
