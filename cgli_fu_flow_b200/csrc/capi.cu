@@ -125,6 +125,12 @@ int ensure_filter(cgli_ctx *c) {
   return rc;
 }
 
+// the coefficient records of the DP-LUR relaxations, on first use
+int ensure_dplur(cgli_ctx *c) {
+  if (c->sw.drec) return CGLI_OK;
+  return alloc(c, (size_t)cgli::REC_N * c->d.X * c->d.di * sizeof(double), (void **)&c->sw.drec);
+}
+
 // device array of a reference name; *is_metric tells whether it is one of
 // the 40 metric arrays
 double *lookup(cgli_ctx *c, const char *name, bool *is_metric = nullptr) {
@@ -756,6 +762,7 @@ int cgli_dplusgs(cgli_ctx *c, double er[5]) {
   rc = need_ready(c); if (rc) return rc;
   if (!er) return fail(CGLI_EINVAL, "null er");
   if (c->p.precision != CGLI_FP64) return fail(CGLI_EINVAL, "DP-LUR needs precision CGLI_FP64");
+  rc = ensure_dplur(c); if (rc) return rc;
   cgli::launch_dplur(c->d, c->sw, c->stream);
   rc = last_launch("dplusgs"); if (rc) return rc;
   return read_norms(c, er, c->update_blocks);
@@ -767,6 +774,7 @@ int cgli_set_inner_solver(cgli_ctx *c, int solver) {
     return fail(CGLI_EINVAL, "inner solver must be CGLI_LUSGS or CGLI_DPLUR");
   if (solver == CGLI_DPLUR && c->p.precision != CGLI_FP64)
     return fail(CGLI_EINVAL, "DP-LUR needs precision CGLI_FP64");
+  if (solver == CGLI_DPLUR) { rc = ensure_dplur(c); if (rc) return rc; }
   if (solver != c->inner_solver) drop_graph(c);
   c->inner_solver = solver;
   return CGLI_OK;

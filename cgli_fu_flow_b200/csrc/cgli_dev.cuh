@@ -467,78 +467,6 @@ __device__ __forceinline__ void block_sum5(double acc[5], double *out) {
 }
 
 // ---------------------------------------------------------------------------
-// Coefficients of the LU-SGS sweeps with each division by a repeated divisor
-// replaced by one reciprocal and multiplications (the reference divides every
-// time; results differ from it by rounding only).  Used by the wavefront
-// sweeps, where these quantities are formed once per cell and pass.
-template <typename T>
-struct SweepCoef {
-  T d11, d22, d51;           // own diagonal, Dual_time_stepping.cpp:887-895
-  Split<T> A[3];             // split Jacobians in x, y, z (A+ entries and A- diagonals)
-  T rho, u, v, w, P, Tt;     // primitive state (for the update)
-};
-
-template <typename T>
-__device__ __forceinline__ Split<T> split_fast(T beta, T C, T P, T Tt, T rrho, T u, T v, T w, T mx, T my, T mz,
-                                               bool xdir, T &lam) {
-  const T K = (T)KG;
-  Split<T> a;
-  T U = mx * u + my * v + mz * w;
-  T S = sqrt(U * U * (beta - 1) * (beta - 1) + 4 * beta * C * (mx * mx + my * my + mz * mz));
-  T lambdaX = ((beta + 1) * fabs(U) + S) * (T)0.5;
-  lam = lambdaX;
-  T dd = fabs(lambdaX);
-  T hPKb = (T)0.5 * P * K * beta;
-  a.p11 = (T)0.5 * (beta * U + dd);
-  a.p12 = hPKb * mx;
-  a.p13 = hPKb * my;
-  a.p14 = hPKb * mz;
-  T hr = (T)0.5 * rrho;
-  a.p21 = hr * mx;
-  a.p22 = (T)0.5 * (U + dd);
-  a.p31 = hr * my;
-  a.p41 = hr * mz;
-  a.p51 = (T)0.5 * U * (K - 1) * (beta - 1) * rrho * (T)(1.0 / KG);
-  T hbT = xdir ? (T)0.5 * beta * Tt * (K - 1) : (T)0.5 * beta * Tt * (K - 1);
-  a.p52 = hbT * mx;
-  a.p53 = hbT * my;
-  a.p54 = hbT * mz;
-  a.m11 = (T)0.5 * (beta * U - dd);
-  a.m22 = (T)0.5 * (U - dd);
-  return a;
-}
-
-// q1..q5 = Q/J of the cell, J its Jacobian, mm its nine metric terms;
-// rdx = 1/deltaXI etc.
-template <typename T>
-__device__ __forceinline__ void sweep_coef(T q1, T q2, T q3, T q4, T q5, T J, const T mm[9], T e, T rdx, T rdy,
-                                           T rdz, T dt, SweepCoef<T> &c) {
-  const T K = (T)KG;
-  T rq1 = (T)1 / q1;
-  T rho = q1 * J;
-  T u = q2 * rq1, v = q3 * rq1, w = q4 * rq1;
-  T VV = u * u + v * v + w * w;
-  T P = (q5 * J - (T)0.5 * rho * VV) * (K - 1);
-  T rrho = (T)1 / rho;
-  T C = K * P * rrho;
-  T Tt = P * rrho;
-  T th = VV / C;
-  T beta = th > e ? th : e;
-  T lx, ly, lz;
-  c.A[0] = split_fast<T>(beta, C, P, Tt, rrho, u, v, w, mm[0], mm[1], mm[2], true, lx);
-  c.A[1] = split_fast<T>(beta, C, P, Tt, rrho, u, v, w, mm[3], mm[4], mm[5], false, ly);
-  c.A[2] = split_fast<T>(beta, C, P, Tt, rrho, u, v, w, mm[6], mm[7], mm[8], false, lz);
-  T lambda = lx * rdx + ly * rdy + lz * rdz;
-  T ld = 2 * lambda * dt;
-  T a1 = (T)1 / (3 * beta + ld);
-  T a2 = (T)1 / (3 + ld);
-  c.d11 = 2 * dt * a1;
-  c.d22 = 2 * dt * a2;
-  c.d51 = -(6 * (K - 1) * (beta - 1) * dt) * (a1 * a2) * rrho * (T)(1.0 / KG);
-  c.rho = rho; c.u = u; c.v = v; c.w = w; c.P = P; c.Tt = Tt;
-}
-
-// ---------------------------------------------------------------------------
 // Compact per-cell record of everything the sweeps need, formed once per inner
 // iteration by the residual kernel (the coefficients are the same in all four
 // passes).  With the face metric (mx, my, mz) of a direction the split

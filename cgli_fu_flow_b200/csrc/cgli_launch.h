@@ -56,6 +56,7 @@ struct SweepArgs {
   unsigned int *ticket;           // tile ticket counters of the two passes
   unsigned long long *clock;      // [0] %globaltimer at the first pass, [1] at the update; [2] iterations run
   const int *order;               // tile visiting order
+  double *drec;                   // DP-LUR: REC_N fields of coefficient records, reference layout (on first use)
   const double *Jtab, *etdytab;   // per-j metrics of a grid uniform in x and z
   int channel_metrics;            // 1: use Jtab / etdytab instead of the 3-D arrays
   int spin_limit;                 // bounded wait (polls) for a neighbouring tile
@@ -108,8 +109,6 @@ void launch_dts_residual(const Dev &d, cudaStream_t s);
 // sums of the squared squared increments in d.partial (nx * ny blocks).
 // Reads the per-j metric tables of sw when sw.channel_metrics is set.
 void launch_dplur(const Dev &d, const SweepArgs &sw, cudaStream_t s);
-// one relaxation NR -> NL (from_nr) or NL -> NR
-void launch_dplur_relax(const Dev &d, const SweepArgs &sw, cudaStream_t s, bool from_nr);
 // residual assembly writing MR and the first sweep's lagged halo planes
 void launch_residual_fast(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed);
 

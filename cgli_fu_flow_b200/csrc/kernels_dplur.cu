@@ -2,216 +2,123 @@
 // split-Jacobian operator of the LU-SGS sweeps, then the primitive-variable
 // update with the pressure increment as the first norm.
 //
-// A relaxation is a 7-point stencil with no ordering between cells, so it is
-// a plain data-parallel kernel.  Each CTA owns a (j, k) tile of TJ rows x 30
-// columns and marches through a chunk of x planes.  Every cell forms its own
-// split Jacobians once per plane and applies them to its own previous
-// iterate: the "lower" product A+ NL (used by the neighbour above it) and the
-// "upper" product A* NL (used by the neighbour below it) in each direction.
-// Neighbours exchange those products instead of re-forming each other's
-// Jacobians: along k by warp shuffles (one warp per j row, lanes 0 and 31
-// the halo columns), along j through shared memory (two extra halo rows),
-// along x in registers (the march).  A cell outside the interior contributes
-// nothing, which is the reference's zero NL ghost rows (DPLUSGS.cpp:190-318).
+// A relaxation is a 7-point stencil with no ordering between cells: a thread
+// per cell gathers the product of each neighbour's split Jacobian with that
+// neighbour's previous iterate.  The split Jacobians come from the coefficient
+// record of the LU-SGS sweeps (make_record), formed once per inner iteration
+// by the residual kernel, so that a product is ten loads and some 25 FP64
+// operations and the kernel needs no exchange between threads.  A cell outside
+// the interior contributes nothing, which is the reference's zero NL ghost
+// rows (DPLUSGS.cpp:190-318).
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
 
 namespace cgli {
 
-namespace {
-
-constexpr int RELAX_TK = 30;     // interior columns per warp (lanes 1..30)
-
-}  // namespace
-
 struct RelaxPtrs {
   const double *src[5];
   double *dst[5];
+  double *rec;                    // [REC_N] fields of coefficient records
+  long long n;                    // words of a field
+  double rdt;                     // 1 / deltaT
   const double *Jtab, *etdytab;   // per-j J and etdy of a grid uniform in x and z
 };
 
-__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-
-template <int TJ, bool CH>
-constexpr size_t relax_smem() {
-  return sizeof(double) * (2 * (TJ + 2) * 10 * 32 + 2 * (CH ? 15 : 25) * (TJ + 2) * 32);
+// The product of one direction that cell c's neighbour sees, -A+ n (UP: A* n),
+// from the record of cell c and the iterate of cell cn (c, or its periodic
+// image); m, q: the face metric of the cell's row and the component of it that
+// is not zero on the channel grid (CH)
+template <int DIR, bool UP, bool CH>
+__device__ __forceinline__ void product(const Dev &d, const RelaxPtrs &a, long long c, long long cn, double m, double o[5]) {
+  constexpr int q = DIR + 1;
+  double r[REC_N], n[5];
+  for (int v : {(int)R_BETA, (int)R_H, (int)R_HR, (int)R_UX + DIR, (int)R_LX + DIR}) r[v] = a.rec[v * a.n + c];
+#pragma unroll
+  for (int v = 0; v < 5; v++) n[v] = a.src[v][cn];
+  if (CH) {
+    const double U = 0.5 * r[R_UX + DIR], l = 0.5 * r[R_LX + DIR], bU = r[R_BETA] * U;
+    const double a0 = r[R_H] * m * n[q], aq = r[R_HR] * m * n[0];
+    const double a4 = rec_g<double>(r) * r[R_UX + DIR] * n[0] + rec_hbt<double>(r) * m * n[q];
+    const double p = UP ? U - l : -(U + l);
+    o[0] = UP ? (bU - l) * n[0] + a0 : -(bU + l) * n[0] - a0;
+#pragma unroll
+    for (int v = 1; v <= 3; v++) o[v] = p * n[v];
+    o[q] += UP ? aq : -aq;
+    o[4] = UP ? p * n[4] + a4 : p * n[4] - a4;
+  } else {
+    const Split<double> A = split_from_record<double>(r, DIR, d.m[3 * DIR][c], d.m[3 * DIR + 1][c], d.m[3 * DIR + 2][c]);
+    if (UP) upper_terms<double>(A, n, o); else lower_terms<double>(A, n, o);
+  }
 }
 
 // One Jacobi relaxation, DPLUSGS.cpp:488-1141: dst = D^-1 (MR - LL(src) -
-// UU(src)) on planes [ilo, ihi] of this CTA's chunk; src on planes 2 and
-// ie+1 is read at its periodic images ie and 3 (the self-copy exchange of
-// :510-531).  The diagonal is that of DPLUSGS.cpp:1068-1107 (inviscid).
-// Each thread copies its cell's inputs of the next plane into shared memory
-// with cp.async while it computes the current plane.  CH: the metrics are
-// those of a grid uniform in x and z, read per row from Jtab / etdytab.
-template <int TJ, bool CH>
-__global__ void __launch_bounds__((TJ + 2) * 32, TJ <= 6 ? 2 : 1) k_dplur_relax(Dev d, RelaxPtrs a, int chunk) {
-  constexpr int NT = (TJ + 2) * 32;
-  constexpr int NV = CH ? 15 : 25;          // staged doubles per cell: U_, src, MR (+ J, 9 metrics)
-  extern __shared__ double sm[];
-  double *const ysm = sm;                   // [2 buffers][TJ+2 rows][10 values][32 lanes]
-  double *const stg = sm + 2 * (TJ + 2) * 10 * 32;   // [2 stages][NV][NT]
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int j = 1 + blockIdx.y * TJ + w;
-  const int k = 1 + blockIdx.x * RELAX_TK + lane;
-  const int ie = d.nx + 2, jn = d.ny + 1, kn = d.nz + 1;
-  const int ilo = 3 + blockIdx.z * chunk;
-  const int ihi = min(ie, ilo + chunk - 1);
-  const bool active = j >= 2 && j <= jn && k >= 2 && k <= kn;
-  const bool row = w >= 1 && w <= TJ;                       // an interior row of the tile
-  const bool out = active && row && lane >= 1 && lane <= RELAX_TK;
-  const double idx = 1.0 / d.dxi, idy = 1.0 / d.det, idz = 1.0 / d.dzt;
-  const double dt = d.dt;
-  double Jc = 0, etc = 0;
-  if (CH && active) { Jc = a.Jtab[j]; etc = a.etdytab[j]; }
-
-  auto issue = [&](int p) {
-    const bool edge = p < ilo || p > ihi;
-    if (!active || (!row && edge)) return;
-    const long long c = ix(d, p, j, k);
-    const int pn = p == 2 ? ie : (p == ie + 1 ? 3 : p);
-    const long long cn = ix(d, pn, j, k);
-    double *s = stg + (size_t)(p & 1) * NV * NT + tid;
+// UU(src)) on the interior; src on planes 2 and ie+1 is read at its periodic
+// images ie and 3 (the self-copy exchange of :510-531).  The diagonal is that
+// of DPLUSGS.cpp:1068-1107 (inviscid).  CH: the metrics are those of a grid
+// uniform in x and z, read per row from etdytab.
+// Bound by the loads: 26 words a cell from memory (38 us at 128x96x96), the
+// neighbours' from L1 (along j and k, blocks of 8 rows) and L2 (along x), four
+// blocks a SM to cover their latency.  128x96x96: 53.5 us, where tiles that
+// marched along x, staged the state in shared memory and formed each split
+// Jacobian once took 116 (two CTAs a SM, one plane's latency after another).
+template <bool CH>
+__global__ void __launch_bounds__(256, 4) k_dplur_relax(Dev d, RelaxPtrs a) {
+  const int k = 2 + blockIdx.x * 32 + (threadIdx.x & 31);
+  const int j = 2 + blockIdx.y * 8 + (threadIdx.x >> 5);
+  const int i = 3 + blockIdx.z;
+  const int ie = d.nx + 2;
+  if (k > d.nz + 1 || j > d.ny + 1) return;
+  const long long c = ix(d, i, j, k);
+  const double idx = d.rdxi, idy = d.rdet, idz = d.rdzt;
+  double o[5], LL[5] = {0, 0, 0, 0, 0}, UU[5] = {0, 0, 0, 0, 0}, ux[5] = {0, 0, 0, 0, 0};
+  // an open slab's end planes hold zero iterates (DPLUSGS.cpp:191-233)
+  if (!(d.x_open && i == 3)) {
+    product<0, false, CH>(d, a, c - d.di, i == 3 ? ix(d, ie, j, k) : c - d.di, 1.0, o);
 #pragma unroll
-    for (int v = 0; v < 5; v++) cp_async8(s + v * NT, d.U_[v] + c);
-#pragma unroll
-    for (int v = 0; v < 5; v++) cp_async8(s + (5 + v) * NT, a.src[v] + cn);
-    if (out && !edge) {
-#pragma unroll
-      for (int v = 0; v < 5; v++) cp_async8(s + (10 + v) * NT, d.MR[v] + c);
-    }
-    if (!CH) {
-      cp_async8(s + 15 * NT, d.J + c);
-#pragma unroll
-      for (int v = 0; v < 9; v++) cp_async8(s + (16 + v) * NT, d.m[v] + c);
-    }
-  };
-
-  double lxp[5] = {0, 0, 0, 0, 0};   // lower x product of plane p-1
-  double part[5] = {0, 0, 0, 0, 0};  // MR - LL - UU(y, z) of plane p-1
-  double d11 = 0, d22 = 0, d51 = 0;  // diagonal of plane p-1
-  issue(ilo - 1);
-  cp_async_commit();
-  for (int p = ilo - 1; p <= ihi + 1; p++) {
-    if (p + 1 <= ihi + 1) issue(p + 1);
-    cp_async_commit();
-    cp_async_wait1();                        // this thread's copies of plane p have landed
-    const bool edge = p < ilo || p > ihi;    // only the x products are needed
-    double lx[5] = {0, 0, 0, 0, 0}, ux[5] = {0, 0, 0, 0, 0};
-    double ly[5] = {0, 0, 0, 0, 0}, uy[5] = {0, 0, 0, 0, 0};
-    double lz[5] = {0, 0, 0, 0, 0}, uz[5] = {0, 0, 0, 0, 0};
-    double mr[5] = {0, 0, 0, 0, 0};
-    double c11 = 0, c22 = 0, c51 = 0;      // diagonal of plane p
-    if (active && (row || !edge)) {
-      const double *s = stg + (size_t)(p & 1) * NV * NT + tid;
-      double mm[9], J;
-      if (CH) {
-        J = Jc;
-        mm[0] = 1; mm[1] = 0; mm[2] = 0; mm[3] = 0; mm[4] = etc; mm[5] = 0; mm[6] = 0; mm[7] = 0; mm[8] = 1;
-      } else {
-        J = s[15 * NT];
-#pragma unroll
-        for (int v = 0; v < 9; v++) mm[v] = s[(16 + v) * NT];
-      }
-      double n[5];
-      // an open slab's end planes hold zero iterates (DPLUSGS.cpp:191-233)
-      const bool zero_end = d.x_open && (p == 2 || p == ie + 1);
-#pragma unroll
-      for (int v = 0; v < 5; v++) n[v] = zero_end ? 0.0 : s[(5 + v) * NT];
-      if (row) {
-        // the cell's three split Jacobians and its diagonal, each repeated
-        // divisor as one reciprocal
-        SweepCoef<double> sc;
-        sweep_coef<double>(s[0], s[NT], s[2 * NT], s[3 * NT], s[4 * NT], J, mm, d.e, idx, idy, idz, dt, sc);
-        lower_terms<double>(sc.A[0], n, lx);
-        upper_terms<double>(sc.A[0], n, ux);
-        if (!edge) {
-          lower_terms<double>(sc.A[1], n, ly);
-          upper_terms<double>(sc.A[1], n, uy);
-          lower_terms<double>(sc.A[2], n, lz);
-          upper_terms<double>(sc.A[2], n, uz);
-          c11 = sc.d11; c22 = sc.d22; c51 = sc.d51;
-        }
-      } else {
-        // a halo row: only its y products are used
-        const double rq1 = 1 / s[0], rho = s[0] * J;
-        const double u = s[NT] * rq1, v = s[2 * NT] * rq1, w = s[3 * NT] * rq1;
-        const double VV = u * u + v * v + w * w;
-        const double P = (s[4 * NT] * J - 0.5 * rho * VV) * (KG - 1);
-        const double rrho = 1 / rho, C = KG * P * rrho, Tt = P * rrho, th = VV / C;
-        const double beta = th > d.e ? th : d.e;
-        double lam;
-        const Split<double> sy = split_fast<double>(beta, C, P, Tt, rrho, u, v, w, mm[3], mm[4], mm[5], false, lam);
-        lower_terms<double>(sy, n, ly);
-        upper_terms<double>(sy, n, uy);
-      }
-      if (out && !edge) {
-#pragma unroll
-        for (int v = 0; v < 5; v++) mr[v] = s[(10 + v) * NT];
-      }
-    }
-    // finish plane p-1 with the upper x product of plane p
-    if (out && p - 1 >= ilo) {
-      const long long c = ix(d, p - 1, j, k);
-      double r[5];
-#pragma unroll
-      for (int v = 0; v < 5; v++) r[v] = part[v] - ux[v] * idx;
-      a.dst[0][c] = d11 * r[0];
-      a.dst[1][c] = d22 * r[1];
-      a.dst[2][c] = d22 * r[2];
-      a.dst[3][c] = d22 * r[3];
-      a.dst[4][c] = d51 * r[0] + d22 * r[4];
-    }
-    if (edge) {
-#pragma unroll
-      for (int v = 0; v < 5; v++) lxp[v] = lx[v];
-      continue;   // p is the same for every thread of the CTA
-    }
-    // k neighbours by shuffles: lower product of k-1, upper product of k+1
-    double lzm[5], uzp[5];
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-      lzm[v] = __shfl_up_sync(0xffffffffu, lz[v], 1);
-      uzp[v] = __shfl_down_sync(0xffffffffu, uz[v], 1);
-    }
-    // j neighbours through shared memory
-    double *buf = ysm + (size_t)(p & 1) * (TJ + 2) * 10 * 32;
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-      buf[(w * 10 + v) * 32 + lane] = ly[v];
-      buf[(w * 10 + 5 + v) * 32 + lane] = uy[v];
-    }
-    __syncthreads();
-    if (out) {
-#pragma unroll
-      for (int v = 0; v < 5; v++) {
-        const double lym = buf[((w - 1) * 10 + v) * 32 + lane];
-        const double uyp = buf[((w + 1) * 10 + 5 + v) * 32 + lane];
-        const double LL = lxp[v] * idx + lym * idy + lzm[v] * idz;
-        const double UUyz = uyp * idy + uzp[v] * idz;
-        part[v] = mr[v] - LL - UUyz;
-      }
-      d11 = c11; d22 = c22; d51 = c51;   // DPLUSGS.cpp:1091-1107
-    }
-#pragma unroll
-    for (int v = 0; v < 5; v++) lxp[v] = lx[v];
+    for (int v = 0; v < 5; v++) LL[v] = o[v] * idx;
   }
+  if (!(d.x_open && i == ie)) product<0, true, CH>(d, a, c + d.di, i == ie ? ix(d, 3, j, k) : c + d.di, 1.0, ux);
+  if (j > 2) {
+    product<1, false, CH>(d, a, c - d.dj, c - d.dj, CH ? a.etdytab[j - 1] : 0.0, o);
+#pragma unroll
+    for (int v = 0; v < 5; v++) LL[v] += o[v] * idy;
+  }
+  if (j < d.ny + 1) {
+    product<1, true, CH>(d, a, c + d.dj, c + d.dj, CH ? a.etdytab[j + 1] : 0.0, o);
+#pragma unroll
+    for (int v = 0; v < 5; v++) UU[v] = o[v] * idy;
+  }
+  if (k > 2) {
+    product<2, false, CH>(d, a, c - 1, c - 1, 1.0, o);
+#pragma unroll
+    for (int v = 0; v < 5; v++) LL[v] += o[v] * idz;
+  }
+  if (k < d.nz + 1) {
+    product<2, true, CH>(d, a, c + 1, c + 1, 1.0, o);
+#pragma unroll
+    for (int v = 0; v < 5; v++) UU[v] += o[v] * idz;
+  }
+  double r[5], rec[REC_N];
+#pragma unroll
+  for (int v = 0; v < 5; v++) r[v] = d.MR[v][c] - LL[v] - UU[v] - ux[v] * idx;
+  for (int v : {(int)R_BETA, (int)R_HR, (int)R_D11, (int)R_D22}) rec[v] = a.rec[v * a.n + c];
+  a.dst[0][c] = rec[R_D11] * r[0];
+  a.dst[1][c] = rec[R_D22] * r[1];
+  a.dst[2][c] = rec[R_D22] * r[2];
+  a.dst[3][c] = rec[R_D22] * r[3];
+  a.dst[4][c] = rec_d51<double>(rec, a.rdt) * r[0] + rec[R_D22] * r[4];
 }
 
 // Residual of DPLUSGS.cpp:324-478 (the same values as Dual_time_stepping.cpp:
 // 737-908 without its zero sponge terms): MR and the first iterate
 // NL = D^-1 MR on the interior cells, with each repeated divisor as one
-// reciprocal.  CH as for the relaxation.
+// (Newton-refined) reciprocal, and the coefficient records of planes 2..ie+1.
+// CH as for the relaxation.
 template <bool CH>
 __global__ void __launch_bounds__(128) k_dplur_residual(Dev d, RelaxPtrs a) {
   int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
   int j = 2 + blockIdx.y;
-  int i = 3 + blockIdx.z;
+  int i = 2 + blockIdx.z;
   if (k > d.nz + 1) return;
   const long long c = ix(d, i, j, k);
   double mm[9], J;
@@ -223,9 +130,15 @@ __global__ void __launch_bounds__(128) k_dplur_residual(Dev d, RelaxPtrs a) {
 #pragma unroll
     for (int v = 0; v < 9; v++) mm[v] = d.m[v][c];
   }
-  const CPrim<double> q = cprim<double>(d.U_[0][c], d.U_[1][c], d.U_[2][c], d.U_[3][c], d.U_[4][c], J, d.e);
+  const double q1 = d.U_[0][c], q2 = d.U_[1][c], q3 = d.U_[2][c], q4 = d.U_[3][c], q5 = d.U_[4][c];
+  double rec[REC_N];
+  make_record(q1, q2, q3, q4, q5, J, mm, d.e, d.rdxi, d.rdet, d.rdzt, d.dt, rec);
+#pragma unroll
+  for (int v = 0; v < REC_N; v++) a.rec[v * a.n + c] = rec[v];
+  if (i == 2 || i == d.nx + 3) return;   // the halo planes enter the products only
+  const CPrim<double> q = cprim<double>(q1, q2, q3, q4, q5, J, d.e);
   const double rho = q.rho, u = q.u, v = q.v, w = q.w, VV = q.VV, T = q.Tt, H = q.H, beta = q.beta;
-  const double irho = 1 / rho, itemp = 1 / (rho * KG);
+  const double irho = nr_rcp(rho), itemp = irho * (1.0 / KG);
   const double d11 = -(H * (KG - 1) + VV - KG * (T + VV)) * beta;
   const double d12 = -(KG - 1) * u * beta, d13 = -(KG - 1) * v * beta, d14 = -(KG - 1) * w * beta;
   const double d15 = (KG - 1) * beta;
@@ -233,12 +146,13 @@ __global__ void __launch_bounds__(128) k_dplur_residual(Dev d, RelaxPtrs a) {
   const double g5 = -(KG - 1) * (1 + (KG - 1) * beta) * itemp;
   const long long fx1 = ix(d, i, j - 1, k - 1), f0 = ix(d, i - 1, j - 1, k - 1);
   const long long fy1 = ix(d, i - 1, j, k - 1), fz1 = ix(d, i - 1, j - 1, k);
-  const double i2dt = 1 / (2 * d.dt), idx = 1 / d.dxi, idy = 1 / d.det, idz = 1 / d.dzt, iJ = 1 / J;
+  const double i2dt = nr_rcp(2 * d.dt), idx = d.rdxi, idy = d.rdet, idz = d.rdzt, iJ = nr_rcp(J);
   const double f = d.scal[0];
+  const double U_[5] = {q1, q2, q3, q4, q5};
   double Rk[5];
 #pragma unroll
   for (int n = 0; n < 5; n++) {
-    const double Rp = -(3 * d.U_[n][c] - 4 * d.U[n][c] + d.Uq[n][c]) * i2dt;
+    const double Rp = -(3 * U_[n] - 4 * d.U[n][c] + d.Uq[n][c]) * i2dt;
     const double Rf = -((d.inF[0][n][fx1] - d.inF[0][n][f0]) * idx + (d.inF[1][n][fy1] - d.inF[1][n][f0]) * idy +
                         (d.inF[2][n][fz1] - d.inF[2][n][f0]) * idz);
     Rk[n] = Rp + Rf;
@@ -253,14 +167,14 @@ __global__ void __launch_bounds__(128) k_dplur_residual(Dev d, RelaxPtrs a) {
   MR[2] = (Rk[2] - v * Rk[0]) * irho;
   MR[3] = (Rk[3] - w * Rk[0]) * irho;
   MR[4] = d51 * Rk[0] + g5 * (u * Rk[1] + v * Rk[2] + w * Rk[3] - Rk[4]);
-  const Diag<double> dg = diag<double>(q, mm, d.dxi, d.det, d.dzt, d.dt);
 #pragma unroll
   for (int n = 0; n < 5; n++) d.MR[n][c] = MR[n];
-  a.dst[0][c] = dg.d11 * MR[0];
-  a.dst[1][c] = dg.d22 * MR[1];
-  a.dst[2][c] = dg.d22 * MR[2];
-  a.dst[3][c] = dg.d22 * MR[3];
-  a.dst[4][c] = dg.d51 * MR[0] + dg.d22 * MR[4];
+  const double g51 = rec_d51<double>(rec, a.rdt);
+  a.dst[0][c] = rec[R_D11] * MR[0];
+  a.dst[1][c] = rec[R_D22] * MR[1];
+  a.dst[2][c] = rec[R_D22] * MR[2];
+  a.dst[3][c] = rec[R_D22] * MR[3];
+  a.dst[4][c] = g51 * MR[0] + rec[R_D22] * MR[4];
 }
 
 // Update of DPLUSGS.cpp:1152-1196 from the last relaxation's result, with
@@ -275,20 +189,21 @@ __global__ void __launch_bounds__(128, 8) k_dplur_update(Dev d, RelaxPtrs a) {
   if (*(volatile int *)d.status) return;   // an iteration before this one failed: keep the state
   for (int kk = k; kk <= d.nz + 1; kk += blockDim.x) {
     long long c = ix(d, i, j, kk);
-    // the divisions by q1, rho, T and J as reciprocals (1/J from the table)
+    // the divisions by q1, rho, T and J as (Newton-refined) reciprocals (1/J
+    // from the table)
     const double J = d.J[c], iJ = d.iJ[c];
-    double q1 = d.U_[0][c], iq1 = 1 / q1;
+    double q1 = d.U_[0][c], iq1 = nr_rcp(q1);
     double rhoold = q1 * J;
     double Uold = d.U_[1][c] * iq1, Vold = d.U_[2][c] * iq1, Wold = d.U_[3][c] * iq1;
     double VVold = Uold * Uold + Vold * Vold + Wold * Wold;
     double Pold = (d.U_[4][c] * J - 0.5 * rhoold * VVold) * (KG - 1);
-    double Told = Pold / rhoold;
+    double Told = Pold * (iq1 * iJ);   // 1 / rho = 1 / (q1 J)
     double P = Pold + nr[0][c] * J;
     double U = Uold + nr[1][c] * J;
     double V = Vold + nr[2][c] * J;
     double W = Wold + nr[3][c] * J;
     double T = Told + nr[4][c] * J;
-    double rho = P / T, rJ = rho * iJ;
+    double rho = P * nr_rcp(T), rJ = rho * iJ;
     d.U_[0][c] = rJ;
     d.U_[1][c] = rJ * U;
     d.U_[2][c] = rJ * V;
@@ -304,17 +219,11 @@ __global__ void __launch_bounds__(128, 8) k_dplur_update(Dev d, RelaxPtrs a) {
 
 namespace {
 
-template <int TJ, bool CH>
-void relax(const Dev &d, const RelaxPtrs &a, cudaStream_t s, int chunk) {
-  constexpr size_t smem = relax_smem<TJ, CH>();
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_dplur_relax<TJ, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 g((d.nz + RELAX_TK - 1) / RELAX_TK, (d.ny + TJ - 1) / TJ, (d.nx + chunk - 1) / chunk);
-  k_dplur_relax<TJ, CH><<<g, (TJ + 2) * 32, smem, s>>>(d, a, chunk);
-}
-
-RelaxPtrs ptrs(double *const *src, double *const *dst, const SweepArgs &sw) {
+RelaxPtrs ptrs(const Dev &d, double *const *src, double *const *dst, const SweepArgs &sw) {
   RelaxPtrs a;
+  a.rec = sw.drec;
+  a.n = (long long)d.X * d.di;
+  a.rdt = 1.0 / d.dt;
   for (int v = 0; v < 5; v++) { a.src[v] = src[v]; a.dst[v] = dst[v]; }
   a.Jtab = sw.Jtab;
   a.etdytab = sw.etdytab;
@@ -323,24 +232,22 @@ RelaxPtrs ptrs(double *const *src, double *const *dst, const SweepArgs &sw) {
 
 }  // namespace
 
-// relaxation tiles of 6 j rows marching over 32 x planes, the shape chosen
-// by measurement at 256x192x192 (14 rows and other plane counts)
-constexpr int kDplurChunk = 32;
-
-void launch_dplur_relax(const Dev &d, const SweepArgs &sw, cudaStream_t s, bool from_nr) {
-  RelaxPtrs a = from_nr ? ptrs(d.NR, d.NL, sw) : ptrs(d.NL, d.NR, sw);
-  if (sw.channel_metrics) relax<6, true>(d, a, s, kDplurChunk);
-  else relax<6, false>(d, a, s, kDplurChunk);
+// one relaxation NR -> NL (from_nr) or NL -> NR
+static void relax(const Dev &d, const SweepArgs &sw, cudaStream_t s, bool from_nr) {
+  const RelaxPtrs a = from_nr ? ptrs(d, d.NR, d.NL, sw) : ptrs(d, d.NL, d.NR, sw);
+  const dim3 g((d.nz + 31) / 32, (d.ny + 7) / 8, d.nx);
+  if (sw.channel_metrics) k_dplur_relax<true><<<g, 256, 0, s>>>(d, a);
+  else k_dplur_relax<false><<<g, 256, 0, s>>>(d, a);
 }
 
 // residual (MR, NR = D^-1 MR), four relaxations NR->NL->NR->NL->NR, update
 void launch_dplur(const Dev &d, const SweepArgs &sw, cudaStream_t s) {
-  RelaxPtrs r = ptrs(d.NL, d.NR, sw);
-  dim3 g((d.nz + 127) / 128, d.ny, d.nx);
+  RelaxPtrs r = ptrs(d, d.NL, d.NR, sw);
+  dim3 g((d.nz + 127) / 128, d.ny, d.nx + 2);
   if (sw.channel_metrics) k_dplur_residual<true><<<g, 128, 0, s>>>(d, r);
   else k_dplur_residual<false><<<g, 128, 0, s>>>(d, r);
-  for (int sweep = 0; sweep < 4; sweep++) launch_dplur_relax(d, sw, s, sweep % 2 == 0);
-  RelaxPtrs a = ptrs(d.NR, d.NL, sw);
+  for (int sweep = 0; sweep < 4; sweep++) relax(d, sw, s, sweep % 2 == 0);
+  RelaxPtrs a = ptrs(d, d.NR, d.NL, sw);
   k_dplur_update<<<dim3(d.ny, d.nx), 128, 0, s>>>(d, a);
 }
 
