@@ -191,11 +191,11 @@ class Clocks:
 
 def launches_per_iteration(ch) -> int:
     """Kernels of one fused LU-SGS inner iteration: x halo, Y and Z boundaries,
-    three fluxes, three viscous kernels, the residual, two sweeps of halo
+    three fluxes, the viscous terms, the residual, two sweeps of halo
     products and two wavefront passes, the update and the norm reduction; an
     open slab adds the X boundary and the sponge target reduction and drops
     the x halo.  A step adds the bulk-flux pair and the time-level shift."""
-    return 18 + (1 if ch.x_open else 0)
+    return 16 + (1 if ch.x_open else 0)
 
 
 def workload_label(ch) -> str:

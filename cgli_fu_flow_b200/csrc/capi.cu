@@ -342,10 +342,7 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
     F(d.U_[v]); F(d.U[v]); F(d.Uq[v]); F(d.Uqq[v]); F(d.MR[v]); F(d.NL[v]); F(d.NR[v]);
     for (int f = 0; f < 3; f++) F(d.inF[f][v]);
   }
-  for (int v = 0; v < 4; v++) {
-    F(d.vF[v]); F(d.vprim[v]);
-    for (int f = 0; f < 3; f++) F(d.vflux[f][v]);
-  }
+  for (int v = 0; v < 4; v++) F(d.vF[v]);
   F(d.J);
   F(d.iJ);
   for (int v = 0; v < 9; v++) F(d.m[v]);

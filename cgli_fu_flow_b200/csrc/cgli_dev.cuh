@@ -41,8 +41,6 @@ struct Dev {
   int face_tables;
   double *inF[3][5], *vF[4];
   double *MR[5], *NL[5], *NR[5];
-  double *vflux[3][4];
-  double *vprim[4];
   double *scal;           // [0] = driving force, [1] = outlet sponge target velocity
   double *partial;        // per-block partial sums of the update norms
   int *status;            // device status word (0 ok)

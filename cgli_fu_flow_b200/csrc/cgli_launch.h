@@ -132,7 +132,10 @@ void launch_bc_z(const Dev &d, cudaStream_t s);
 void launch_flux_x(const Dev &d, cudaStream_t s);
 void launch_flux_y(const Dev &d, cudaStream_t s);
 void launch_flux_z(const Dev &d, cudaStream_t s);
+// Viscous_terms.cpp:260-904: vF of every interior cell (kernels_viscous.cu)
 void launch_viscous(const Dev &d, cudaStream_t s);
+// planes per CTA of a kernel that marches `cols` columns of nx planes
+int march_chunk(int nx, int cols, int resident, int start);
 // residual, sweeps and update of the reference-granularity path; leaves
 // per-block partial sums of the squared increments in d.partial
 void launch_dts(const Dev &d, cudaStream_t s, int update_blocks_x);

@@ -5,17 +5,12 @@
 // cgli_inner_iteration lives in kernels_fused.cu.
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
-#include "viscous_face.cuh"
 
-// CTAs of 64 threads per SM the inviscid flux and the viscous face kernels
-// are compiled for (register caps: 12 CTAs leave the fluxes 80 registers, a
-// few spilled, 18 % faster than the uncapped 116 at 256x192x192; 8 CTAs
-// leave the viscous faces 128, 3 % faster than 154, 10 CTAs are slower)
+// CTAs of 64 threads per SM the inviscid flux kernels are compiled for
+// (register cap: 12 CTAs leave 80 registers, a few spilled, 18 % faster than
+// the uncapped 116 at 256x192x192)
 #ifndef CGLI_FLUX_MINBLOCKS
 #define CGLI_FLUX_MINBLOCKS 12
-#endif
-#ifndef CGLI_VISCOUS_MINBLOCKS
-#define CGLI_VISCOUS_MINBLOCKS 8
 #endif
 
 namespace cgli {
@@ -320,109 +315,6 @@ __global__ void __launch_bounds__(64, CGLI_FLUX_MINBLOCKS) k_flux_z(Dev d) {
   for (int v = 0; v < 5; v++) d.inF[2][v][f] = F[v];
 }
 
-// ---------------------------------------------------------------- viscous
-// velocity and temperature of every cell the viscous face fluxes read
-// (Viscous_terms.cpp:260-394): planes 2..ie+1, rows 1..nyy, k 1..nzz
-__global__ void k_vprim(Dev d) {
-  int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  int j = 1 + blockIdx.y;
-  int i = 2 + blockIdx.z;
-  if (k > d.nz + 2) return;
-  long long c = ix(d, i, j, k);
-  // the divisions by rho, rho R and J as Newton-refined reciprocals
-  double rho = d.U_[0][c], irho = nr_rcp(rho);
-  double U = d.U_[1][c] * irho, V = d.U_[2][c] * irho, W = d.U_[3][c] * irho;
-  double P = (d.U_[4][c] - 0.5 * rho * (U * U + V * V + W * W)) * (KG - 1) * d.J[c];
-  double T = P * (irho * (1.0 / RG)) * nr_rcp(d.J[c]);
-  d.vprim[0][c] = U; d.vprim[1][c] = V; d.vprim[2][c] = W; d.vprim[3][c] = T;
-}
-
-struct VP { double U, V, W, T; };
-__device__ __forceinline__ VP vp(const Dev &d, long long c) {
-  VP r; r.U = d.vprim[0][c]; r.V = d.vprim[1][c]; r.W = d.vprim[2][c]; r.T = d.vprim[3][c]; return r;
-}
-
-// face viscous fluxes of cell (i,j,k): x face i-1/2 for j<=jn, k<=kn; y face
-// j-1/2 for i<=ie, k<=kn; z face k-1/2 for i<=ie, j<=jn (the faces the
-// divergence of Viscous_terms.cpp:875-904 reads).  CH: the face metrics have
-// the channel's form (d.face_tables), so the per-row tables give eta_y and
-// 1/J and the channel forms of the face fluxes apply.
-// (the channel form fits 64 registers without spills: held at 16 CTAs per
-// SM, 32 warps to hide its stencil loads)
-template <bool CH>
-__global__ void __launch_bounds__(64, (CH && CGLI_VISCOUS_MINBLOCKS < 16) ? 16 : CGLI_VISCOUS_MINBLOCKS)
-    k_viscous_faces(Dev d) {
-  int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  int j = 2 + blockIdx.y;
-  int i = 3 + blockIdx.z;
-  int ie = d.nx + 2, jn = d.ny + 1, kn = d.nz + 1;
-  if (k > kn + 1) return;
-  long long c = ix(d, i, j, k);
-  long long f = ix(d, i - 1, j - 1, k - 1);
-  const long long di = d.di, dj = d.dj;
-  VP o = vp(d, c);
-  if (j <= jn && k <= kn) {
-    double out[4];
-    if (CH) {
-      const double *t = d.ftab + (0LL * d.Y + (j - 1)) * 4;
-      visc_face_x_channel(d.rdxi, d.rdet, d.rdzt, d.mu, d.rpr, t[0], o, vp(d, c - di), vp(d, c + dj),
-                          vp(d, c - di + dj), vp(d, c - dj), vp(d, c - di - dj), vp(d, c + 1), vp(d, c - di + 1),
-                          vp(d, c - 1), vp(d, c - di - 1), t[2], out);
-    } else {
-      double mm[9], Jf, iJf;
-      face_metrics(d, 0, f, j - 1, mm, Jf, iJf);
-      visc_face_x(d.rdxi, d.rdet, d.rdzt, d.mu, d.rpr, o, vp(d, c - di), vp(d, c + dj), vp(d, c - di + dj), vp(d, c - dj),
-                  vp(d, c - di - dj), vp(d, c + 1), vp(d, c - di + 1), vp(d, c - 1), vp(d, c - di - 1), mm, iJf, out);
-    }
-    for (int v = 0; v < 4; v++) d.vflux[0][v][c] = out[v];
-  }
-  if (i <= ie && k <= kn) {
-    double out[4];
-    if (CH) {
-      const double *t = d.ftab + (1LL * d.Y + (j - 1)) * 4;
-      visc_face_y_channel(d.rdxi, d.rdet, d.rdzt, d.mu, d.rpr, t[0], o, vp(d, c - dj), vp(d, c + di),
-                          vp(d, c + di - dj), vp(d, c - di), vp(d, c - di - dj), vp(d, c + 1), vp(d, c - dj + 1),
-                          vp(d, c - 1), vp(d, c - dj - 1), t[2], out);
-    } else {
-      double mm[9], Jf, iJf;
-      face_metrics(d, 1, f, j - 1, mm, Jf, iJf);
-      visc_face_y(d.rdxi, d.rdet, d.rdzt, d.mu, d.rpr, o, vp(d, c - dj), vp(d, c + di), vp(d, c + di - dj), vp(d, c - di),
-                  vp(d, c - di - dj), vp(d, c + 1), vp(d, c - dj + 1), vp(d, c - 1), vp(d, c - dj - 1), mm, iJf, out);
-    }
-    for (int v = 0; v < 4; v++) d.vflux[1][v][c] = out[v];
-  }
-  if (i <= ie && j <= jn) {
-    double out[4];
-    if (CH) {
-      const double *t = d.ftab + (2LL * d.Y + (j - 1)) * 4;
-      visc_face_z_channel(d.rdxi, d.rdet, d.rdzt, d.mu, d.rpr, t[0], o, vp(d, c - 1), vp(d, c + di),
-                          vp(d, c + di - 1), vp(d, c - di), vp(d, c - di - 1), vp(d, c + dj), vp(d, c + dj - 1),
-                          vp(d, c - dj), vp(d, c - dj - 1), t[2], out);
-    } else {
-      double mm[9], Jf, iJf;
-      face_metrics(d, 2, f, j - 1, mm, Jf, iJf);
-      visc_face_z(d.rdxi, d.rdet, d.rdzt, d.mu, d.rpr, o, vp(d, c - 1), vp(d, c + di), vp(d, c + di - 1), vp(d, c - di),
-                  vp(d, c - di - 1), vp(d, c + dj), vp(d, c + dj - 1), vp(d, c - dj), vp(d, c - dj - 1),
-                  vp(d, c - di + dj), mm, iJf, out);
-    }
-    for (int v = 0; v < 4; v++) d.vflux[2][v][c] = out[v];
-  }
-}
-
-// Viscous_terms.cpp:875-904
-__global__ void k_viscous_div(Dev d) {
-  int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  int j = 2 + blockIdx.y;
-  int i = 3 + blockIdx.z;
-  if (k > d.nz + 1) return;
-  long long c = ix(d, i, j, k);
-  const double invXI = d.rdxi, invET = d.rdet, invZT = d.rdzt;
-  for (int v = 0; v < 4; v++)
-    d.vF[v][c] = (d.vflux[0][v][c + d.di] - d.vflux[0][v][c]) * invXI +
-                 (d.vflux[1][v][c + d.dj] - d.vflux[1][v][c]) * invET +
-                 (d.vflux[2][v][c + 1] - d.vflux[2][v][c]) * invZT;
-}
-
 // ---------------------------------------------------- dual-time residual
 // Dual_time_stepping.cpp:737-922 (the sponge Residual terms are zero for a
 // domain without inlet / outlet layers and are left out)
@@ -656,12 +548,6 @@ void launch_flux_y(const Dev &d, cudaStream_t s) {
 }
 void launch_flux_z(const Dev &d, cudaStream_t s) {
   k_flux_z<<<cellgrid(d.nz + 1, d.ny, d.nx, 64), 64, 0, s>>>(d);
-}
-void launch_viscous(const Dev &d, cudaStream_t s) {
-  k_vprim<<<cellgrid(d.nz + 2, d.ny + 2, d.nx + 2, 64), 64, 0, s>>>(d);
-  if (d.face_tables) k_viscous_faces<true><<<cellgrid(d.nz + 1, d.ny + 1, d.nx + 1, 64), 64, 0, s>>>(d);
-  else k_viscous_faces<false><<<cellgrid(d.nz + 1, d.ny + 1, d.nx + 1, 64), 64, 0, s>>>(d);
-  k_viscous_div<<<cellgrid(d.nz, d.ny, d.nx, 64), 64, 0, s>>>(d);
 }
 void launch_dts_residual(const Dev &d, cudaStream_t s) {
   k_dts_residual<<<cellgrid(d.nz, d.ny, d.nx, 64), 64, 0, s>>>(d);
