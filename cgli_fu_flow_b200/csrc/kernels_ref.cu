@@ -594,8 +594,21 @@ __global__ void k_norms(const double *partial, int nblocks, double scale, double
 // a.clock[2] counts the iterations.
 __global__ void k_iteration_result(Dev d, SweepArgs a, int nblocks, double scale, IterResult *ring, int slots, int timed) {
   double acc[5] = {0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int v = 0; v < 5; v++) acc[v] += d.partial[5 * (long long)b + v];
+  // four blocks' loads at a time, added up in order
+  for (int b0 = threadIdx.x; b0 < nblocks; b0 += 4 * blockDim.x) {
+    double p[4][5];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int b = b0 + q * blockDim.x;
+#pragma unroll
+      for (int v = 0; v < 5; v++) p[q][v] = b < nblocks ? d.partial[5 * (long long)b + v] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int v = 0; v < 5; v++)
+        if (b0 + q * blockDim.x < nblocks) acc[v] += p[q][v];
+  }
   __shared__ double tot[5];
   block_sum5(acc, tot);
   __syncthreads();
@@ -623,11 +636,33 @@ void launch_iteration_result(const Dev &d, const SweepArgs &a, cudaStream_t s, i
 // reduction in a fixed order (per-block partials, then one block)
 __global__ void k_bulk_partial(Dev d, double *part) {
   double acc[5] = {0, 0, 0, 0, 0};
-  const long long n = (long long)d.nx * d.ny * d.nz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int k = (int)(t % d.nz), j = (int)((t / d.nz) % d.ny), i = (int)(t / ((long long)d.nz * d.ny));
-    long long c = ix(d, i + 3, j + 2, k + 2);
-    acc[0] += (d.U_[1][c] * d.J[c]) * 1. / d.J[c];
+  const long long n = (long long)d.nx * d.ny * d.nz, step = (long long)gridDim.x * blockDim.x;
+  // eight cells' loads at a time, added up in order; the next cell of a thread
+  // lies (si, sj, sk) further, with carries
+  const int sk = (int)(step % d.nz), sj = (int)((step / d.nz) % d.ny), si = (int)(step / ((long long)d.nz * d.ny));
+  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  int k = (int)(t % d.nz), j = (int)((t / d.nz) % d.ny), i = (int)(t / ((long long)d.nz * d.ny));
+  while (t < n) {
+    double u[8], J[8];
+    int m = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      if (t < n) {
+        const long long c = ix(d, i + 3, j + 2, k + 2);
+        u[q] = d.U_[1][c];
+        J[q] = d.J[c];
+        m = q + 1;
+      }
+      t += step;
+      k += sk;
+      j += sj + (k >= d.nz);
+      if (k >= d.nz) k -= d.nz;
+      i += si + (j >= d.ny);
+      if (j >= d.ny) j -= d.ny;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (q < m) acc[0] += (u[q] * J[q]) * 1. / J[q];
   }
   __shared__ double tot[5];
   block_sum5(acc, tot);
@@ -639,12 +674,19 @@ __global__ void k_bulk_final(Dev d, const double *part, int nblk, double *out) {
   for (int b = threadIdx.x; b < nblk; b += blockDim.x) acc[0] += part[b];
   __shared__ double tot[5];
   block_sum5(acc, tot);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double Jsum = 0;
-    for (int j = 2; j <= d.ny + 1; j++) Jsum = Jsum + 1. / d.J[ix(d, 3, j, 3)];
-    out[0] = tot[0] / Jsum / d.nx / d.nz;
+  // the column's volumes by all threads, their sum in order by one
+  __shared__ double vol[256];
+  double Jsum = 0;
+  for (int j0 = 2; j0 <= d.ny + 1; j0 += 256) {
+    const int m = min(256, d.ny + 2 - j0);
+    __syncthreads();
+    if ((int)threadIdx.x < m) vol[threadIdx.x] = 1. / d.J[ix(d, 3, j0 + threadIdx.x, 3)];
+    __syncthreads();
+    if (threadIdx.x == 0)
+#pragma unroll 8
+      for (int q = 0; q < m; q++) Jsum = Jsum + vol[q];
   }
+  if (threadIdx.x == 0) out[0] = tot[0] / Jsum / d.nx / d.nz;
 }
 
 // main.cpp:364-386 over planes 2..ie+1, all rows; Q^(n-2) is kept as well

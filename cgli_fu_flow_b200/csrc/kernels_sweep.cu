@@ -736,17 +736,29 @@ inline unsigned sweep_update_grid_y(const Dev &d) { return (unsigned)((d.nz + UP
 template <typename T>
 __global__ void __launch_bounds__(256) k_update_skewed(Dev d, SweepArgs a) {
   constexpr int NS = UPD_KC + UPD_TJ - 1;   // steps holding the block's cells
-  static_assert(SWEEP_TJ % UPD_TJ == 0 && 256 % UPD_TJ == 0, "column staging");
+  static_assert(SWEEP_TJ % UPD_TJ == 0 && UPD_TJ == 16, "column staging; two rows per warp");
   __shared__ T sdq[5][NS][UPD_TJ + 1];       // (+1: the update reads a column down the steps)
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.clock[1] = globaltimer();
-  // a wavefront pass that gave up left dQ incomplete: keep the state
-  if (*(volatile int *)d.status) return;
+  const int status = *(volatile int *)d.status;
   const int ntu = (d.ny + UPD_TJ - 1) / UPD_TJ, S = sweep_steps(d);
   const int row = blockIdx.x / ntu, j0 = blockIdx.x % ntu * UPD_TJ;   // 0-based row and first column
   const int ntj = (d.ny + SWEEP_TJ - 1) / SWEEP_TJ, l0 = j0 % SWEEP_TJ;
   const int k0 = blockIdx.y * UPD_KC;        // first k of the block (0-based)
   const int s0 = k0 + l0;                    // step of the cell (first column, k0)
   const T *const dq = a.buf<T>(a.dq) + ((long long)row * ntj + j0 / SWEEP_TJ) * S * (5 * SWEEP_TJ) + l0;
+  // the warp's two rows of the state, in flight while dQ is staged
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = 3 + row, kl = k0 + lane;
+  double q[2][5], Jc[2], iJc[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int j = 2 + j0 + warp + 8 * h;
+    if (j > d.ny + 1 || kl >= d.nz) continue;
+    const long long c = ix(d, i, j, 2 + kl), cj = a.channel_metrics ? ix(d, 3, j, 2) : c;
+#pragma unroll
+    for (int v = 0; v < 5; v++) q[h][v] = d.U_[v][c];
+    Jc[h] = d.J[cj];
+    iJc[h] = d.iJ[cj];
+  }
   for (int e = threadIdx.x; e < NS * UPD_TJ; e += blockDim.x) {
     const int ls = e / UPD_TJ, jl = e % UPD_TJ, st = s0 + ls;
     if (st < S) {
@@ -754,21 +766,22 @@ __global__ void __launch_bounds__(256) k_update_skewed(Dev d, SweepArgs a) {
       for (int v = 0; v < 5; v++) sdq[v][ls][jl] = dq[(long long)st * (5 * SWEEP_TJ) + v * SWEEP_TJ + jl];
     }
   }
+  // a wavefront pass that gave up left dQ incomplete: keep the state
+  if (status) return;
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int i = 3 + row;
   double acc[5] = {0, 0, 0, 0, 0};
-  for (int jl = warp; jl < UPD_TJ; jl += nw) {
-    const int j = 2 + j0 + jl, kl = k0 + lane;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int jl = warp + 8 * h, j = 2 + j0 + jl;
     if (j > d.ny + 1 || kl >= d.nz) continue;
     const int ls = lane + jl;            // step of the cell, relative to s0
     const long long c = ix(d, i, j, 2 + kl);
-    const double J = d.J[c], iJ = d.iJ[c];
-    const double q1 = d.U_[0][c], iq1 = nr_rcp(q1);
+    const double J = Jc[h], iJ = iJc[h];
+    const double q1 = q[h][0], iq1 = nr_rcp(q1);
     const double rhoold = q1 * J;
-    const double Uold = d.U_[1][c] * iq1, Vold = d.U_[2][c] * iq1, Wold = d.U_[3][c] * iq1;
+    const double Uold = q[h][1] * iq1, Vold = q[h][2] * iq1, Wold = q[h][3] * iq1;
     const double VVold = Uold * Uold + Vold * Vold + Wold * Wold;
-    const double Pold = (d.U_[4][c] * J - 0.5 * rhoold * VVold) * (KG - 1);
+    const double Pold = (q[h][4] * J - 0.5 * rhoold * VVold) * (KG - 1);
     const double Told = Pold * (iq1 * iJ);   // 1 / rho = 1 / (q1 J)
     const double P = Pold + (double)sdq[0][ls][jl] * J, U = Uold + (double)sdq[1][ls][jl] * J;
     const double V = Vold + (double)sdq[2][ls][jl] * J, W = Wold + (double)sdq[3][ls][jl] * J;
