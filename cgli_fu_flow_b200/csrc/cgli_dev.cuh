@@ -206,6 +206,10 @@ __device__ __forceinline__ void side2(const Dev &d, long long a, long long b, do
 // face metric, sq its norm and insqr = 1/sq; iJf the reciprocal of the face
 // Jacobian.  Also returns Fav3 and iP+P_ for the wall faces of
 // Flux_Y.cpp:400-408.
+// AX: the one component of the face metric that is not zero (the channel
+// grid), whose terms alone are formed then (the others are products with zero,
+// so the values are the same); -1: any metric.
+template <int AX>
 __device__ __forceinline__ void roe_face(const double L[5], const double R[5], double mx, double my,
                                          double mz, double sq, double insqr, double iJf, double e, double F[5],
                                          double &Fav3o, double &ppo) {
@@ -217,17 +221,21 @@ __device__ __forceinline__ void roe_face(const double L[5], const double R[5], d
   // Newton-refined ones (results differ from the reference's in the last
   // bits only).
   constexpr double rkg = 1.0 / (KG - 1);
+  const auto dot = [&](double a, double b, double c) {
+    return AX == 0 ? mx * a : AX == 1 ? my * b : AX == 2 ? mz * c : mx * a + my * b + mz * c;
+  };
+  constexpr bool AXX = AX < 0 || AX == 0, AXY = AX < 0 || AX == 1, AXZ = AX < 0 || AX == 2;
   const double NX = mx * insqr, NY = my * insqr, NZ = mz * insqr;
   const double _rho = L[0], irl = nr_rcp(_rho);
   const double _u = L[1] * irl, _v = L[2] * irl, _w = L[3] * irl;
-  const double iU = mx * _u + my * _v + mz * _w;
+  const double iU = dot(_u, _v, _w);
   const double _VV = _u * _u + _v * _v + _w * _w;
   const double iP = (L[4] - 0.5 * _rho * _VV) * (KG - 1);
   const double iC = KG * iP * irl;
   const double _H = 0.5 * _VV + iC * rkg;
   const double rho_ = R[0], irr = nr_rcp(rho_);
   const double u_ = R[1] * irr, v_ = R[2] * irr, w_ = R[3] * irr;
-  const double U_ = mx * u_ + my * v_ + mz * w_;
+  const double U_ = dot(u_, v_, w_);
   const double VV_ = u_ * u_ + v_ * v_ + w_ * w_;
   const double P_ = (R[4] - 0.5 * rho_ * VV_) * (KG - 1);
   const double C_ = KG * P_ * irr;
@@ -265,15 +273,18 @@ __device__ __forceinline__ void roe_face(const double L[5], const double R[5], d
   const double deltaP = U_p * iS * dP + (C_p - fabs(U) * insqr + temp4) * rho * dUn;
   const double aU = fabs(Un);
   const double Fav1 = aU * dU1 + deltaU * rho;
-  const double Fav2 = aU * dU2 + deltaU * rho * u + deltaP * NX;
-  const double Fav3 = aU * dU3 + deltaU * rho * v + deltaP * NY;
-  const double Fav4 = aU * dU4 + deltaU * rho * w + deltaP * NZ;
+  const double fav2 = aU * dU2 + deltaU * rho * u, Fav2 = AXX ? fav2 + deltaP * NX : fav2;
+  const double fav3 = aU * dU3 + deltaU * rho * v, Fav3 = AXY ? fav3 + deltaP * NY : fav3;
+  const double fav4 = aU * dU4 + deltaU * rho * w, Fav4 = AXZ ? fav4 + deltaP * NZ : fav4;
   const double Fav5 = aU * dU5 + deltaU * rho * H + deltaP * Un;
   const double h = 0.5 * iJf;
   F[0] = ((_rho * iU + rho_ * U_) - Fav1 * sq) * h;
-  F[1] = ((_rho * _u * iU + rho_ * u_ * U_ + mx * (iP + P_)) - Fav2 * sq) * h;
-  F[2] = ((_rho * _v * iU + rho_ * v_ * U_ + my * (iP + P_)) - Fav3 * sq) * h;
-  F[3] = ((_rho * _w * iU + rho_ * w_ * U_ + mz * (iP + P_)) - Fav4 * sq) * h;
+  const double f1 = _rho * _u * iU + rho_ * u_ * U_;
+  F[1] = ((AXX ? f1 + mx * (iP + P_) : f1) - Fav2 * sq) * h;
+  const double f2 = _rho * _v * iU + rho_ * v_ * U_;
+  F[2] = ((AXY ? f2 + my * (iP + P_) : f2) - Fav3 * sq) * h;
+  const double f3 = _rho * _w * iU + rho_ * w_ * U_;
+  F[3] = ((AXZ ? f3 + mz * (iP + P_) : f3) - Fav4 * sq) * h;
   F[4] = ((iU * (3.5 * iP + 0.5 * _rho * _VV) + U_ * (3.5 * P_ + 0.5 * rho_ * VV_)) - Fav5 * sq) * h;
   Fav3o = Fav3;
   ppo = iP + P_;

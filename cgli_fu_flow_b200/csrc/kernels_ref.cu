@@ -6,13 +6,6 @@
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
 
-// CTAs of 64 threads per SM the inviscid flux kernels are compiled for
-// (register cap: 12 CTAs leave 80 registers, a few spilled, 18 % faster than
-// the uncapped 116 at 256x192x192)
-#ifndef CGLI_FLUX_MINBLOCKS
-#define CGLI_FLUX_MINBLOCKS 12
-#endif
-
 namespace cgli {
 
 // ---------------------------------------------------------------- halos
@@ -209,35 +202,66 @@ __global__ void k_target_u(Dev d) {
 }
 
 // ---------------------------------------------------------------- fluxes
+// Bound by the FP64 pipe (some 280 instructions a face in the channel form:
+// 160 us at 256x192x192) and, before it, by the loads of six arrays' stencils.
+// Caps of 12 CTAs per SM (80 registers, no spills in the channel form, where
+// only the live metric terms are formed) and 16 for the z faces (64 registers)
+// were the fastest of 10 to 16.  x and y faces march `chunk` faces along their stencil
+// (MARCH), so that five of six stencil cells come from L1 (flux_march).  x / y
+// / z at 256x192x192: 300 / 335 / 340 us with the general form, a block per 64
+// faces of a row; 255 / 285 / 254 now (160x128x128 91 / 101 / 113 -> 80 / 90 /
+// 81, 91x53x75 25 / 26 / 25 -> 19 / 19 / 19).
+//
+// Face (i, j, k) of this thread, i from 2, j and k from 1, of planes of nj
+// rows of nk faces: a block of 64 per piece of a row, or (FLAT) of the plane's
+// faces as one run, which leaves no lanes idle at the row ends but costs the
+// division and addresses that differ between the lanes.
+template <bool FLAT>
+__device__ __forceinline__ bool face_of(int nk, int nj, int &i, int &j, int &k) {
+  const int t = blockIdx.x * 64 + threadIdx.x;
+  k = 1 + (FLAT ? t % nk : t);
+  j = 1 + (FLAT ? t / nk : (int)blockIdx.y);
+  i = 2 + blockIdx.z;
+  return FLAT ? j <= nj : k <= nk;
+}
+
 // x faces i = 2..ie, tangential j = 1..jn-1, k = 1..kn-1 (Flux_X.cpp:96-357)
-__global__ void __launch_bounds__(64, CGLI_FLUX_MINBLOCKS) k_flux_x(Dev d) {
-  int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  int j = 1 + blockIdx.y;
-  int i = 2 + blockIdx.z;
-  if (k > d.nz) return;
-  long long f = ix(d, i, j, k);
-  // left state ML[i] from cells i-2..i+2, right state MR[i] from i-1..i+3
-  long long c = ix(d, i, j + 1, k + 1);
-  double L[5], R[5], F[5], fav3, pp;
-  const int ie = d.nx + 2;
-  const long long di = d.di;
-  if (d.x_open && (i <= 3 || i >= ie - 1)) {
-    // the first and last rank's reduced stencils, Flux_X.cpp:139-216
-    if (i == 2) side2(d, c, c + di, L);
-    else if (i == 3 || i == ie) side3L(d, c - di, di, L);
-    else side5L(d, c - 2 * di, di, L);
-    if (i == 2 || i == ie - 1) side3R(d, c, di, R);
-    else if (i == ie) side2(d, c, c + di, R);
-    else side5R(d, c - di, di, R);
-  } else {
-    side5L(d, c - 2 * di, di, L);
-    side5R(d, c - di, di, R);
+template <bool CH, bool FLAT, bool MARCH>
+__global__ void __launch_bounds__(64, 12) k_flux_x(Dev d, int chunk) {
+  int i0, j, k;
+  if (!face_of<FLAT>(d.nz, d.ny, i0, j, k)) return;
+  i0 = 2 + (i0 - 2) * chunk;
+  const int i1 = min(d.nx + 2, i0 + chunk - 1);
+#pragma unroll 1
+  for (int i = i0; MARCH ? i <= i1 : i == i0; i++) {
+    long long f = ix(d, i, j, k);
+    // left state ML[i] from cells i-2..i+2, right state MR[i] from i-1..i+3
+    long long c = ix(d, i, j + 1, k + 1);
+    double L[5], R[5], F[5], fav3, pp;
+    const int ie = d.nx + 2;
+    const long long di = d.di;
+    if (d.x_open && (i <= 3 || i >= ie - 1)) {
+      // the first and last rank's reduced stencils, Flux_X.cpp:139-216
+      if (i == 2) side2(d, c, c + di, L);
+      else if (i == 3 || i == ie) side3L(d, c - di, di, L);
+      else side5L(d, c - 2 * di, di, L);
+      if (i == 2 || i == ie - 1) side3R(d, c, di, R);
+      else if (i == ie) side2(d, c, c + di, R);
+      else side5R(d, c - di, di, R);
+    } else {
+      side5L(d, c - 2 * di, di, L);
+      side5R(d, c - di, di, R);
+    }
+    if (CH) {
+      roe_face<0>(L, R, 1, 0, 0, 1, 1, d.ftab[(0LL * d.Y + j) * 4 + 2], d.e, F, fav3, pp);
+    } else {
+      double mm[9], Jf, iJf, sq, insqr;
+      face_metrics(d, 0, f, j, mm, Jf, iJf);
+      face_norm(d, 0, j, mm[0], mm[1], mm[2], sq, insqr);
+      roe_face<-1>(L, R, mm[0], mm[1], mm[2], sq, insqr, iJf, d.e, F, fav3, pp);
+    }
+    for (int v = 0; v < 5; v++) d.inF[0][v][f] = F[v];
   }
-  double mm[9], Jf, iJf, sq, insqr;
-  face_metrics(d, 0, f, j, mm, Jf, iJf);
-  face_norm(d, 0, j, mm[0], mm[1], mm[2], sq, insqr);
-  roe_face(L, R, mm[0], mm[1], mm[2], sq, insqr, iJf, d.e, F, fav3, pp);
-  for (int v = 0; v < 5; v++) d.inF[0][v][f] = F[v];
 }
 
 // left / right MUSCL states of all five variables at y face j+1/2 of column
@@ -259,30 +283,43 @@ __device__ __forceinline__ void muscl_y(const Dev &d, int i, int j, int k, doubl
 }
 
 // y faces j = 1..jn, i = 2..ie-1, k = 1..kn-1 (Flux_Y.cpp:94-413)
-__global__ void __launch_bounds__(64, CGLI_FLUX_MINBLOCKS) k_flux_y(Dev d) {
-  int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  int j = 1 + blockIdx.y;
-  int i = 2 + blockIdx.z;
-  if (k > d.nz) return;
-  int jn = d.ny + 1;
-  long long f = ix(d, i, j, k);
-  double L[5], R[5], F[5], fav3, pp;
-  muscl_y(d, i + 1, j, k + 1, L, R);
-  double mm[9], Jf, iJf, sq, insqr;
-  face_metrics(d, 1, f, j, mm, Jf, iJf);
-  const double ety = mm[4];
-  face_norm(d, 1, j, mm[3], ety, mm[5], sq, insqr);
-  roe_face(L, R, mm[3], ety, mm[5], sq, insqr, iJf, d.e, F, fav3, pp);
-  if (j == 1 || j == jn) {
-    F[0] = 0; F[1] = 0; F[3] = 0; F[4] = 0;
-    F[2] = 0.5 * (ety * pp - 1. * fav3) * iJf;
-    if (d.curved_walls) {
-      // a curved wall also carries the x and z pressure force
-      F[1] = 0.5 * (mm[3] * pp) * iJf;
-      F[3] = 0.5 * (mm[5] * pp) * iJf;
+template <bool CH, bool FLAT, bool MARCH>
+__global__ void __launch_bounds__(64, 12) k_flux_y(Dev d, int chunk) {
+  int i, j0, k;
+  const int nc = (d.ny + chunk) / chunk;
+  if (!face_of<FLAT>(d.nz, nc, i, j0, k)) return;
+  j0 = 1 + (j0 - 1) * chunk;
+  const int j1 = min(d.ny + 1, j0 + chunk - 1);
+#pragma unroll 1
+  for (int j = j0; MARCH ? j <= j1 : j == j0; j++) {
+    int jn = d.ny + 1;
+    long long f = ix(d, i, j, k);
+    double L[5], R[5], F[5], fav3, pp;
+    muscl_y(d, i + 1, j, k + 1, L, R);
+    double etx = 0, ety, etz = 0, iJf;
+    if (CH) {
+      const double *t = d.ftab + (1LL * d.Y + j) * 4;
+      ety = t[0];
+      iJf = t[2];
+      roe_face<1>(L, R, 0, ety, 0, fabs(ety), t[3], iJf, d.e, F, fav3, pp);
+    } else {
+      double mm[9], Jf, sq, insqr;
+      face_metrics(d, 1, f, j, mm, Jf, iJf);
+      etx = mm[3]; ety = mm[4]; etz = mm[5];
+      face_norm(d, 1, j, etx, ety, etz, sq, insqr);
+      roe_face<-1>(L, R, etx, ety, etz, sq, insqr, iJf, d.e, F, fav3, pp);
     }
+    if (j == 1 || j == jn) {
+      F[0] = 0; F[1] = 0; F[3] = 0; F[4] = 0;
+      F[2] = 0.5 * (ety * pp - 1. * fav3) * iJf;
+      if (d.curved_walls) {
+        // a curved wall also carries the x and z pressure force
+        F[1] = 0.5 * (etx * pp) * iJf;
+        F[3] = 0.5 * (etz * pp) * iJf;
+      }
+    }
+    for (int v = 0; v < 5; v++) d.inF[1][v][f] = F[v];
   }
-  for (int v = 0; v < 5; v++) d.inF[1][v][f] = F[v];
 }
 
 // left / right states of all five variables at z face k+1/2
@@ -300,18 +337,21 @@ __device__ __forceinline__ void muscl_z(const Dev &d, int i, int j, int k, doubl
 }
 
 // z faces k = 1..kn, i = 2..ie-1, j = 1..jn-1 (Flux_Z.cpp:91-359)
-__global__ void __launch_bounds__(64, CGLI_FLUX_MINBLOCKS) k_flux_z(Dev d) {
-  int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  int j = 1 + blockIdx.y;
-  int i = 2 + blockIdx.z;
-  if (k > d.nz + 1) return;
+template <bool CH, bool FLAT, bool MARCH>
+__global__ void __launch_bounds__(64, CH ? 16 : 12) k_flux_z(Dev d, int) {
+  int i, j, k;
+  if (!face_of<FLAT>(d.nz + 1, d.ny, i, j, k)) return;
   long long f = ix(d, i, j, k);
   double L[5], R[5], F[5], fav3, pp;
   muscl_z(d, i + 1, j + 1, k, L, R);
-  double mm[9], Jf, iJf, sq, insqr;
-  face_metrics(d, 2, f, j, mm, Jf, iJf);
-  face_norm(d, 2, j, mm[6], mm[7], mm[8], sq, insqr);
-  roe_face(L, R, mm[6], mm[7], mm[8], sq, insqr, iJf, d.e, F, fav3, pp);
+  if (CH) {
+    roe_face<2>(L, R, 0, 0, 1, 1, 1, d.ftab[(2LL * d.Y + j) * 4 + 2], d.e, F, fav3, pp);
+  } else {
+    double mm[9], Jf, iJf, sq, insqr;
+    face_metrics(d, 2, f, j, mm, Jf, iJf);
+    face_norm(d, 2, j, mm[6], mm[7], mm[8], sq, insqr);
+    roe_face<-1>(L, R, mm[6], mm[7], mm[8], sq, insqr, iJf, d.e, F, fav3, pp);
+  }
   for (int v = 0; v < 5; v++) d.inF[2][v][f] = F[v];
 }
 
@@ -540,15 +580,36 @@ void launch_bc_z(const Dev &d, cudaStream_t s) {
   long long rows = (long long)d.X * d.Y;
   k_bc_z<<<dim3((unsigned)((rows + 255) / 256), 5), 256, 0, s>>>(d);
 }
+// FLAT where a fifth or more of the row blocks' lanes would be idle (the z
+// faces of 192 cells, 193 in four blocks: 340 -> 283 us at 256x192x192, and at
+// 91x53x75 25 -> 19 us each; but with 192 x faces a row, which fill their
+// blocks, it costs 300 -> 317 us)
+#define FLUX(kern, march, nk, nj, ni)                                                                \
+  do {                                                                                               \
+    const bool flat = ((nk) + 63) / 64 * 64 * 4 >= (nk) * 5;                                         \
+    const dim3 g(flat ? (unsigned)(((long long)(nk) * (nj) + 63) / 64) : ((nk) + 63) / 64, flat ? 1 : (nj), ni); \
+    if (d.face_tables) {                                                                             \
+      if (flat) kern<true, true, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                         \
+      else kern<true, false, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                             \
+    } else {                                                                                         \
+      if (flat) kern<false, true, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                        \
+      else kern<false, false, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                            \
+    }                                                                                                \
+  } while (0)
+// x and y: 4 faces per thread along the stencil where that leaves four waves
+// of blocks (160x128x128 x / y 87 / 95 -> 80 / 90 us, general metrics 109 / 111
+// -> 98 / 105; at 128x96x96, 2.6 waves, 45 / 52 -> 44 / 56 and general y 61 ->
+// 71; 8 faces are slower than 4 everywhere)
+static bool flux_march(long long faces) { return faces / (4 * 64) >= 4 * 12 * 148; }
 void launch_flux_x(const Dev &d, cudaStream_t s) {
-  k_flux_x<<<cellgrid(d.nz, d.ny, d.nx + 1, 64), 64, 0, s>>>(d);
+  if (flux_march((long long)d.nz * d.ny * (d.nx + 1))) FLUX(k_flux_x, true, d.nz, d.ny, (d.nx + 4) / 4);
+  else FLUX(k_flux_x, false, d.nz, d.ny, d.nx + 1);
 }
 void launch_flux_y(const Dev &d, cudaStream_t s) {
-  k_flux_y<<<cellgrid(d.nz, d.ny + 1, d.nx, 64), 64, 0, s>>>(d);
+  if (flux_march((long long)d.nz * (d.ny + 1) * d.nx)) FLUX(k_flux_y, true, d.nz, (d.ny + 4) / 4, d.nx);
+  else FLUX(k_flux_y, false, d.nz, d.ny + 1, d.nx);
 }
-void launch_flux_z(const Dev &d, cudaStream_t s) {
-  k_flux_z<<<cellgrid(d.nz + 1, d.ny, d.nx, 64), 64, 0, s>>>(d);
-}
+void launch_flux_z(const Dev &d, cudaStream_t s) { FLUX(k_flux_z, false, d.nz + 1, d.ny, d.nx); }
 void launch_dts_residual(const Dev &d, cudaStream_t s) {
   k_dts_residual<<<cellgrid(d.nz, d.ny, d.nx, 64), 64, 0, s>>>(d);
 }
