@@ -25,20 +25,13 @@ __global__ void k_halo_x(Dev d) {
 // Y_boundary_condition.cpp:94-182 for interior planes i = 3..ie: the
 // zero-gradient copy of :100-112, replaced inside the heated section
 // (planes nx_inlet+3 .. Nx-nx_outlet+2, :114) by the isothermal no-slip
-// reflection
-__global__ void k_bc_y(Dev d) {
-  int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  int i = 3 + blockIdx.y;
-  int side = blockIdx.z;
-  int jn = d.ny + 1, kn = d.nz + 1;
-  if (k > kn) return;
-  int js = side ? jn : 2, jg = side ? jn + 1 : 1;
-  long long c = ix(d, i, js, k), g = ix(d, i, jg, k);
-  if (!(i > d.nx_inlet + 2 && i < d.nx - d.nx_outlet + 3)) {
-    for (int v = 0; v < 5; v++) d.U_[v][g] = d.U_[v][c];
-    return;
-  }
-  double q1 = d.U_[0][c], q2 = d.U_[1][c], q3 = d.U_[2][c], q4 = d.U_[3][c], q5 = d.U_[4][c];
+// reflection.  The ghost cell of (i, k) at the lower (side 0) or upper wall.
+__device__ __forceinline__ void wall_ghost(const Dev &d, int i, int k, int side, double o[5]) {
+  const int jn = d.ny + 1, js = side ? jn : 2, jg = side ? jn + 1 : 1;
+  const long long c = ix(d, i, js, k), g = ix(d, i, jg, k);
+  for (int v = 0; v < 5; v++) o[v] = d.U_[v][c];
+  if (!(i > d.nx_inlet + 2 && i < d.nx - d.nx_outlet + 3)) return;
+  double q1 = o[0], q2 = o[1], q3 = o[2], q4 = o[3], q5 = o[4];
   double Jc = d.J[c], Jg = d.J[g];
   double rho = q1 * Jc;
   double U = q2 / q1, V = q3 / q1, W = q4 / q1;
@@ -46,11 +39,18 @@ __global__ void k_bc_y(Dev d) {
   double P = (q5 * Jc - 0.5 * rho * VV) * (KG - 1);
   double T = side ? d.twh : d.twl;
   rho = P / RG / T;
-  d.U_[0][g] = rho / Jg;
-  d.U_[1][g] = -rho * U / Jg;
-  d.U_[2][g] = -rho * V / Jg;
-  d.U_[3][g] = -rho * W / Jg;
-  d.U_[4][g] = (P / (KG - 1) + 0.5 * rho * VV) / Jg;
+  o[0] = rho / Jg;
+  o[1] = -rho * U / Jg;
+  o[2] = -rho * V / Jg;
+  o[3] = -rho * W / Jg;
+  o[4] = (P / (KG - 1) + 0.5 * rho * VV) / Jg;
+}
+__global__ void k_bc_y(Dev d) {
+  const int k = 2 + blockIdx.x * blockDim.x + threadIdx.x, i = 3 + blockIdx.y, side = blockIdx.z;
+  if (k > d.nz + 1) return;
+  double q[5];
+  wall_ghost(d, i, k, side, q);
+  for (int v = 0; v < 5; v++) d.U_[v][ix(d, i, side ? d.ny + 2 : 1, k)] = q[v];
 }
 
 // Z_boundary_condition.cpp:39-66: all rows 0..nyyy of planes 0..ie+3
@@ -69,6 +69,62 @@ __global__ void k_bc_z(Dev d) {
   double *q = d.U_[v];
   q[row + 1] = q[row + kn];
   q[row + kn + 1] = q[row + 2];
+}
+
+// k_halo_x, k_bc_y and k_bc_z of a periodic slab in one launch: the same
+// values, each ghost cell formed from interior cells (and from ghost rows as
+// they were) without waiting for another ghost cell.  Three launches of 3.8 us
+// of the iteration's serial chain become one.
+//   blocks [0, na): the halo planes but for the two wall ghost rows; column 1
+//     (kn+1) is the image of column kn (2), which the z copy would fetch
+//   blocks [na, nb): the wall ghost rows of the interior planes, one thread
+//     per (plane, side, k = 1..kn+1).  The x halo copies these rows as they
+//     were, so the thread that overwrites a cell first writes its images
+//   blocks [nb, ..): columns 1 and kn+1 of the interior planes' other rows
+__global__ void __launch_bounds__(128) k_halo_bc(Dev d, unsigned na, unsigned nb) {
+  const int ie = d.nx + 2, jn = d.ny + 1, kn = d.nz + 1;
+  if (blockIdx.x < na) {
+    const long long t = blockIdx.x * 128LL + threadIdx.x;
+    if (t >= 6 * d.di) return;
+    const int p = (int)(t / d.di), r = (int)(t % d.di), j = r / d.Z, k = r % d.Z;
+    if ((j == 1 || j == jn + 1) && k >= 1 && k <= kn + 1) return;
+    const int i = p < 3 ? p : ie + 1 + p - 3, is = p < 3 ? ie - 2 + p : p;
+    const long long c = ix(d, is, j, k == 1 ? kn : k == kn + 1 ? 2 : k);
+    for (int v = 0; v < 5; v++) d.U_[v][i * d.di + r] = d.U_[v][c];
+    return;
+  }
+  if (blockIdx.x < nb) {
+    const long long t = (blockIdx.x - na) * 128LL + threadIdx.x;
+    const int side = (int)(t / (kn + 1) % 2), k = 1 + (int)(t % (kn + 1)), jg = side ? jn + 1 : 1;
+    const int i = 3 + (int)(t / (2 * (kn + 1)));
+    if (i > ie) return;
+    const long long g = ix(d, i, jg, k);
+    double q[5];
+    wall_ghost(d, i, k == 1 ? kn : k == kn + 1 ? 2 : k, side, q);
+    if (k > 1 && k <= kn) {
+      const int lo = i - (ie - 2), hi = ie + 1 + i - 3;   // the planes that hold this cell's images
+      for (int v = 0; v < 5; v++) {
+        const double old = d.U_[v][g];
+        for (int h = 0; h < 2; h++) {
+          if (h ? i > 5 : lo < 0) continue;
+          double *const o = d.U_[v] + ix(d, h ? hi : lo, jg, 0);
+          o[k] = old;
+          if (k == kn) o[1] = old;
+          if (k == 2) o[kn + 1] = old;
+        }
+      }
+    }
+    for (int v = 0; v < 5; v++) d.U_[v][g] = q[v];
+    return;
+  }
+  const long long t = (blockIdx.x - nb) * 128LL + threadIdx.x;
+  const int right = (int)(t & 1), j = (int)(t / 2 % d.Y), i = 3 + (int)(t / 2 / d.Y);
+  if (i > ie || j == 1 || j == jn + 1) return;
+  const long long row = ix(d, i, j, 0);
+  for (int v = 0; v < 5; v++) {
+    double *const o = d.U_[v] + row;
+    o[right ? kn + 1 : 1] = o[right ? 2 : kn];
+  }
 }
 
 // X_boundary_condition.cpp:73-338 on an open slab: one pseudo-time step of
@@ -206,11 +262,11 @@ __global__ void k_target_u(Dev d) {
 // 160 us at 256x192x192) and, before it, by the loads of six arrays' stencils.
 // Caps of 12 CTAs per SM (80 registers, no spills in the channel form, where
 // only the live metric terms are formed) and 16 for the z faces (64 registers)
-// were the fastest of 10 to 16.  x and y faces march `chunk` faces along their stencil
-// (MARCH), so that five of six stencil cells come from L1 (flux_march).  x / y
-// / z at 256x192x192: 300 / 335 / 340 us with the general form, a block per 64
-// faces of a row; 255 / 285 / 254 now (160x128x128 91 / 101 / 113 -> 80 / 90 /
-// 81, 91x53x75 25 / 26 / 25 -> 19 / 19 / 19).
+// were the fastest of 10 to 16.  On large grids x and y faces march `chunk`
+// faces along their stencil (MARCH), so that five of six stencil cells come
+// from L1.  x / y / z at 256x192x192: 300 / 335 / 340 us with the general form
+// and a block per 64 faces of a row; 254 / 284 / 254 now (160x128x128 91 / 101
+// / 113 -> 80 / 91 / 82, 91x53x75 25 / 26 / 25 -> 19 / 20 / 19).
 //
 // Face (i, j, k) of this thread, i from 2, j and k from 1, of planes of nj
 // rows of nk faces: a block of 64 per piece of a row, or (FLAT) of the plane's
@@ -539,11 +595,16 @@ static dim3 cellgrid(int nk, int nj, int ni, int bx) { return dim3((nk + bx - 1)
 
 // main.cpp:167-210: halo exchange, then Y, X, Z boundaries
 void launch_halo_bc(const Dev &d, cudaStream_t s) {
-  launch_halo_x(d, s);
-  k_bc_y<<<dim3((d.nz + 127) / 128, d.nx, 2), 128, 0, s>>>(d);
+  if (!d.x_open) {
+    const unsigned na = (unsigned)((6 * d.di + 127) / 128),
+                   nb = na + (unsigned)((2LL * d.nx * (d.nz + 2) + 127) / 128),
+                   nc = nb + (unsigned)((2LL * d.nx * d.Y + 127) / 128);
+    k_halo_bc<<<nc, 128, 0, s>>>(d, na, nb);
+    return;
+  }
+  launch_bc_y(d, s);
   launch_bc_x(d, s);
-  long long rows = (long long)d.X * d.Y;
-  k_bc_z<<<dim3((unsigned)((rows + 255) / 256), 5), 256, 0, s>>>(d);
+  launch_bc_z(d, s);
 }
 void launch_halo_x(const Dev &d, cudaStream_t s) {
   if (d.x_open) return;   // both neighbours absent
