@@ -3,11 +3,6 @@
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
 
-// CTAs per SM the residual kernel is compiled for (register cap)
-#ifndef CGLI_RESIDUAL_MINBLOCKS
-#define CGLI_RESIDUAL_MINBLOCKS 1
-#endif
-
 namespace cgli {
 
 // the nine metric terms of cell c (row j): per-row tables on the channel grid
@@ -27,16 +22,28 @@ __device__ __forceinline__ void cell_metrics(const Dev &d, const SweepArgs &a, i
 // exchanges planes ie and 3 before its first pass, :942-976).  CH: the grid
 // is uniform in x and z (a.channel_metrics), J and etdy come from the per-row
 // tables instead of ten 3-D metric arrays.
-// (the mixed-precision channel instance is held at six CTAs per SM, the
-// occupancy of the other instances: uncapped it takes ten registers more and
-// drops to five)
+// Bound by its bytes: 34 words in and 16 out a cell (606 us at 256x192x192 with
+// the streams' ramps), at eight CTAs per SM (128 registers, no spills).
+// 256x192x192 786 -> 670 us, 585 in mixed precision (632), 160x128x128 228 ->
+// 195, of which 14 us are the eight CTAs (six, at 166 registers, without the
+// cap) and the rest the store of whole lines; ten CTAs take 220, twelve 219.
 template <bool MIXED, bool CH>
-__global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 6) ? 6 : CGLI_RESIDUAL_MINBLOCKS)
+__global__ void __launch_bounds__(64, 8)
     k_residual_fast(Dev d, SweepArgs a) {
-  int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
+  // a warp's blocks of record and MR, [cell][vector]: written to memory as
+  // whole lines, several cells per instruction (a cell's own 16-byte stores, a
+  // line apart from lane to lane, cost the load/store unit 32 passes each)
+  constexpr int NV = MIXED ? 4 : 8;   // 16-byte vectors per cell
+  __shared__ uint4 s_out[2][32 * NV];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kw = 2 + blockIdx.x * 64 + warp * 32;
   int j = 2 + blockIdx.y;
   int i = 2 + blockIdx.z;
-  if (k > d.nz + 1) return;
+  if (kw > d.nz + 1) return;
+  const bool cell = kw + lane <= d.nz + 1;
+  const int k = cell ? kw + lane : d.nz + 1;   // (a lane without a cell repeats the last one)
+  // position of vector u of this lane's cell in s_out (the lanes of a quarter
+  // warp on different banks)
+  const auto at = [&](int u) { return lane * NV + (u ^ (MIXED ? (lane >> 1) & 3 : lane & 7)); };
   long long c = ix(d, i, j, k);
   const double J = CH ? a.Jtab[j] : d.J[c], deltaT = d.dt;
 
@@ -53,6 +60,7 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
                 deltaT, r);
     const long long h = (long long)j * d.dj + k;
     if (halo_plane) {
+      if (!cell) return;
       void *const hrec = a.hrec[i == 2 ? 0 : 1];
       for (int v2 = 0; v2 < REC_N; v2++) {
         if (MIXED) a.buf<float>(hrec)[v2 * d.di + h] = (float)r[v2];
@@ -66,13 +74,13 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
     // slot's position in its step block, whose size is a multiple of 8)
     const int t = (int)(slot & 7);
     if (MIXED) {
-      float4 *o = reinterpret_cast<float4 *>(a.buf<float>(a.cellrec) + slot * CR_N);
-      o[rec_vec_pos<float>(0, t)] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
-      o[rec_vec_pos<float>(1, t)] = make_float4((float)r[4], (float)r[5], (float)r[6], (float)r[7]);
+      float4 *o = reinterpret_cast<float4 *>(s_out[warp]);
+      o[at(rec_vec_pos<float>(0, t))] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
+      o[at(rec_vec_pos<float>(1, t))] = make_float4((float)r[4], (float)r[5], (float)r[6], (float)r[7]);
     } else {
-      double2 *o = reinterpret_cast<double2 *>(a.buf<double>(a.cellrec) + slot * CR_N);
+      double2 *o = reinterpret_cast<double2 *>(s_out[warp]);
 #pragma unroll
-      for (int q = 0; q < 5; q++) o[rec_vec_pos<double>(q, t)] = make_double2(r[2 * q], r[2 * q + 1]);
+      for (int q = 0; q < 5; q++) o[at(rec_vec_pos<double>(q, t))] = make_double2(r[2 * q], r[2 * q + 1]);
     }
     r8 = r[8];
     r9 = r[9];
@@ -120,19 +128,29 @@ __global__ void __launch_bounds__(64, (MIXED && CH && CGLI_RESIDUAL_MINBLOCKS < 
   // (record words 0..10, MR 11..15)
   const int t = (int)(slot & 7);
   if (MIXED) {
-    float4 *o = reinterpret_cast<float4 *>(a.buf<float>(a.cellrec) + slot * CR_N);
-    o[rec_vec_pos<float>(2, t)] = make_float4((float)r8, (float)r9, (float)r10, (float)MR[0]);
-    o[rec_vec_pos<float>(3, t)] = make_float4((float)MR[1], (float)MR[2], (float)MR[3], (float)MR[4]);
+    float4 *o = reinterpret_cast<float4 *>(s_out[warp]);
+    o[at(rec_vec_pos<float>(2, t))] = make_float4((float)r8, (float)r9, (float)r10, (float)MR[0]);
+    o[at(rec_vec_pos<float>(3, t))] = make_float4((float)MR[1], (float)MR[2], (float)MR[3], (float)MR[4]);
   } else {
-    double2 *o = reinterpret_cast<double2 *>(a.buf<double>(a.cellrec) + slot * CR_N);
+    double2 *o = reinterpret_cast<double2 *>(s_out[warp]);
     (void)r8;
     (void)r9;
-    o[rec_vec_pos<double>(5, t)] = make_double2(r10, MR[0]);
-    o[rec_vec_pos<double>(6, t)] = make_double2(MR[1], MR[2]);
-    o[rec_vec_pos<double>(7, t)] = make_double2(MR[3], MR[4]);
+    o[at(rec_vec_pos<double>(5, t))] = make_double2(r10, MR[0]);
+    o[at(rec_vec_pos<double>(6, t))] = make_double2(MR[1], MR[2]);
+    o[at(rec_vec_pos<double>(7, t))] = make_double2(MR[3], MR[4]);
+  }
+  __syncwarp();
+  // cell by cell: the warp's cells lie one step block (SWEEP_TJ slots) apart
+  const long long first = skew_slot(d, i, j, kw);
+  uint4 *const out = reinterpret_cast<uint4 *>(a.cellrec) + first * NV;
+#pragma unroll
+  for (int q = 0; q < NV; q++) {
+    const int e = q * (32 / NV) + lane / NV, u = lane % NV;   // cell and vector
+    if (kw + e <= d.nz + 1)
+      out[(long long)e * (SWEEP_TJ * NV) + u] = s_out[warp][e * NV + (u ^ (MIXED ? (e >> 1) & 3 : e & 7))];
   }
   // the lagged halos of the first sweep; an open slab's stay zero
-  if (!d.x_open && (i == ie || i == 3)) {
+  if (cell && !d.x_open && (i == ie || i == 3)) {
     double mm[9];
     cell_metrics<CH>(d, a, j, c, mm);
     Diag<double> dd = diag<double>(q, mm, d.dxi, d.det, d.dzt, deltaT);

@@ -119,13 +119,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void *map, uint3
       "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
       : "memory");
 }
-// untiled bulk copy global -> this CTA's shared memory (addresses 16-byte
-// aligned, size a multiple of 16), completing on an mbarrier
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"((uint64_t)src), "r"(bytes), "r"(bar)
-               : "memory");
-}
 __device__ __forceinline__ void tma_prefetch_desc(const void *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
