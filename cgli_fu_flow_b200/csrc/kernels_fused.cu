@@ -24,9 +24,9 @@ __device__ __forceinline__ void cell_metrics(const Dev &d, const SweepArgs &a, i
 // tables instead of ten 3-D metric arrays.
 // Bound by its bytes: 34 words in and 16 out a cell (606 us at 256x192x192 with
 // the streams' ramps), at eight CTAs per SM (128 registers, no spills).
-// 256x192x192 786 -> 670 us, 585 in mixed precision (632), 160x128x128 228 ->
-// 195, of which 14 us are the eight CTAs (six, at 166 registers, without the
-// cap) and the rest the store of whole lines; ten CTAs take 220, twelve 219.
+// 256x192x192 786 -> 670 us (102 by the store of whole lines, 14 by the eight
+// CTAs; six, at 166 registers, without the cap), 632 -> 585 in mixed precision;
+// 160x128x128 228 -> 195 (twelve CTAs: 219), mixed 185 -> 172 (ten: 225).
 template <bool MIXED, bool CH>
 __global__ void __launch_bounds__(64, 8)
     k_residual_fast(Dev d, SweepArgs a) {

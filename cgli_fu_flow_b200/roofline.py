@@ -20,13 +20,14 @@ PEAKS = os.path.join(os.path.dirname(HERE), "MEASURED_PEAKS.json")
 SWEEP_BYTES_PER_CELL = {"fp64": 25 * 8, "mixed": 25 * 4}
 
 # DRAM bytes (read + write) per cell of one sweep pass from an ncu capture of
-# the current k_sweep (16 x 16-column FP64 tiles; dram__bytes_read.sum +
-# dram__bytes_write.sum, forward 202 B and backward 250 B per cell, averaged)
-# on the 160x128x128 channel; traffic grows with the cell count, so it is
-# scaled to the benchmark grid.  The passes read each cell's 16-word record +
-# MR slot (the backward pass also its forward result) and write 5 words.  See
+# k_sweep (dram__bytes_read.sum + dram__bytes_write.sum, mean of the four
+# passes of an inner iteration: FP64 forward 165 / 165, backward 181 (only the
+# halo planes are stored) / 213; FP32 80 / 80, 91 / 103) on the 160x128x128
+# channel; traffic grows with the cell count, so it is scaled to the benchmark
+# grid.  The passes read each cell's 16-word record + MR slot (the backward
+# pass also its forward result) and write 5 words.  See
 # profiles/k_sweep_channel_160x128x128.md.
-MEASURED_TRAFFIC_PER_CELL = {"fp64": (202.2 + 250.2) / 2, "mixed": None}
+MEASURED_TRAFFIC_PER_CELL = {"fp64": (165 + 181 + 165 + 213) / 4, "mixed": (80 + 91 + 80 + 103) / 4}
 
 
 def hbm_peak() -> tuple[float, str]:
@@ -62,12 +63,12 @@ RESIDUAL_STAGES = ("halo_bc", "flux_x", "flux_y", "flux_z", "viscous", "residual
 
 # FP64 instructions per cell (thread level) of the residual side's kernels,
 # from ncu (sm__inst_executed_pipe_fp64.sum x 32 / cells) on the
-# 160x128x128 channel: fluxes 294 / 297 / 377 per face (x / y / z), k_vprim
-# 27, viscous faces 279 (channel form), k_viscous_div 24, residual assembly
-# 260.  With the FP64 pipe's measured rate on this GPU (a standalone FMA
-# probe: 34 TFLOP/s = 17 T FP64 instructions/s) this is a lower bound on the
-# side's time.  See profiles/k_flux_k_viscous_k_residual_fast_channel_160x128x128.md.
-RESIDUAL_FP64_OPS_PER_CELL = 294 + 297 + 377 + 27 + 279 + 24 + 260
+# 160x128x128 channel: fluxes 272 / 284 / 293 per face (x / y / z), the viscous
+# terms 335, residual assembly 260.  With the FP64 pipe's measured rate on this
+# GPU (a standalone FMA probe: 34 TFLOP/s = 17 T FP64 instructions/s) this is a
+# lower bound on the side's time.  See
+# profiles/k_flux_k_viscous_k_residual_fast_channel_160x128x128.md.
+RESIDUAL_FP64_OPS_PER_CELL = 272 + 284 + 293 + 335 + 260
 FP64_INST_PER_S = 17.0e12
 
 
@@ -77,7 +78,7 @@ def residual_roofline(ch, stage_ms: dict) -> dict:
     achieved = RESIDUAL_BYTES_PER_CELL * ch.cells / (dur_ms / 1e3) / 1e9
     fp64_ms = RESIDUAL_FP64_OPS_PER_CELL * ch.cells / FP64_INST_PER_S * 1e3
     peak, kind = hbm_peak()
-    return {"kernels": "halo/boundaries, k_flux_x/y/z, k_vprim + k_viscous_faces + k_viscous_div, k_residual_fast",
+    return {"kernels": "halo/boundaries, k_flux_x/y/z, k_viscous, k_residual_fast",
             "bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "peak_kind": kind, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "algorithmic_bytes_per_iteration": RESIDUAL_BYTES_PER_CELL * ch.cells,
             "ms_per_iteration": round(dur_ms, 4),
