@@ -113,9 +113,14 @@ __global__ void __launch_bounds__(256, 4) k_dplur_relax(Dev d, RelaxPtrs a) {
 // 737-908 without its zero sponge terms): MR and the first iterate
 // NL = D^-1 MR on the interior cells, with each repeated divisor as one
 // (Newton-refined) reciprocal, and the coefficient records of planes 2..ie+1.
-// CH as for the relaxation.
+// CH as for the relaxation.  Bound by its 55 words a cell (80 us at 128x96x96).
+// In the channel form the balance comes first, four blocks a SM, so that its 33
+// loads are under way together: a step of ten iterations there 5.79 -> 5.46 ms,
+// 256x192x192 42.9 -> 40.9; six and eight blocks give 5.55 and 5.62.  With nine
+// metric terms more to load (general grids) the same order is slower (7.68 ->
+// 7.73 at four blocks, 7.81 at three).
 template <bool CH>
-__global__ void __launch_bounds__(128) k_dplur_residual(Dev d, RelaxPtrs a) {
+__global__ void __launch_bounds__(128, CH ? 4 : 8) k_dplur_residual(Dev d, RelaxPtrs a) {
   int k = 2 + blockIdx.x * blockDim.x + threadIdx.x;
   int j = 2 + blockIdx.y;
   int i = 2 + blockIdx.z;
@@ -131,11 +136,29 @@ __global__ void __launch_bounds__(128) k_dplur_residual(Dev d, RelaxPtrs a) {
     for (int v = 0; v < 9; v++) mm[v] = d.m[v][c];
   }
   const double q1 = d.U_[0][c], q2 = d.U_[1][c], q3 = d.U_[2][c], q4 = d.U_[3][c], q5 = d.U_[4][c];
+  const bool halo = i == 2 || i == d.nx + 3;   // the halo planes enter the products only
+  double Rk[5];
+  const auto balance = [&]() {   // time derivative, flux differences, viscous terms
+    const long long fx1 = ix(d, i, j - 1, k - 1), f0 = ix(d, i - 1, j - 1, k - 1);
+    const long long fy1 = ix(d, i - 1, j, k - 1), fz1 = ix(d, i - 1, j - 1, k);
+    const double i2dt = nr_rcp(2 * d.dt), idx = d.rdxi, idy = d.rdet, idz = d.rdzt;
+    const double U_[5] = {q1, q2, q3, q4, q5};
+#pragma unroll
+    for (int n = 0; n < 5; n++) {
+      const double Rp = -(3 * U_[n] - 4 * d.U[n][c] + d.Uq[n][c]) * i2dt;
+      const double Rf = -((d.inF[0][n][fx1] - d.inF[0][n][f0]) * idx + (d.inF[1][n][fy1] - d.inF[1][n][f0]) * idy +
+                          (d.inF[2][n][fz1] - d.inF[2][n][f0]) * idz);
+      Rk[n] = Rp + Rf;
+    }
+#pragma unroll
+    for (int n = 1; n < 5; n++) Rk[n] = Rk[n] + d.vF[n - 1][c];
+  };
+  if (CH && !halo) balance();
   double rec[REC_N];
   make_record(q1, q2, q3, q4, q5, J, mm, d.e, d.rdxi, d.rdet, d.rdzt, d.dt, rec);
 #pragma unroll
   for (int v = 0; v < REC_N; v++) a.rec[v * a.n + c] = rec[v];
-  if (i == 2 || i == d.nx + 3) return;   // the halo planes enter the products only
+  if (halo) return;
   const CPrim<double> q = cprim<double>(q1, q2, q3, q4, q5, J, d.e);
   const double rho = q.rho, u = q.u, v = q.v, w = q.w, VV = q.VV, T = q.Tt, H = q.H, beta = q.beta;
   const double irho = nr_rcp(rho), itemp = irho * (1.0 / KG);
@@ -144,23 +167,10 @@ __global__ void __launch_bounds__(128) k_dplur_residual(Dev d, RelaxPtrs a) {
   const double d15 = (KG - 1) * beta;
   const double d51 = (KG - 1) * (VV + KG * T * beta + (KG - 1) * VV * beta + H * (-1 + beta - KG * beta)) * itemp;
   const double g5 = -(KG - 1) * (1 + (KG - 1) * beta) * itemp;
-  const long long fx1 = ix(d, i, j - 1, k - 1), f0 = ix(d, i - 1, j - 1, k - 1);
-  const long long fy1 = ix(d, i - 1, j, k - 1), fz1 = ix(d, i - 1, j - 1, k);
-  const double i2dt = nr_rcp(2 * d.dt), idx = d.rdxi, idy = d.rdet, idz = d.rdzt, iJ = nr_rcp(J);
-  const double f = d.scal[0];
-  const double U_[5] = {q1, q2, q3, q4, q5};
-  double Rk[5];
-#pragma unroll
-  for (int n = 0; n < 5; n++) {
-    const double Rp = -(3 * U_[n] - 4 * d.U[n][c] + d.Uq[n][c]) * i2dt;
-    const double Rf = -((d.inF[0][n][fx1] - d.inF[0][n][f0]) * idx + (d.inF[1][n][fy1] - d.inF[1][n][f0]) * idy +
-                        (d.inF[2][n][fz1] - d.inF[2][n][f0]) * idz);
-    Rk[n] = Rp + Rf;
-  }
-  Rk[1] = Rk[1] + d.vF[0][c] + f * iJ;
-  Rk[2] = Rk[2] + d.vF[1][c];
-  Rk[3] = Rk[3] + d.vF[2][c];
-  Rk[4] = Rk[4] + d.vF[3][c] + f * u * iJ;
+  if (!CH) balance();
+  const double iJ = nr_rcp(J), f = d.scal[0];
+  Rk[1] = Rk[1] + f * iJ;
+  Rk[4] = Rk[4] + f * u * iJ;
   double MR[5];
   MR[0] = d11 * Rk[0] + d12 * Rk[1] + d13 * Rk[2] + d14 * Rk[3] + d15 * Rk[4];
   MR[1] = (Rk[1] - u * Rk[0]) * irho;
