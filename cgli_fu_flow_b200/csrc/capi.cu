@@ -86,13 +86,17 @@ namespace {
 
 constexpr int kRing = 32;
 
+// Zeroed device memory.  The fill goes to the context's stream: that is a
+// non-blocking stream, which nothing orders against a fill of the default
+// stream (asynchronous to the host, and behind whatever the caller has queued
+// there), so the fill could come after the kernels that write the buffer.
 int alloc(cgli_ctx *c, size_t bytes, void **out) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e != cudaSuccess) return fail(CGLI_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  e = cudaMemset(p, 0, bytes);
-  if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
   c->allocs.push_back(p);
+  e = cudaMemsetAsync(p, 0, bytes, c->stream);
+  if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
   c->bytes += (long long)bytes;
   *out = p;
   return CGLI_OK;
@@ -337,6 +341,8 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
   d.buoyancy = p->buoyancy ? 1 : 0;
   d.high = p->high;
   int rc = CGLI_OK;
+  if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
+    rc = fail(CGLI_ECUDA, "cudaStreamCreate");
 #define F(x) if (rc == CGLI_OK) rc = field(c, &(x))
   for (int v = 0; v < 5; v++) {
     F(d.U_[v]); F(d.U[v]); F(d.Uq[v]); F(d.Uqq[v]); F(d.MR[v]); F(d.NL[v]); F(d.NR[v]);
@@ -381,7 +387,7 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
     if (rc == CGLI_OK) rc = alloc(c, a.hand_bytes, &a.xbuf);
     if (rc == CGLI_OK) {
       a.ybuf = (char *)a.xbuf + xb;
-      if (cudaMemset(a.xbuf, 0xff, a.hand_bytes) != cudaSuccess) rc = fail(CGLI_ECUDA, "cudaMemset");   // the sentinel
+      if (cudaMemsetAsync(a.xbuf, 0xff, a.hand_bytes, c->stream) != cudaSuccess) rc = fail(CGLI_ECUDA, "cudaMemsetAsync");   // the sentinel
     }
     if (rc == CGLI_OK) rc = alloc(c, 64, (void **)&a.ticket);
     if (rc == CGLI_OK) rc = alloc(c, 64, (void **)&a.clock);
@@ -406,14 +412,15 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
     cgli::sweep_tile_order((nti + a.cluster_x - 1) / a.cluster_x, cgli::sweep_tiles_y(p->ny), ti * a.cluster_x, order);
     int *dorder = nullptr;
     rc = alloc(c, sizeof(int) * order.size(), (void **)&dorder);
-    if (rc == CGLI_OK) cudaMemcpy(dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice);
+    if (rc == CGLI_OK && cudaMemcpyAsync(dorder, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice,
+                                         c->stream) != cudaSuccess)
+      rc = fail(CGLI_ECUDA, "cudaMemcpyAsync");
+    if (rc == CGLI_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = fail(CGLI_ECUDA, "cudaStreamSynchronize");
     a.order = dorder;
   }
   if (rc == CGLI_OK && (cudaMallocHost(&c->h_norms, 16 * sizeof(double)) != cudaSuccess ||
                         cudaMallocHost(&c->ring, kRing * sizeof(cgli::IterResult)) != cudaSuccess))
     rc = fail(CGLI_ENOMEM, "cudaMallocHost");
-  if (rc == CGLI_OK && cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
-    rc = fail(CGLI_ECUDA, "cudaStreamCreate");
   if (rc != CGLI_OK) {
     std::string keep = g_err;
     cgli_destroy(c);
@@ -428,14 +435,16 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
       rc = fail(CGLI_ECUDA, "cudaStreamCreate");
   if (rc == CGLI_OK && cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) != cudaSuccess)
     rc = fail(CGLI_ECUDA, "cudaEventCreate");
+  const double f = p->force;
+  if (rc == CGLI_OK && (cudaMemcpyAsync(d.scal, &f, sizeof f, cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+                        cudaStreamSynchronize(c->stream) != cudaSuccess))
+    rc = fail(CGLI_ECUDA, "driving force to the device");
   if (rc != CGLI_OK) {
     std::string keep = g_err;
     cgli_destroy(c);
     g_err = keep;
     return rc;
   }
-  double f = p->force;
-  cudaMemcpy(d.scal, &f, sizeof f, cudaMemcpyHostToDevice);
   *out = c;
   return CGLI_OK;
 }
