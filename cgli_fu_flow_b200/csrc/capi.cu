@@ -211,6 +211,16 @@ int read_norms(cgli_ctx *c, double er[5], int nblocks) {
   return CGLI_OK;
 }
 
+// After a pass that gave up or a norm that was not finite: clears the status
+// word and puts the sentinel back into the hand-over buffers (products that
+// were never read are left behind), on the stream of the passes, and waits.
+int clear_failure(cgli_ctx *c) {
+  CUDA_TRY(cudaMemsetAsync(c->d.status, 0, sizeof(int), c->stream));
+  CUDA_TRY(cudaMemsetAsync(c->sw.xbuf, 0xff, c->sw.hand_bytes, c->stream));
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return CGLI_OK;
+}
+
 // Launches the iteration graph n (<= kRing) times and waits; the iterations
 // need nothing from the host in between.  Returns how many of them are good
 // and their results; a failed one (its successors leave the state alone) sets
@@ -234,11 +244,10 @@ int run_iterations(cgli_ctx *c, int n, const cgli::IterResult *res[kRing], int *
       if (r.sweep_ms > 0) { c->sweep_ms += r.sweep_ms; c->sweep_passes += 4; }
       continue;
     }
-    cudaMemset(c->d.status, 0, sizeof(int));
-    // products that were never read are left behind: only the sentinel again
-    cudaMemset(c->sw.xbuf, 0xff, c->sw.hand_bytes);
-    *rc = r.status ? fail(CGLI_ETIMEOUT, "a wavefront tile gave up waiting for its neighbour (bounded spin)")
-                   : fail(CGLI_EDIVERGED, "update norm is not finite");
+    *rc = clear_failure(c);
+    if (*rc == CGLI_OK)
+      *rc = r.status ? fail(CGLI_ETIMEOUT, "a wavefront tile gave up waiting for its neighbour (bounded spin)")
+                     : fail(CGLI_EDIVERGED, "update norm is not finite");
     return it;
   }
   return n;

@@ -1,0 +1,72 @@
+"""What a failed inner iteration leaves behind: the status word is cleared and
+the hand-over buffers hold the sentinel again before the call returns, on the
+stream of the passes, so the next call runs normally.
+
+The timeout is forced with a wait limit of 0 polls (see test_failure.py).
+Grids: 12 x 2 CTAs of 4 rows x 32 columns along x and y, in clusters of up to 8
+along x, so products cross inside clusters, between clusters and between
+column blocks.  The compared context applies the boundary conditions once by
+hand, which is all that the failed iteration leaves in the state (the halo
+planes' wall ghost rows lag by one application), and must then give the same
+words."""
+import os
+import re
+
+import numpy as np
+import pytest
+
+from cgli_fu_flow_b200.channel import Channel
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cgli_fu_flow_b200", "csrc")
+ETIMEOUT = -6
+LIMIT = 4194304
+DIMS = (45, 40, 16)
+
+
+def test_no_fill_on_the_default_stream():
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "capi.cu")).read())
+    assert not re.search(r"\bcudaMemset\(", text)
+
+
+def words(g):
+    return g.q().view(np.int64)
+
+
+def boundaries(g):
+    g.halo_x()
+    g.y_boundary_condition()
+    g.x_boundary_condition()
+    g.z_boundary_condition()
+
+
+def time_out(call):
+    from cgli_fu_flow_b200.solver import CgliError
+    with pytest.raises(CgliError) as ei:
+        call()
+    assert ei.value.code == ETIMEOUT
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("queued", [False, True])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_retry_right_after_a_timeout(cuda_lib, precision, queued):
+    import torch
+    from cgli_fu_flow_b200.solver import Solver
+    g, h = Solver(Channel(*DIMS), precision), Solver(Channel(*DIMS), precision)
+    g.init()
+    h.init()
+    boundaries(h)
+    h.step(3)
+    g.set_wait_limit(0)
+    if queued:   # some 30 ms of the caller's work on the default stream
+        a = torch.ones(4096, 4096, device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        for _ in range(300):
+            torch.matmul(a, a)
+    time_out(g.inner_iteration)
+    g.set_wait_limit(LIMIT)
+    g.step(3)
+    torch.cuda.synchronize()
+    assert np.array_equal(words(g), words(h))
+    g.close()
+    h.close()
