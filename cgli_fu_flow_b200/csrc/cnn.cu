@@ -850,13 +850,16 @@ int cfail(int code, const std::string &m) {
     if (e_ != cudaSuccess) return cfail(CGLI_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Zeroed device memory, filled on the network's stream (a non-blocking one,
+// without an order against the default stream).  The buffers are also used on
+// a solver's stream: who allocates waits for n->stream before that.
 int calloc_dev(cgli_cnn *n, size_t bytes, void **out) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e != cudaSuccess) return cfail(CGLI_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  e = cudaMemset(p, 0, bytes);
-  if (e != cudaSuccess) return cfail(CGLI_ECUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
   n->allocs.push_back(p);
+  e = cudaMemsetAsync(p, 0, bytes, n->stream);
+  if (e != cudaSuccess) return cfail(CGLI_ECUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
   *out = p;
   return CGLI_OK;
 }
@@ -905,6 +908,7 @@ int ensure_training(cgli_cnn *n) {
   for (int i = 0; i < 2; i++)
     if (!act_map(&n->g6[i], n->g[i], n->nx, n->ny, n->nz, 6) || !act_map(&n->g4[i], n->g[i], n->nx, n->ny, n->nz, 4))
       return cfail(CGLI_ECUDA, "cuTensorMapEncodeTiled failed (gradient buffers)");
+  CC(cudaStreamSynchronize(n->stream));
   n->training = true;
   return CGLI_OK;
 }
@@ -914,7 +918,9 @@ int check_status(cgli_cnn *n, cudaStream_t s) {
   CC(cudaMemcpyAsync(&st, n->status, sizeof(int), cudaMemcpyDeviceToHost, s));
   CC(cudaStreamSynchronize(s));
   if (st) {
-    cudaMemsetAsync(n->status, 0, sizeof(int), s);
+    // the next call may use another stream
+    CC(cudaMemsetAsync(n->status, 0, sizeof(int), s));
+    CC(cudaStreamSynchronize(s));
     return cfail(CGLI_ETIMEOUT, "tensor-core kernel gave up waiting on a pipeline barrier");
   }
   return CGLI_OK;
@@ -1108,6 +1114,7 @@ int cgli_cnn_create(int nx, int ny, int nz, cgli_cnn **out) {
         !act_map(&n->act6[l], n->act[l], nx, ny, nz, 6) || !act_map(&n->act7[l], n->act[l], nx, ny, nz, 7))
       rc = cfail(CGLI_ECUDA, "cuTensorMapEncodeTiled failed");
   }
+  if (!rc && cudaStreamSynchronize(n->stream) != cudaSuccess) rc = cfail(CGLI_ECUDA, "cudaStreamSynchronize failed");
   for (int v = 0; v < 5; v++) {
     n->sc.mean[v] = 0.f; n->sc.inv_std[v] = 1.f; n->sc.inv_d1[v] = 1.f; n->sc.inv_d2[v] = 1.f;
     n->sc.oscale[v] = 1.f; n->sc.inv_oscale[v] = 1.f;

@@ -110,3 +110,33 @@ def test_statistics_and_filter_of_a_running_context(cuda_lib):
     for a, b in zip(*out):
         assert np.array_equal(a, b, equal_nan=True)
     assert np.array_equal(out[1][-1], y)
+
+
+def test_network_fills_are_on_a_stream():
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "cnn.cu")).read())
+    assert not re.search(r"\bcudaMemset\(", text)
+
+
+@pytest.mark.gpu
+def test_network_made_behind_queued_work(cuda_lib):
+    import torch
+    from cgli_fu_flow_b200.cnn import Network
+    from oracle import cnn_oracle as O
+    dims = (12, 8, 32)
+    rng = np.random.default_rng(5)
+    theta = O.init_params(5)
+    x0, target = rng.standard_normal((15,) + dims), rng.standard_normal((5,) + dims)
+    torch.cuda.synchronize()
+    out = []
+    for queued in (False, True):
+        if queued:
+            queue_work()
+        net = Network(*dims)
+        net.set_params(theta)
+        loss, grad = net.loss_grad(x0, target)   # allocates the training buffers
+        torch.cuda.synchronize()
+        out.append((loss, grad, net.get_params(), net.forward(x0)))
+        net.close()
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(a, b)
