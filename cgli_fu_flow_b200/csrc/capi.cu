@@ -54,7 +54,7 @@ struct cgli_ctx {
   std::vector<void *> allocs;
   long long bytes = 0;
   bool have_metrics = false, have_state = false;
-  double *h_norms = nullptr;   // pinned, 8 doubles
+  double *h_norms = nullptr;   // pinned: 8 doubles, then the status word
   double *d_out = nullptr;     // device scratch for norms / bulk flux
   int update_blocks = 0;         // partial sums of the per-row update kernels (routine path, DP-LUR)
   int sweep_update_blocks = 0;   // partial sums of the update after the wavefront passes
@@ -200,17 +200,6 @@ int last_launch(const char *what) {
   return CGLI_OK;
 }
 
-int read_norms(cgli_ctx *c, double er[5], int nblocks) {
-  double scale = 1.0 / ((double)c->p.nx * c->p.ny * c->p.nz);
-  cgli::launch_norms(c->d, c->stream, nblocks, scale, c->d_out);
-  CUDA_TRY(cudaMemcpyAsync(c->h_norms, c->d_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
-  for (int v = 0; v < 5; v++) er[v] = c->h_norms[v];
-  for (int v = 0; v < 5; v++)
-    if (!std::isfinite(er[v])) return fail(CGLI_EDIVERGED, "update norm is not finite");
-  return CGLI_OK;
-}
-
 // After a pass that gave up or a norm that was not finite: clears the status
 // word and puts the sentinel back into the hand-over buffers (products that
 // were never read are left behind), on the stream of the passes, and waits.
@@ -218,6 +207,35 @@ int clear_failure(cgli_ctx *c) {
   CUDA_TRY(cudaMemsetAsync(c->d.status, 0, sizeof(int), c->stream));
   CUDA_TRY(cudaMemsetAsync(c->sw.xbuf, 0xff, c->sw.hand_bytes, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return CGLI_OK;
+}
+
+// the error of a failed iteration, with what it left behind cleared; status
+// as its passes left it (0: a norm that is not finite)
+int report_failure(cgli_ctx *c, int status) {
+  int rc = clear_failure(c); if (rc) return rc;
+  return status == cgli::CGLI_TIMEOUT_CODE
+             ? fail(CGLI_ETIMEOUT, "a wavefront tile gave up waiting for its neighbour (bounded spin)")
+             : fail(CGLI_EDIVERGED, "update norm is not finite");
+}
+
+// waits for the stream and reports a status word that is set (a pass launched
+// outside the iteration graph has no other reader)
+int check_status(cgli_ctx *c) {
+  int *const status = (int *)(c->h_norms + 8);
+  CUDA_TRY(cudaMemcpyAsync(status, c->d.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return *status ? report_failure(c, *status) : CGLI_OK;
+}
+
+int read_norms(cgli_ctx *c, double er[5], int nblocks) {
+  double scale = 1.0 / ((double)c->p.nx * c->p.ny * c->p.nz);
+  cgli::launch_norms(c->d, c->stream, nblocks, scale, c->d_out);
+  CUDA_TRY(cudaMemcpyAsync(c->h_norms, c->d_out, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  int rc = check_status(c); if (rc) return rc;
+  for (int v = 0; v < 5; v++) er[v] = c->h_norms[v];
+  for (int v = 0; v < 5; v++)
+    if (!std::isfinite(er[v])) return fail(CGLI_EDIVERGED, "update norm is not finite");
   return CGLI_OK;
 }
 
@@ -244,10 +262,7 @@ int run_iterations(cgli_ctx *c, int n, const cgli::IterResult *res[kRing], int *
       if (r.sweep_ms > 0) { c->sweep_ms += r.sweep_ms; c->sweep_passes += 4; }
       continue;
     }
-    *rc = clear_failure(c);
-    if (*rc == CGLI_OK)
-      *rc = r.status ? fail(CGLI_ETIMEOUT, "a wavefront tile gave up waiting for its neighbour (bounded spin)")
-                     : fail(CGLI_EDIVERGED, "update norm is not finite");
+    *rc = report_failure(c, r.status);
     return it;
   }
   return n;
@@ -1114,8 +1129,9 @@ int cgli_profile_stages(cgli_ctx *c, int reps, double *ms) {
     cgli::launch_sweep_pass(c->d, c->sw, c->stream, mixed, false, true);
     cgli::launch_sweep_pass(c->d, c->sw, c->stream, mixed, true, true);
     cgli::launch_sweep_update(c->d, c->sw, c->stream, mixed);
-    rc = last_launch("profile_stages"); if (rc) return rc;
-    CUDA_TRY(cudaStreamSynchronize(c->stream));
+    rc = last_launch("profile_stages");
+    if (!rc) rc = check_status(c);
+    if (rc) break;
     for (int s = 0; s < CGLI_NSTAGES; s++) {
       float t = 0;
       CUDA_TRY(cudaEventElapsedTime(&t, ev[s], ev[s + 1]));
@@ -1123,6 +1139,7 @@ int cgli_profile_stages(cgli_ctx *c, int reps, double *ms) {
     }
   }
   for (auto &e : ev) cudaEventDestroy(e);
+  if (rc) return rc;
   for (int s = 0; s < CGLI_NSTAGES; s++) ms[s] = tot[s] / reps;
   return CGLI_OK;
 }

@@ -70,3 +70,33 @@ def test_retry_right_after_a_timeout(cuda_lib, precision, queued):
     assert np.array_equal(words(g), words(h))
     g.close()
     h.close()
+
+
+def routine_fluxes(g):
+    boundaries(g)
+    g.flux_x()
+    g.flux_y()
+    g.flux_z()
+    g.viscous_terms()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("reps", [1, 2])
+def test_profile_reports_a_timeout_and_the_routines_after_it_are_right(cuda_lib, reps):
+    from cgli_fu_flow_b200.solver import Solver
+    g, h = Solver(Channel(*DIMS)), Solver(Channel(*DIMS))
+    g.init()
+    h.init()
+    boundaries(h)
+    g.set_wait_limit(0)
+    time_out(lambda: g.profile_stages(reps))
+    g.set_wait_limit(LIMIT)
+    for routine in ("dplusgs", "dual_time_stepping"):
+        for s in (g, h):
+            routine_fluxes(s)
+        eg, eh = getattr(g, routine)(), getattr(h, routine)()
+        assert np.array_equal(eg, eh) and np.all(eg > 0)
+        assert np.array_equal(words(g), words(h))
+    assert all(t > 0 for t in g.profile_stages(1).values())
+    g.close()
+    h.close()
