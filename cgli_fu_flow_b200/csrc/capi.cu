@@ -242,8 +242,8 @@ int read_norms(cgli_ctx *c, double er[5], int nblocks) {
 // Launches the iteration graph n (<= kRing) times and waits; the iterations
 // need nothing from the host in between.  Returns how many of them are good
 // and their results; a failed one (its successors leave the state alone) sets
-// *rc and clears what it left behind.
-int run_iterations(cgli_ctx *c, int n, const cgli::IterResult *res[kRing], int *rc) {
+// *rc and clears what it left behind, and if it diverged er takes its norms.
+int run_iterations(cgli_ctx *c, int n, const cgli::IterResult *res[kRing], int *rc, double er[5]) {
   const long long first = c->launched;
   *rc = CGLI_OK;
   for (int it = 0; it < n; it++) {
@@ -263,6 +263,7 @@ int run_iterations(cgli_ctx *c, int n, const cgli::IterResult *res[kRing], int *
       continue;
     }
     *rc = report_failure(c, r.status);
+    if (*rc == CGLI_EDIVERGED) std::copy(r.norm, r.norm + 5, er);
     return it;
   }
   return n;
@@ -854,7 +855,7 @@ int cgli_inner_iteration(cgli_ctx *c, double er[5]) {
   if (!er) return fail(CGLI_EINVAL, "null er");
   rc = ensure_graph(c); if (rc) return rc;
   const cgli::IterResult *res[kRing];
-  if (run_iterations(c, 1, res, &rc) == 1) std::copy(res[0]->norm, res[0]->norm + 5, er);
+  if (run_iterations(c, 1, res, &rc, er) == 1) std::copy(res[0]->norm, res[0]->norm + 5, er);
   return rc;
 }
 
@@ -1012,7 +1013,8 @@ int cgli_step(cgli_ctx *c, int fixed_iters, double drop, int cap, int *iters, do
     // a fixed number of iterations needs no norms on the way
     const int n = fixed_iters > 0 ? std::min(fixed_iters - it, kRing) : 1;
     const cgli::IterResult *res[kRing];
-    const int good = run_iterations(c, n, res, &rc);
+    double failed[5];
+    const int good = run_iterations(c, n, res, &rc, failed);
     for (int q = 0; q < good; q++) {
       it++;
       std::copy(res[q]->norm, res[q]->norm + 5, er);
@@ -1025,6 +1027,7 @@ int cgli_step(cgli_ctx *c, int fixed_iters, double drop, int cap, int *iters, do
       }
       stop = fixed_iters > 0 ? it >= fixed_iters : done || it >= cap;
     }
+    if (rc == CGLI_EDIVERGED) std::copy(failed, failed + 5, er);
     if (rc) return rc;
   }
   *iters = it;

@@ -188,7 +188,8 @@ int cgli_set_inner_solver(cgli_ctx *ctx, int solver);
 /* One complete inner iteration (main.cpp:167-264) through the fused fast
  * path: halo + boundaries, fluxes, viscous terms, the dual-time residual,
  * then the wavefront sweeps and the update (CGLI_LUSGS) or the relaxations
- * and the update (CGLI_DPLUR). */
+ * and the update (CGLI_DPLUR).  er: the five update norms, also with
+ * CGLI_EDIVERGED (some of them not finite then). */
 int cgli_inner_iteration(cgli_ctx *ctx, double er[5]);
 
 /* Driven_force.cpp:14-74: bulk mass flux (volume-weighted mean of rho*u) */
@@ -203,7 +204,8 @@ int cgli_set_force(cgli_ctx *ctx, double force);
  * its running maximum over the run (main.cpp:287-297, reset by
  * cgli_set_state) is below `drop`, or `cap` iterations ran (fixed_iters > 0
  * runs exactly that many), then the time-level shift (Q^(n-2) is kept too).
- * Returns the iteration count and the final norms. */
+ * Returns the iteration count and the final norms.  CGLI_EDIVERGED: er holds
+ * the norms of the iteration that had one that is not finite. */
 int cgli_step(cgli_ctx *ctx, int fixed_iters, double drop, int cap, int *iters, double er[5]);
 /* The five norms of every inner iteration of the last cgli_step, iteration
  * by iteration (norms[5*i + v]); copies min(iterations, max_iters) rows and

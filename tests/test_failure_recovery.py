@@ -100,3 +100,24 @@ def test_profile_reports_a_timeout_and_the_routines_after_it_are_right(cuda_lib,
     assert all(t > 0 for t in g.profile_stages(1).values())
     g.close()
     h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solver", ["lusgs", "dplur"])
+def test_divergence_leaves_its_norms(cuda_lib, solver):
+    import ctypes
+    from cgli_fu_flow_b200.solver import Solver
+    ch = Channel(8, 12, 8)
+    q = ch.initial_conserved().copy()
+    q[2, 4, 5, 3] = np.nan
+    g = Solver(ch)
+    g.set_inner_solver(solver)
+    calls = {"iteration": lambda er: g.L.cgli_inner_iteration(g.h, er),
+             "fixed": lambda er: g.L.cgli_step(g.h, 4, 1e-3, 30, ctypes.byref(ctypes.c_int()), er),
+             "drop": lambda er: g.L.cgli_step(g.h, 0, 1e-3, 30, ctypes.byref(ctypes.c_int()), er)}
+    for name, call in calls.items():
+        g.init(q)
+        er = (ctypes.c_double * 5)(*[7.0] * 5)
+        assert call(er) == -5, name
+        assert 7.0 not in er[:] and not np.all(np.isfinite(er[:])), (name, er[:])
+    g.close()
