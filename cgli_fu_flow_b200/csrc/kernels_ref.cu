@@ -22,6 +22,13 @@ __global__ void k_halo_x(Dev d) {
   q[t] = q[(long long)(ie - 2) * plane + t];
 }
 
+// An iteration queued behind one that failed (a pass gave up, a norm was not
+// finite) leaves U_ alone, ghost cells included: the boundaries advance some of
+// them at every application (the end planes of an open slab, the halo planes'
+// wall rows).  Read with the cells that the kernel needs, tested before its
+// stores.
+__device__ __forceinline__ int iteration_failed(const Dev &d) { return *(const volatile int *)d.status; }
+
 // Y_boundary_condition.cpp:94-182 for interior planes i = 3..ie: the
 // zero-gradient copy of :100-112, replaced inside the heated section
 // (planes nx_inlet+3 .. Nx-nx_outlet+2, :114) by the isothermal no-slip
@@ -48,8 +55,10 @@ __device__ __forceinline__ void wall_ghost(const Dev &d, int i, int k, int side,
 __global__ void k_bc_y(Dev d) {
   const int k = 2 + blockIdx.x * blockDim.x + threadIdx.x, i = 3 + blockIdx.y, side = blockIdx.z;
   if (k > d.nz + 1) return;
+  const int failed = iteration_failed(d);
   double q[5];
   wall_ghost(d, i, k, side, q);
+  if (failed) return;
   for (int v = 0; v < 5; v++) d.U_[v][ix(d, i, side ? d.ny + 2 : 1, k)] = q[v];
 }
 
@@ -67,8 +76,11 @@ __global__ void k_bc_z(Dev d) {
   long long row = t * d.dj;
   int kn = d.nz + 1;
   double *q = d.U_[v];
-  q[row + 1] = q[row + kn];
-  q[row + kn + 1] = q[row + 2];
+  const int failed = iteration_failed(d);
+  const double left = q[row + kn], right = q[row + 2];
+  if (failed) return;
+  q[row + 1] = left;
+  q[row + kn + 1] = right;
 }
 
 // k_halo_x, k_bc_y and k_bc_z of a periodic slab in one launch: the same
@@ -83,6 +95,7 @@ __global__ void k_bc_z(Dev d) {
 //   blocks [nb, ..): columns 1 and kn+1 of the interior planes' other rows
 __global__ void __launch_bounds__(128) k_halo_bc(Dev d, unsigned na, unsigned nb) {
   const int ie = d.nx + 2, jn = d.ny + 1, kn = d.nz + 1;
+  const int failed = iteration_failed(d);
   if (blockIdx.x < na) {
     const long long t = blockIdx.x * 128LL + threadIdx.x;
     if (t >= 6 * d.di) return;
@@ -90,7 +103,10 @@ __global__ void __launch_bounds__(128) k_halo_bc(Dev d, unsigned na, unsigned nb
     if ((j == 1 || j == jn + 1) && k >= 1 && k <= kn + 1) return;
     const int i = p < 3 ? p : ie + 1 + p - 3, is = p < 3 ? ie - 2 + p : p;
     const long long c = ix(d, is, j, k == 1 ? kn : k == kn + 1 ? 2 : k);
-    for (int v = 0; v < 5; v++) d.U_[v][i * d.di + r] = d.U_[v][c];
+    double q[5];
+    for (int v = 0; v < 5; v++) q[v] = d.U_[v][c];
+    if (failed) return;
+    for (int v = 0; v < 5; v++) d.U_[v][i * d.di + r] = q[v];
     return;
   }
   if (blockIdx.x < nb) {
@@ -101,6 +117,7 @@ __global__ void __launch_bounds__(128) k_halo_bc(Dev d, unsigned na, unsigned nb
     const long long g = ix(d, i, jg, k);
     double q[5];
     wall_ghost(d, i, k == 1 ? kn : k == kn + 1 ? 2 : k, side, q);
+    if (failed) return;
     if (k > 1 && k <= kn) {
       const int lo = i - (ie - 2), hi = ie + 1 + i - 3;   // the planes that hold this cell's images
       for (int v = 0; v < 5; v++) {
@@ -121,10 +138,10 @@ __global__ void __launch_bounds__(128) k_halo_bc(Dev d, unsigned na, unsigned nb
   const int right = (int)(t & 1), j = (int)(t / 2 % d.Y), i = 3 + (int)(t / 2 / d.Y);
   if (i > ie || j == 1 || j == jn + 1) return;
   const long long row = ix(d, i, j, 0);
-  for (int v = 0; v < 5; v++) {
-    double *const o = d.U_[v] + row;
-    o[right ? kn + 1 : 1] = o[right ? 2 : kn];
-  }
+  double q[5];
+  for (int v = 0; v < 5; v++) q[v] = d.U_[v][row + (right ? 2 : kn)];
+  if (failed) return;
+  for (int v = 0; v < 5; v++) d.U_[v][row + (right ? kn + 1 : 1)] = q[v];
 }
 
 // X_boundary_condition.cpp:73-338 on an open slab: one pseudo-time step of
@@ -141,6 +158,7 @@ __global__ void k_bc_x(Dev d) {
   const int ie = d.nx + 2;
   const long long c = ix(d, side ? ie : 3, j, k), g = ix(d, side ? ie + 1 : 2, j, k);
   const double K = KG, deltaT = d.dt, deltaTau = deltaT / 200., rdx = 1 / d.dxi;
+  const int failed = iteration_failed(d);
   double q[5], qi[5];
 #pragma unroll
   for (int v = 0; v < 5; v++) { q[v] = d.U_[v][g]; qi[v] = d.U_[v][c]; }
@@ -206,6 +224,7 @@ __global__ void k_bc_x(Dev d) {
   const double iJg = 1 / Jg, i2dt = 1 / (2 * deltaT);
 #pragma unroll
   for (int v = 0; v < 5; v++) KAL[v] = KAL[v] * iJg + (3 * q[v] - 4 * d.U[v][g] + d.Uq[v][g]) * i2dt;
+  if (failed) return;
 #pragma unroll
   for (int v = 0; v < 5; v++)
     d.U_[v][g] = q[v] - deltaTau * (dm[v][0] * KAL[0] + dm[v][1] * KAL[1] + dm[v][2] * KAL[2] + dm[v][3] * KAL[3] +

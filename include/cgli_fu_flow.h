@@ -205,7 +205,9 @@ int cgli_set_force(cgli_ctx *ctx, double force);
  * cgli_set_state) is below `drop`, or `cap` iterations ran (fixed_iters > 0
  * runs exactly that many), then the time-level shift (Q^(n-2) is kept too).
  * Returns the iteration count and the final norms.  CGLI_EDIVERGED: er holds
- * the norms of the iteration that had one that is not finite. */
+ * the norms of the iteration that had one that is not finite.  After an error
+ * U_ is as the failing iteration left it; with fixed_iters, iterations already
+ * queued behind it still form inF, vF (and MR, NL, NR with CGLI_DPLUR). */
 int cgli_step(cgli_ctx *ctx, int fixed_iters, double drop, int cap, int *iters, double er[5]);
 /* The five norms of every inner iteration of the last cgli_step, iteration
  * by iteration (norms[5*i + v]); copies min(iterations, max_iters) rows and

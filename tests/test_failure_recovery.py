@@ -121,3 +121,51 @@ def test_divergence_leaves_its_norms(cuda_lib, solver):
         assert call(er) == -5, name
         assert 7.0 not in er[:] and not np.all(np.isfinite(er[:])), (name, er[:])
     g.close()
+
+
+OPEN = dict(x_open=True, nx_inlet=4, nx_outlet=5, buoyancy=True, twall_lo=343.0592)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("kw", [{}, dict(wavy=True, wave=0.01), OPEN], ids=["flat", "wavy", "open"])
+def test_iterations_behind_a_timeout_leave_the_state_alone(cuda_lib, kw, precision):
+    """A step whose first iteration times out, with nine more behind it, leaves
+    the words of one iteration that timed out (ghost cells included), and so
+    does the retry."""
+    from cgli_fu_flow_b200.solver import Solver
+    ch = Channel(*DIMS, **kw)
+    g, h = Solver(ch, precision), Solver(ch, precision)
+    g.init()
+    h.init()
+    for s, call in ((g, lambda: g.step(10)), (h, h.inner_iteration)):
+        s.set_wait_limit(0)
+        time_out(call)
+        s.set_wait_limit(LIMIT)
+    assert np.array_equal(words(g), words(h))
+    g.step(2)
+    h.step(2)
+    assert np.array_equal(words(g), words(h))
+    g.close()
+    h.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solver", ["lusgs", "dplur"])
+@pytest.mark.parametrize("kw", [{}, OPEN], ids=["flat", "open"])
+def test_iterations_behind_a_divergence_leave_the_state_alone(cuda_lib, kw, solver):
+    from cgli_fu_flow_b200.solver import CgliError, Solver
+    ch = Channel(17, 12, 8, **kw)
+    q = ch.initial_conserved().copy()
+    q[2, 8, 5, 3] = np.nan
+    out = []
+    for fixed in (True, False):
+        g = Solver(ch)
+        g.set_inner_solver(solver)
+        g.init(q)
+        with pytest.raises(CgliError) as ei:
+            g.step(10) if fixed else g.inner_iteration()
+        assert ei.value.code == -5
+        out.append(words(g))
+        g.close()
+    assert np.array_equal(out[0], out[1])
