@@ -93,7 +93,10 @@ constexpr int kRing = 32;
 int alloc(cgli_ctx *c, size_t bytes, void **out) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) return fail(CGLI_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // reported here: the next call's launch check must not find it
+    return fail(CGLI_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   c->allocs.push_back(p);
   e = cudaMemsetAsync(p, 0, bytes, c->stream);
   if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
@@ -444,8 +447,10 @@ int cgli_create(const cgli_params *p, cgli_ctx **out) {
     a.order = dorder;
   }
   if (rc == CGLI_OK && (cudaMallocHost(&c->h_norms, 16 * sizeof(double)) != cudaSuccess ||
-                        cudaMallocHost(&c->ring, kRing * sizeof(cgli::IterResult)) != cudaSuccess))
+                        cudaMallocHost(&c->ring, kRing * sizeof(cgli::IterResult)) != cudaSuccess)) {
+    cudaGetLastError();
     rc = fail(CGLI_ENOMEM, "cudaMallocHost");
+  }
   if (rc != CGLI_OK) {
     std::string keep = g_err;
     cgli_destroy(c);

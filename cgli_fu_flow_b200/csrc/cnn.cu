@@ -856,7 +856,10 @@ int cfail(int code, const std::string &m) {
 int calloc_dev(cgli_cnn *n, size_t bytes, void **out) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) return cfail(CGLI_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // reported here: the next call's launch check must not find it
+    return cfail(CGLI_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   n->allocs.push_back(p);
   e = cudaMemsetAsync(p, 0, bytes, n->stream);
   if (e != cudaSuccess) return cfail(CGLI_ECUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
@@ -1108,7 +1111,10 @@ int cgli_cnn_create(int nx, int ny, int nz, cgli_cnn **out) {
   if (!rc) rc = calloc_dev(n, sizeof(float) * 4, (void **)&n->loss);
   if (!rc) rc = calloc_dev(n, sizeof(double) * ((n->cells + 255) / 256 + 1), (void **)&n->blk_loss);
   if (!rc) rc = calloc_dev(n, sizeof(int) * 4, (void **)&n->status);
-  if (!rc && cudaMallocHost(&n->h_loss, sizeof(float) * 4) != cudaSuccess) rc = cfail(CGLI_ENOMEM, "cudaMallocHost failed");
+  if (!rc && cudaMallocHost(&n->h_loss, sizeof(float) * 4) != cudaSuccess) {
+    cudaGetLastError();
+    rc = cfail(CGLI_ENOMEM, "cudaMallocHost failed");
+  }
   for (int l = 0; l < NL && !rc; l++) {
     if (!weight_map(&n->wf_map[l], n->wf[l]) || !weight_map(&n->wt_map[l], n->wt[l]) ||
         !act_map(&n->act6[l], n->act[l], nx, ny, nz, 6) || !act_map(&n->act7[l], n->act[l], nx, ny, nz, 7))
@@ -1252,7 +1258,10 @@ int cgli_cnn_reserve_levels(cgli_cnn *n, int count) {
   for (int i = 0; i < count; i++) {
     float *p = nullptr;
     cudaError_t e = cudaMalloc(&p, (size_t)n->cells * 5 * 4);
-    if (e != cudaSuccess) return cfail(CGLI_ENOMEM, std::string("cudaMalloc (levels): ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return cfail(CGLI_ENOMEM, std::string("cudaMalloc (levels): ") + cudaGetErrorString(e));
+    }
     n->levels.push_back(p);
   }
   return CGLI_OK;
