@@ -60,6 +60,7 @@ struct cgli_ctx {
   int sweep_update_blocks = 0;   // partial sums of the update after the wavefront passes
   cgli::SweepArgs sw;
   bool metrics_checked = false;
+  bool met_current = false;      // sw.met holds the present metrics
   cudaGraphExec_t iter_graph = nullptr;
   cudaEvent_t events[8] = {};
   double Emax[5] = {0, 0, 0, 0, 0};   // running maximum of the norms over the run
@@ -105,6 +106,12 @@ int alloc(cgli_ctx *c, size_t bytes, void **out) {
   return CGLI_OK;
 }
 
+int last_launch(const char *what) {
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  return CGLI_OK;
+}
+
 int field(cgli_ctx *c, double **out) {
   size_t n = (size_t)c->d.X * c->d.Y * c->d.Z;
   return alloc(c, n * sizeof(double), (void **)out);
@@ -136,6 +143,22 @@ int ensure_filter(cgli_ctx *c) {
 int ensure_dplur(cgli_ctx *c) {
   if (c->sw.drec) return CGLI_OK;
   return alloc(c, (size_t)cgli::REC_N * c->d.X * c->d.di * sizeof(double), (void **)&c->sw.drec);
+}
+
+// the metric terms in the wavefront passes' step order (general grids), before
+// the first passes on new metrics: a context that runs none needs no room for
+// them
+int ensure_metric_stream(cgli_ctx *c) {
+  if (c->sw.channel_metrics || c->met_current) return CGLI_OK;
+  const bool mixed = c->p.precision == CGLI_MIXED;
+  if (!c->sw.met) {
+    int rc = alloc(c, (size_t)cgli::skew_size(c->d) * 9 * (mixed ? sizeof(float) : sizeof(double)), &c->sw.met);
+    if (rc) return rc;
+  }
+  cgli::launch_metric_stream(c->d, c->sw, c->stream, mixed);
+  int rc = last_launch("metric stream"); if (rc) return rc;
+  c->met_current = true;
+  return CGLI_OK;
 }
 
 // device array of a reference name; *is_metric tells whether it is one of
@@ -194,12 +217,6 @@ int need_ready(cgli_ctx *c) {
   if (!c->have_state) return fail(CGLI_ESTATE, "state not set (cgli_set_state)");
   // quantities derived from the metrics (1/J, the channel tables), once per change
   if (!c->metrics_checked) { int rc = check_channel_metrics(c); if (rc) return rc; }
-  return CGLI_OK;
-}
-
-int last_launch(const char *what) {
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return fail(CGLI_ECUDA, std::string(what) + ": " + cudaGetErrorString(e));
   return CGLI_OK;
 }
 
@@ -310,14 +327,7 @@ int check_channel_metrics(cgli_ctx *c) {
     CUDA_TRY(cudaMemcpy((void *)c->sw.etdytab, et.data(), sizeof(double) * d.Y, cudaMemcpyHostToDevice));
   }
   c->sw.channel_metrics = ok ? 1 : 0;
-  if (!ok) {
-    const bool mixed = c->p.precision == CGLI_MIXED;
-    if (!c->sw.met) {
-      int rc = alloc(c, (size_t)cgli::skew_size(d) * 9 * (mixed ? sizeof(float) : sizeof(double)), &c->sw.met);
-      if (rc) return rc;
-    }
-    cgli::launch_metric_stream(d, c->sw, c->stream, mixed);
-  }
+  c->met_current = false;
   c->d.face_tables = 0;
   c->d.face_tables = cgli::check_face_tables(c->d, c->d.status + 8, c->stream) ? 1 : 0;
   cgli::launch_inverse_j(d, c->stream);
@@ -820,6 +830,7 @@ int cgli_set_inner_solver(cgli_ctx *c, int solver) {
 static int ensure_graph(cgli_ctx *c) {
   if (c->iter_graph) return CGLI_OK;
   const bool dplur = c->inner_solver == CGLI_DPLUR, mixed = c->p.precision == CGLI_MIXED;
+  if (!dplur) { int rc = ensure_metric_stream(c); if (rc) return rc; }
   cudaStream_t s = c->stream;
   cudaGraph_t g;
   CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -1003,6 +1014,7 @@ int cgli_step(cgli_ctx *c, int fixed_iters, double drop, int cap, int *iters, do
   rc = need_ready(c); if (rc) return rc;
   if (!iters || !er) return fail(CGLI_EINVAL, "null argument");
   if (fixed_iters <= 0 && (cap <= 0 || !(drop > 0))) return fail(CGLI_EINVAL, "need fixed_iters > 0 or cap > 0 and drop > 0");
+  rc = ensure_graph(c); if (rc) return rc;   // (before the guess changes U_: it may allocate)
   if (c->predictor == 2 && c->history >= 2) {
     CUDA_TRY(cgli::cnn_predict(c->cnn, c->d, c->stream));
   } else if (c->predictor >= 1 && c->history >= 1) {
@@ -1012,7 +1024,6 @@ int cgli_step(cgli_ctx *c, int fixed_iters, double drop, int cap, int *iters, do
   }
   int it = 0;
   c->step_norms.clear();
-  rc = ensure_graph(c); if (rc) return rc;
   bool stop = false;
   while (!stop) {
     // a fixed number of iterations needs no norms on the way
@@ -1111,6 +1122,7 @@ int cgli_profile_stages(cgli_ctx *c, int reps, double *ms) {
   rc = need_ready(c); if (rc) return rc;
   if (!ms || reps < 1) return fail(CGLI_EINVAL, "bad argument");
   if (!c->metrics_checked) { rc = check_channel_metrics(c); if (rc) return rc; }
+  rc = ensure_metric_stream(c); if (rc) return rc;
   const bool mixed = c->p.precision == CGLI_MIXED;
   cudaEvent_t ev[CGLI_NSTAGES + 1];
   for (auto &e : ev) CUDA_TRY(cudaEventCreate(&e));
