@@ -287,6 +287,8 @@ __global__ void k_target_u(Dev d) {
 // and a block per 64 faces of a row; 254 / 284 / 254 now (160x128x128 91 / 101
 // / 113 -> 80 / 91 / 82, 91x53x75 25 / 26 / 25 -> 19 / 20 / 19).
 //
+constexpr int FLUX_CTAS = 12;   // CTAs per SM of the x and y faces
+
 // Face (i, j, k) of this thread, i from 2, j and k from 1, of planes of nj
 // rows of nk faces: a block of 64 per piece of a row, or (FLAT) of the plane's
 // faces as one run, which leaves no lanes idle at the row ends but costs the
@@ -302,7 +304,7 @@ __device__ __forceinline__ bool face_of(int nk, int nj, int &i, int &j, int &k) 
 
 // x faces i = 2..ie, tangential j = 1..jn-1, k = 1..kn-1 (Flux_X.cpp:96-357)
 template <bool CH, bool FLAT, bool MARCH>
-__global__ void __launch_bounds__(64, 12) k_flux_x(Dev d, int chunk) {
+__global__ void __launch_bounds__(64, FLUX_CTAS) k_flux_x(Dev d, int chunk) {
   int i0, j, k;
   if (!face_of<FLAT>(d.nz, d.ny, i0, j, k)) return;
   i0 = 2 + (i0 - 2) * chunk;
@@ -359,7 +361,7 @@ __device__ __forceinline__ void muscl_y(const Dev &d, int i, int j, int k, doubl
 
 // y faces j = 1..jn, i = 2..ie-1, k = 1..kn-1 (Flux_Y.cpp:94-413)
 template <bool CH, bool FLAT, bool MARCH>
-__global__ void __launch_bounds__(64, 12) k_flux_y(Dev d, int chunk) {
+__global__ void __launch_bounds__(64, FLUX_CTAS) k_flux_y(Dev d, int chunk) {
   int i, j0, k;
   const int nc = (d.ny + chunk) / chunk;
   if (!face_of<FLAT>(d.nz, nc, i, j0, k)) return;
@@ -413,7 +415,7 @@ __device__ __forceinline__ void muscl_z(const Dev &d, int i, int j, int k, doubl
 
 // z faces k = 1..kn, i = 2..ie-1, j = 1..jn-1 (Flux_Z.cpp:91-359)
 template <bool CH, bool FLAT, bool MARCH>
-__global__ void __launch_bounds__(64, CH ? 16 : 12) k_flux_z(Dev d, int) {
+__global__ void __launch_bounds__(64, CH ? 16 : FLUX_CTAS) k_flux_z(Dev d, int) {
   int i, j, k;
   if (!face_of<FLAT>(d.nz + 1, d.ny, i, j, k)) return;
   long long f = ix(d, i, j, k);
@@ -680,7 +682,12 @@ void launch_bc_z(const Dev &d, cudaStream_t s) {
 // of blocks (160x128x128 x / y 87 / 95 -> 80 / 90 us, general metrics 109 / 111
 // -> 98 / 105; at 128x96x96, 2.6 waves, 45 / 52 -> 44 / 56 and general y 61 ->
 // 71; 8 faces are slower than 4 everywhere)
-static bool flux_march(long long faces) { return faces / (4 * 64) >= 4 * 12 * 148; }
+static bool flux_march(long long faces) {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return faces / (4 * 64) >= 4LL * FLUX_CTAS * sms;
+}
 void launch_flux_x(const Dev &d, cudaStream_t s) {
   if (flux_march((long long)d.nz * d.ny * (d.nx + 1))) FLUX(k_flux_x, true, d.nz, d.ny, (d.nx + 4) / 4);
   else FLUX(k_flux_x, false, d.nz, d.ny, d.nx + 1);
