@@ -101,9 +101,6 @@ int sweep_update_blocks(const Dev &d);
 // one pass of the first or the last sweep (a forward one with both passes'
 // halo products)
 void launch_sweep_pass(const Dev &d, const SweepArgs &a, cudaStream_t s, bool mixed, bool backward, bool last);
-// Dual_time_stepping.cpp:737-922 residual on the natural layout: MR and
-// NL = NR = D^-1 MR on the interior cells
-void launch_dts_residual(const Dev &d, cudaStream_t s);
 // DP-LUR inner solver of DPLUSGS.cpp (kernels_dplur.cu): residual, four
 // Jacobi relaxations (final result in NR), update with per-block partial
 // sums of the squared squared increments in d.partial (nx * ny blocks).

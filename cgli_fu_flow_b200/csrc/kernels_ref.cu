@@ -3,6 +3,8 @@
 // as the reference, so every entry point of include/cgli_fu_flow.h can be
 // checked against its counterpart on its own.  The fused fast path of
 // cgli_inner_iteration lives in kernels_fused.cu.
+#include <type_traits>
+
 #include "cgli_dev.cuh"
 #include "cgli_launch.h"
 
@@ -414,8 +416,8 @@ __device__ __forceinline__ void muscl_z(const Dev &d, int i, int j, int k, doubl
 }
 
 // z faces k = 1..kn, i = 2..ie-1, j = 1..jn-1 (Flux_Z.cpp:91-359)
-template <bool CH, bool FLAT, bool MARCH>
-__global__ void __launch_bounds__(64, CH ? 16 : FLUX_CTAS) k_flux_z(Dev d, int) {
+template <bool CH, bool FLAT>
+__global__ void __launch_bounds__(64, CH ? 16 : FLUX_CTAS) k_flux_z(Dev d) {
   int i, j, k;
   if (!face_of<FLAT>(d.nz + 1, d.ny, i, j, k)) return;
   long long f = ix(d, i, j, k);
@@ -666,18 +668,20 @@ void launch_bc_z(const Dev &d, cudaStream_t s) {
 // faces of 192 cells, 193 in four blocks: 340 -> 283 us at 256x192x192, and at
 // 91x53x75 25 -> 19 us each; but with 192 x faces a row, which fill their
 // blocks, it costs 300 -> 317 us)
-#define FLUX(kern, march, nk, nj, ni)                                                                \
-  do {                                                                                               \
-    const bool flat = ((nk) + 63) / 64 * 64 * 4 >= (nk) * 5;                                         \
-    const dim3 g(flat ? (unsigned)(((long long)(nk) * (nj) + 63) / 64) : ((nk) + 63) / 64, flat ? 1 : (nj), ni); \
-    if (d.face_tables) {                                                                             \
-      if (flat) kern<true, true, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                         \
-      else kern<true, false, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                             \
-    } else {                                                                                         \
-      if (flat) kern<false, true, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                        \
-      else kern<false, false, march><<<g, 64, 0, s>>>(d, march ? 4 : 1);                                            \
-    }                                                                                                \
-  } while (0)
+template <class Launch>
+static void launch_faces(const Dev &d, int nk, int nj, int ni, Launch kernel) {
+  const std::true_type yes;
+  const std::false_type no;
+  const bool flat = (nk + 63) / 64 * 64 * 4 >= nk * 5;
+  const dim3 g(flat ? (unsigned)(((long long)nk * nj + 63) / 64) : (nk + 63) / 64, flat ? 1 : nj, ni);
+  if (d.face_tables) {
+    if (flat) kernel(g, yes, yes);
+    else kernel(g, yes, no);
+  } else {
+    if (flat) kernel(g, no, yes);
+    else kernel(g, no, no);
+  }
+}
 // x and y: 4 faces per thread along the stencil where that leaves four waves
 // of blocks (160x128x128 x / y 87 / 95 -> 80 / 90 us, general metrics 109 / 111
 // -> 98 / 105; at 128x96x96, 2.6 waves, 45 / 52 -> 44 / 56 and general y 61 ->
@@ -688,17 +692,32 @@ static bool flux_march(long long faces) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return faces / (4 * 64) >= 4LL * FLUX_CTAS * sms;
 }
+template <bool MARCH>
+static void flux_x(const Dev &d, cudaStream_t s) {
+  constexpr int chunk = MARCH ? 4 : 1;
+  launch_faces(d, d.nz, d.ny, (d.nx + chunk) / chunk, [&](dim3 g, auto ch, auto flat) {
+    k_flux_x<decltype(ch)::value, decltype(flat)::value, MARCH><<<g, 64, 0, s>>>(d, chunk);
+  });
+}
+template <bool MARCH>
+static void flux_y(const Dev &d, cudaStream_t s) {
+  constexpr int chunk = MARCH ? 4 : 1;
+  launch_faces(d, d.nz, (d.ny + chunk) / chunk, d.nx, [&](dim3 g, auto ch, auto flat) {
+    k_flux_y<decltype(ch)::value, decltype(flat)::value, MARCH><<<g, 64, 0, s>>>(d, chunk);
+  });
+}
 void launch_flux_x(const Dev &d, cudaStream_t s) {
-  if (flux_march((long long)d.nz * d.ny * (d.nx + 1))) FLUX(k_flux_x, true, d.nz, d.ny, (d.nx + 4) / 4);
-  else FLUX(k_flux_x, false, d.nz, d.ny, d.nx + 1);
+  if (flux_march((long long)d.nz * d.ny * (d.nx + 1))) flux_x<true>(d, s);
+  else flux_x<false>(d, s);
 }
 void launch_flux_y(const Dev &d, cudaStream_t s) {
-  if (flux_march((long long)d.nz * (d.ny + 1) * d.nx)) FLUX(k_flux_y, true, d.nz, (d.ny + 4) / 4, d.nx);
-  else FLUX(k_flux_y, false, d.nz, d.ny + 1, d.nx);
+  if (flux_march((long long)d.nz * (d.ny + 1) * d.nx)) flux_y<true>(d, s);
+  else flux_y<false>(d, s);
 }
-void launch_flux_z(const Dev &d, cudaStream_t s) { FLUX(k_flux_z, false, d.nz + 1, d.ny, d.nx); }
-void launch_dts_residual(const Dev &d, cudaStream_t s) {
-  k_dts_residual<<<cellgrid(d.nz, d.ny, d.nx, 64), 64, 0, s>>>(d);
+void launch_flux_z(const Dev &d, cudaStream_t s) {
+  launch_faces(d, d.nz + 1, d.ny, d.nx, [&](dim3 g, auto ch, auto flat) {
+    k_flux_z<decltype(ch)::value, decltype(flat)::value><<<g, 64, 0, s>>>(d);
+  });
 }
 
 void launch_dts(const Dev &d, cudaStream_t s, int update_blocks_x) {
