@@ -1,11 +1,13 @@
 """Roofline bookkeeping of the dominant kernel (the wavefront sweep passes).
 
-Algorithmic bytes of one sweep pass per cell, the per-unit figure of the
-hot-path scope (compulsory traffic with each array touched once per pass):
-the FP64 pass reads Q/J (5), J and nine metric terms (10) and MR or NL (5)
-and writes NL or NR (5): 25 doubles = 200 B; with the sweep state, metrics
-and MR/NL/NR in float (CGLI_MIXED) the same 25 words are 100 B.  The bound is
-HBM bandwidth (no dense contraction); the peak is the measured copy bandwidth
+Algorithmic bytes of one sweep pass per cell: what the four passes of an inner
+iteration cannot do without, given the record + MR slot of 16 words that the
+residual leaves per cell, over four.  A forward pass reads the slot and writes
+its result (16 + 5 words); a backward pass reads the slot and that result; the
+last one writes its own (16 + 5 + 5), the first sweep's stores only the halo
+planes (16 + 5).  Together 89 words, a mean of 178 B (FP64) or 89 B (CGLI_MIXED)
+per pass; on a general grid every pass also reads nine metric words.  The bound
+is HBM bandwidth (no dense contraction); the peak is the measured copy bandwidth
 of this GPU type (MEASURED_PEAKS.json, the burst figure, since the pass is
 timed alone), else 6650 GB/s, an earlier measurement on the same hardware.
 """
@@ -17,17 +19,21 @@ import os
 HERE = os.path.dirname(os.path.abspath(__file__))
 PEAKS = os.path.join(os.path.dirname(HERE), "MEASURED_PEAKS.json")
 
-SWEEP_BYTES_PER_CELL = {"fp64": 25 * 8, "mixed": 25 * 4}
+SWEEP_WORDS_PER_CELL = (21 + 21 + 21 + 26) / 4
+GENERAL_METRIC_WORDS = 9
+WORD_BYTES = {"fp64": 8, "mixed": 4}
 
 # DRAM bytes (read + write) per cell of one sweep pass from an ncu capture of
 # k_sweep (dram__bytes_read.sum + dram__bytes_write.sum, mean of the four
 # passes of an inner iteration: FP64 forward 165 / 165, backward 181 (only the
 # halo planes are stored) / 213; FP32 80 / 80, 91 / 103) on the 160x128x128
 # channel; traffic grows with the cell count, so it is scaled to the benchmark
-# grid.  The passes read each cell's 16-word record + MR slot (the backward
-# pass also its forward result) and write 5 words.  See
-# profiles/k_sweep_channel_160x128x128.md.
+# grid.  Channel metrics only.
 MEASURED_TRAFFIC_PER_CELL = {"fp64": (165 + 181 + 165 + 213) / 4, "mixed": (80 + 91 + 80 + 103) / 4}
+
+
+def sweep_bytes_per_cell(precision: str, general: bool = False) -> float:
+    return (SWEEP_WORDS_PER_CELL + (GENERAL_METRIC_WORDS if general else 0)) * WORD_BYTES[precision]
 
 
 def hbm_peak() -> tuple[float, str]:
@@ -41,15 +47,15 @@ def hbm_peak() -> tuple[float, str]:
 def sweep_roofline(ch, pass_ms: float, precision: str) -> dict:
     """pass_ms: mean device time of one wavefront pass."""
     cells = ch.cells
-    bpc = SWEEP_BYTES_PER_CELL[precision]
+    bpc = sweep_bytes_per_cell(precision, ch.wavy)
     dur_ms = pass_ms
     achieved = bpc * cells / (dur_ms / 1e3) / 1e9
     peak, kind = hbm_peak()
-    tpc = MEASURED_TRAFFIC_PER_CELL.get(precision)
+    tpc = None if ch.wavy else MEASURED_TRAFFIC_PER_CELL.get(precision)
     return {"kernel": "k_sweep (LU-SGS wavefront pass, forward/backward mean)", "bound": "hbm",
             "achieved": round(achieved, 1), "peak": peak, "peak_kind": kind, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "traffic": None if tpc is None else int(tpc * cells),
-            "algorithmic_bytes_per_launch": bpc * cells, "launch_ms": round(dur_ms, 4)}
+            "algorithmic_bytes_per_launch": int(bpc * cells), "launch_ms": round(dur_ms, 4)}
 
 
 # Algorithmic bytes of the residual side of one inner iteration per cell
@@ -66,8 +72,7 @@ RESIDUAL_STAGES = ("halo_bc", "flux_x", "flux_y", "flux_z", "viscous", "residual
 # 160x128x128 channel: fluxes 272 / 284 / 293 per face (x / y / z), the viscous
 # terms 335, residual assembly 260.  With the FP64 pipe's measured rate on this
 # GPU (a standalone FMA probe: 34 TFLOP/s = 17 T FP64 instructions/s) this is a
-# lower bound on the side's time.  See
-# profiles/k_flux_k_viscous_k_residual_fast_channel_160x128x128.md.
+# lower bound on the side's time.
 RESIDUAL_FP64_OPS_PER_CELL = 272 + 284 + 293 + 335 + 260
 FP64_INST_PER_S = 17.0e12
 
