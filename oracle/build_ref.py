@@ -37,7 +37,17 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REPO = os.path.dirname(HERE)
-REF_SRC = os.environ.get("CGLI_REFERENCE_DIR", "/root/reference")
+
+
+def _reference_dir() -> str:
+    """The reference tree, or the path of the source that it lacks: an empty
+    folder counts as absent for whoever asks whether this is a directory."""
+    tree = os.environ.get("CGLI_REFERENCE_DIR", "/root/reference")
+    probe = os.path.join(tree, "Jacobian.cpp")
+    return tree if os.path.isfile(probe) else probe
+
+
+REF_SRC = _reference_dir()
 
 SOURCES = [
     "Jacobian.cpp", "Jacobian_u.cpp", "Jacobian_v.cpp", "Jacobian_w.cpp",
