@@ -58,9 +58,10 @@ __device__ __forceinline__ void product(const Dev &d, const RelaxPtrs &a, long l
 // uniform in x and z, read per row from etdytab.
 // Bound by the loads: 26 words a cell from memory (38 us at 128x96x96), the
 // neighbours' from L1 (along j and k, blocks of 8 rows) and L2 (along x), four
-// blocks a SM to cover their latency.  128x96x96: 53.5 us, where tiles that
-// marched along x, staged the state in shared memory and formed each split
-// Jacobian once took 116 (two CTAs a SM, one plane's latency after another).
+// blocks a SM to cover their latency (64 registers; general metrics spill 24 B).
+// 128x96x96: 53.5 us, where tiles that marched along x, staged the state in
+// shared memory and formed each split Jacobian once took 116 (two CTAs a SM, one
+// plane's latency after another).
 template <bool CH>
 __global__ void __launch_bounds__(256, 4) k_dplur_relax(Dev d, RelaxPtrs a) {
   const int k = 2 + blockIdx.x * 32 + (threadIdx.x & 31);

@@ -292,9 +292,10 @@ __global__ void k_target_u(Dev d) {
 // ---------------------------------------------------------------- fluxes
 // Bound by the FP64 pipe (some 280 instructions a face in the channel form:
 // 160 us at 256x192x192) and, before it, by the loads of six arrays' stencils.
-// Caps of 12 CTAs per SM (80 registers, no spills in the channel form, where
-// only the live metric terms are formed) and 16 for the z faces (64 registers)
-// were the fastest of 10 to 16.  On large grids x and y faces march `chunk`
+// Caps of 12 CTAs per SM (80 registers; in the channel form, where only the live
+// metric terms are formed, without spills but for the y faces that march over
+// planes as one run: 36 / 32 B; general metrics up to 68 / 64 B) and 16 for the
+// channel's z faces (64 registers) were the fastest of 10 to 16.  On large grids x and y faces march `chunk`
 // faces along their stencil (MARCH), so that five of six stencil cells come
 // from L1.  x / y / z at 256x192x192: 300 / 335 / 340 us with the general form
 // and a block per 64 faces of a row; 254 / 284 / 254 now (160x128x128 91 / 101

@@ -64,9 +64,9 @@
 // it records the timeout code in the status word and posts what it has, so
 // that every warp runs to the end of the pass without waiting, computing
 // values nobody will use; the ring waits inside a CTA follow the dead flag
-// too (but not those on pushed products, push_wait).  The update kernel then
-// leaves the state alone, the host reports CGLI_ETIMEOUT and refills the
-// buffers with the sentinel.
+// too (but not those on pushed products, which end with the row before them:
+// push_wait).  The update kernel then leaves the state alone, the host reports
+// CGLI_ETIMEOUT and refills the buffers with the sentinel.
 // Clusters take tickets in the order in which the wavefront reaches them,
 // where every dependency holds a smaller ticket, so a waiting CTA only ever
 // waits on CTAs that are already running.

@@ -212,7 +212,8 @@ int march_chunk(int nx, int cols, int resident, int start) {
 // form needs 114 registers; at 256x192x192 7 rows with three CTAs per SM (64
 // registers) take 522 us, 9 rows with two (80) 505, 5 rows with three (80) 495,
 // 13 rows 418.  General metrics at 160x128x128: 6 rows with two 457, 5 rows
-// with two 410, 9 rows with one 442, 13 rows 360.
+// with two 410, 9 rows with one 442, 13 rows 360 (128 registers, 344 B of spill
+// stores and 240 of loads).
 void launch_viscous(const Dev &d, cudaStream_t s) {
   if (d.face_tables) viscous<true, 13, 1>(d, s);
   else viscous<false, 13, 1>(d, s);

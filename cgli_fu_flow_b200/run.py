@@ -10,8 +10,8 @@ the last norms and the device time of the step); --iterations N runs N bare
 inner iterations from the seeded field (the five norms of each), the form
 used for kernel profiles; --stages REPS runs two inner iterations, then times
 each stage of one inner iteration REPS times (cgli_profile_stages) and also
-reports the wavefront passes per dependent step of the tile wavefront (the
-tile shape the library was built with, cgli_sweep_tile_shape).  --dims runs the seeded channel on any grid instead of a named
+reports the wavefront passes per dependent step (of the rows and columns per
+CTA that the library was built with, cgli_sweep_tile_shape).  --dims runs the seeded channel on any grid instead of a named
 workload.  One JSON line per step / iteration / stage report.
 """
 from __future__ import annotations

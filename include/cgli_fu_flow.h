@@ -226,10 +226,13 @@ int cgli_set_predictor(cgli_ctx *ctx, int mode);
  * tiles (the reference has none: its OpenMP barriers wait without limit): a
  * tile waiting for its neighbour's products polls at most `polls` times
  * (default CGLI_WAIT_LIMIT_DEFAULT, well over a second), then records a
- * timeout; from then on no wait of the pass waits again, the pass runs to
- * its end computing values that are discarded, the update leaves U_
+ * timeout; from then on every such poll gives up, the pass runs to its end
+ * computing values that are discarded, the update leaves the interior of U_
  * unchanged, the call returns CGLI_ETIMEOUT and the next call runs normally.
- * 0 makes those waits give up at once (for tests of the timeout path). */
+ * Waits between neighbouring CTAs of one cluster and inside a CTA hold no
+ * poll of their own: they end with the rows before them, which run on after a
+ * timeout (a fixed count bounds them against a failing device only).  0 makes
+ * the polls give up at once (for tests of the timeout path). */
 #define CGLI_WAIT_LIMIT_DEFAULT 4194304
 int cgli_set_wait_limit(cgli_ctx *ctx, int polls);
 /* The (i, j) column tile of the wavefront passes this library was built
