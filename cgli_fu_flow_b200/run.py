@@ -11,8 +11,9 @@ inner iterations from the seeded field (the five norms of each), the form
 used for kernel profiles; --stages REPS runs two inner iterations, then times
 each stage of one inner iteration REPS times (cgli_profile_stages) and also
 reports the wavefront passes per dependent step (of the rows and columns per
-CTA that the library was built with, cgli_sweep_tile_shape).  --dims runs the seeded channel on any grid instead of a named
-workload.  One JSON line per step / iteration / stage report.
+CTA that the library was built with, cgli_sweep_tile_shape).  --dims runs the
+seeded channel on any grid instead of a named workload.  One JSON line per
+step / iteration / stage report.
 """
 from __future__ import annotations
 

@@ -67,3 +67,23 @@ def test_iterations_after_a_timeout(cuda_lib, dims, precision, grid):
     assert np.array_equal(g.q().view(np.int64), h.q().view(np.int64))
     g.close()
     h.close()
+
+
+@pytest.mark.parametrize("grid", list(GRIDS))
+@pytest.mark.parametrize("precision", [0, 1])
+def test_nan_products_are_values(cuda_lib, precision, grid):
+    """The polls through memory wait for a bit pattern that no arithmetic
+    produces: products that are NaN arrive like any other, so a state that is
+    not finite is a divergence, not a timeout."""
+    from cgli_fu_flow_b200.solver import CgliError, Solver
+    ch = Channel(*SHAPES[0], **GRIDS[grid])
+    q = ch.initial_conserved().copy()
+    q[2, 4, 5, 3] = np.nan
+    g = Solver(ch, precision)
+    for sign in (1, -1):
+        q[2, 4, 5, 3] = np.copysign(np.nan, sign)
+        g.init(q)
+        with pytest.raises(CgliError) as ei:
+            g.step(4)
+        assert ei.value.code == -5
+    g.close()
